@@ -146,6 +146,22 @@ struct Dft<T, 3, INV> {
   }
 };
 
+// 6 = 2 x 3 by the Chinese remainder map: no twiddles.
+template <typename T, bool INV>
+struct Dft<T, 6, INV> {
+  static __device__ __forceinline__ void run(cplx<T>* v) {
+    cplx<T> s[3] = {cadd(v[0], v[3]), cadd(v[2], v[5]), cadd(v[4], v[1])};
+    cplx<T> d[3] = {csub(v[0], v[3]), csub(v[2], v[5]), csub(v[4], v[1])};
+    Dft<T, 3, INV>::run(s);
+    Dft<T, 3, INV>::run(d);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      v[(4 * k) % 6] = s[k];
+      v[(3 + 4 * k) % 6] = d[k];
+    }
+  }
+};
+
 template <typename T, bool INV>
 struct Dft<T, 5, INV> {
   static __device__ __forceinline__ void run(cplx<T>* v) {
@@ -224,6 +240,7 @@ __device__ __forceinline__ void fft_stage_rt(int R, cplx<T>* buf, const Batch& B
     case 3: fft_stage<T, 3, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 4: fft_stage<T, 4, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 5: fft_stage<T, 5, INV>(buf, B, n, Ls, tw, buf_len); break;
+    case 6: fft_stage<T, 6, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 8: fft_stage<T, 8, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 16: fft_stage<T, 16, INV>(buf, B, n, Ls, tw, buf_len); break;
     default: break;
@@ -256,30 +273,26 @@ __device__ __forceinline__ void fft_inverse(cplx<T>* buf, const Batch& B, const 
 // Compile-time transforms for power-of-two lengths and for 12, 24 and 48.
 // Same DIF/DIT algorithm and slot order as above (the host builds its
 // digit-reversal tables from ct_radix), but every index is a compile-time
-// expression, the radices are 16 and 8 (two shared-memory stages for
-// n <= 256; 12, 24, 48 add a radix-3 stage), and twiddles come from a
-// shared-memory copy of the table.  Stage plans: 4:[4] 8:[8] 16:[16] 32:[8,4]
-// 64:[4,16] 128:[16,8] 256:[16,16] 512:[16,8,4] 12:[4,3] 24:[8,3] 48:[16,3].
-// 64 starts with radix 4 so
-// that its first stage (16 butterflies per transform, elements 16 apart) can
-// read a 64-point row straight from global memory in 128-byte runs.
+// expression, two stages cover n <= 256, and twiddles come from a
+// shared-memory copy of the table.  The radices suit fft_lane.cuh's kernels:
+// the last radix of a half row m = Lx/2 is even (two neighbouring x slots
+// form one FP32 element), the first radix of every length is even (the x
+// pass pairs the butterflies of k and -k), and a butterfly is at most 16
+// elements (64 registers).
 __host__ __device__ constexpr bool ct_supported(int n) {
   return n == 4 || n == 8 || n == 16 || n == 32 || n == 64 || n == 128 || n == 256 || n == 512 || n == 12 ||
          n == 24 || n == 48;
 }
-// 12, 24, 48 (the 24^3 and 48^3 supercells of the batched sweeps): a
-// power-of-two stage, then a radix-3 one (the runtime plan's order for 12
-// and 24)
-__host__ __device__ constexpr int ct_nst(int n) {
-  return (n == 12 || n == 24 || n == 48) ? 2 : (n <= 16 ? 1 : (n <= 256 ? 2 : 3));
-}
+__host__ __device__ constexpr int ct_nst(int n) { return n == 4 ? 1 : (n <= 256 ? 2 : 3); }
 __host__ __device__ constexpr int ct_radix(int n, int st) {
-  return n == 12 ? (st == 0 ? 4 : 3)
-       : n == 24 ? (st == 0 ? 8 : 3)
-       : n == 48 ? (st == 0 ? 16 : 3)
-       : n <= 16 ? n
+  return n == 4 ? 4
+       : n == 8 ? (st == 0 ? 4 : 2)
+       : n == 12 ? (st == 0 ? 6 : 2)
+       : n == 16 ? (st == 0 ? 8 : 2)
+       : n == 24 ? (st == 0 ? 6 : 4)
        : n == 32 ? (st == 0 ? 8 : 4)
-       : n == 64 ? (st == 0 ? 4 : 16)
+       : n == 48 ? (st == 0 ? 8 : 6)
+       : n == 64 ? (st == 0 ? 16 : 4)
        : n == 128 ? (st == 0 ? 16 : 8)
        : n == 256 ? 16
        : (st == 0 ? 16 : (st == 1 ? 8 : 4));

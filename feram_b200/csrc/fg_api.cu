@@ -23,7 +23,6 @@ using namespace fg;
 
 namespace {
 
-constexpr int kThreadsFFT = 512;
 constexpr int kThreadsZ = 256;
 constexpr int kThreadsElem = 256;
 
@@ -248,23 +247,23 @@ int check_device_error(fg_ctx* ctx) {
 // runtime-plan kernels take every other size.
 template <typename T, int MODE, class F>
 void with_xy_fwd(int m, int Ly, F f) {
-  if (m == 64 && Ly == 128) f(k_xy_fwd<T, MODE, 64, 128>);
-  else if (m == 32 && Ly == 64) f(k_xy_fwd<T, MODE, 32, 64>);
-  else if (m == 16 && Ly == 32) f(k_xy_fwd<T, MODE, 16, 32>);
-  else if (m == 8 && Ly == 16) f(k_xy_fwd<T, MODE, 8, 16>);
-  else if (m == 24 && Ly == 48) f(k_xy_fwd<T, MODE, 24, 48>);
-  else if (m == 12 && Ly == 24) f(k_xy_fwd<T, MODE, 12, 24>);
-  else f(k_xy_fwd<T, MODE, 0, 0>);
+  if (m == 64 && Ly == 128) f(k_xy_fwd<T, MODE, 64, 128>, xy_threads<T, 64, 128>());
+  else if (m == 32 && Ly == 64) f(k_xy_fwd<T, MODE, 32, 64>, xy_threads<T, 32, 64>());
+  else if (m == 16 && Ly == 32) f(k_xy_fwd<T, MODE, 16, 32>, xy_threads<T, 16, 32>());
+  else if (m == 8 && Ly == 16) f(k_xy_fwd<T, MODE, 8, 16>, xy_threads<T, 8, 16>());
+  else if (m == 24 && Ly == 48) f(k_xy_fwd<T, MODE, 24, 48>, xy_threads<T, 24, 48>());
+  else if (m == 12 && Ly == 24) f(k_xy_fwd<T, MODE, 12, 24>, xy_threads<T, 12, 24>());
+  else f(k_xy_fwd<T, MODE, 0, 0>, xy_threads<T, 0, 0>());
 }
 template <typename T, class F>
 void with_xy_inv(int m, int Ly, F f) {
-  if (m == 64 && Ly == 128) f(k_xy_inv<T, 64, 128>);
-  else if (m == 32 && Ly == 64) f(k_xy_inv<T, 32, 64>);
-  else if (m == 16 && Ly == 32) f(k_xy_inv<T, 16, 32>);
-  else if (m == 8 && Ly == 16) f(k_xy_inv<T, 8, 16>);
-  else if (m == 24 && Ly == 48) f(k_xy_inv<T, 24, 48>);
-  else if (m == 12 && Ly == 24) f(k_xy_inv<T, 12, 24>);
-  else f(k_xy_inv<T, 0, 0>);
+  if (m == 64 && Ly == 128) f(k_xy_inv<T, 64, 128>, xy_threads<T, 64, 128>());
+  else if (m == 32 && Ly == 64) f(k_xy_inv<T, 32, 64>, xy_threads<T, 32, 64>());
+  else if (m == 16 && Ly == 32) f(k_xy_inv<T, 16, 32>, xy_threads<T, 16, 32>());
+  else if (m == 8 && Ly == 16) f(k_xy_inv<T, 8, 16>, xy_threads<T, 8, 16>());
+  else if (m == 24 && Ly == 48) f(k_xy_inv<T, 24, 48>, xy_threads<T, 24, 48>());
+  else if (m == 12 && Ly == 24) f(k_xy_inv<T, 12, 24>, xy_threads<T, 12, 24>());
+  else f(k_xy_inv<T, 0, 0>, xy_threads<T, 0, 0>());
 }
 template <typename T>
 constexpr int z_cw_cap() { return sizeof(T) == 4 ? 8 : 4; }
@@ -343,8 +342,8 @@ template <typename T, int MODE>
 int launch_xy_fwd(fg_ctx* ctx, const T* src, cplx<T>* spec, int ncomp, int smem, const cplx<T>* twx,
                   const cplx<T>* twm, const cplx<T>* twy, const T* zstar = nullptr, int zu0 = 0) {
   const Geom& g = ctx->g;
-  with_xy_fwd<T, MODE>(g.m, g.Ly, [&](auto kern) {
-    launch_dep(ctx, kern, dim3(g.Lz, ncomp), kThreadsFFT, smem, src, spec, g, ctx->px, ctx->py, twx, twm, twy,
+  with_xy_fwd<T, MODE>(g.m, g.Ly, [&](auto kern, int nt) {
+    launch_dep(ctx, kern, dim3(g.Lz, ncomp), nt, smem, src, spec, g, ctx->px, ctx->py, twx, twm, twy,
                ctx->posm, 0, zstar, zu0, (const RepArgs*)nullptr);
   });
   CKL();
@@ -356,8 +355,8 @@ int launch_xy_fwd(fg_ctx* ctx, const T* src, cplx<T>* spec, int ncomp, int smem,
 template <typename T>
 int launch_xy_inv(fg_ctx* ctx, const cplx<T>* spec, T* out, int ncomp, bool strain_prologue = false) {
   const Geom& g = ctx->g;
-  with_xy_inv<T>(g.m, g.Ly, [&](auto kern) {
-    launch_dep(ctx, kern, dim3(g.Lz, ncomp), kThreadsFFT, ctx->smem_xy,
+  with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
+    launch_dep(ctx, kern, dim3(g.Lz, ncomp), nt, ctx->smem_xy,
         spec, out, g, ctx->px, ctx->py, (const cplx<T>*)ctx->twx, (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy,
         ctx->posm, 0, strain_prologue ? ctx->ph : nullptr, ctx->sc, ctx->part_k, ctx->zt.nreg + ctx->zt.nnyq,
         (const RepArgs*)nullptr);
@@ -605,8 +604,8 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
              (const T*)nullptr, (const DevScalars*)nullptr, g, (const double*)nullptr, (const T*)nullptr, grp);
   CKL();
   c0->pdl = true;
-  with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto kern) {
-    launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), kThreadsFFT, c0->smem_xy, (const T*)nullptr, (cplx<T>*)nullptr,
+  with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto kern, int nt) {
+    launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), nt, c0->smem_xy, (const T*)nullptr, (cplx<T>*)nullptr,
                g, c0->px, c0->py, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm, (const cplx<T>*)c0->twy,
                c0->posm, 0, (const T*)nullptr, 0, grp);
   });
@@ -618,8 +617,8 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
                (unsigned int*)nullptr, (const T*)nullptr, grp);
   });
   CKL();
-  with_xy_inv<T>(g.m, g.Ly, [&](auto kern) {
-    launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), kThreadsFFT, c0->smem_xy, (const cplx<T>*)nullptr, (T*)nullptr, g,
+  with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
+    launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), nt, c0->smem_xy, (const cplx<T>*)nullptr, (T*)nullptr, g,
                c0->px, c0->py, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm, (const cplx<T>*)c0->twy, c0->posm,
                0, (const Phys*)c0->ph, (DevScalars*)nullptr, (const double*)nullptr, c0->zt.nreg + c0->zt.nnyq, grp);
   });
@@ -875,10 +874,10 @@ int create_impl(fg_ctx* ctx) {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
       if (e != cudaSuccess) ea = e;
     };
-    with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto k) { setattr(k, ctx->smem_xy); });
-    with_xy_fwd<T, SRC_FIELD>(g.m, g.Ly, [&](auto k) { setattr(k, ctx->smem_xy); });
-    with_xy_fwd<double, SRC_FIELD>(g.m, g.Ly, [&](auto k) { setattr(k, ctx->smem_xy64); });
-    with_xy_inv<T>(g.m, g.Ly, [&](auto k) { setattr(k, ctx->smem_xy); });
+    with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
+    with_xy_fwd<T, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
+    with_xy_fwd<double, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy64); });
+    with_xy_inv<T>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
     with_z_kspace<T>(g.Lz, ctx->zt.CW, ctx->acou, false, [&](auto k) { setattr(k, ctx->smem_z); });
     with_z_pass<T, false>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
     with_z_pass<T, true>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });

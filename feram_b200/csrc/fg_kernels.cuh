@@ -17,7 +17,7 @@
 //   k_assemble   per site: dipole-dipole + anharmonic + field + homogeneous
 //                and inhomogeneous strain coupling forces
 #pragma once
-#include "fft_smem.cuh"
+#include "fft_lane.cuh"
 
 namespace fg {
 
@@ -267,13 +267,14 @@ enum { SRC_U9 = 0, SRC_FIELD = 1 };
 // Z* (zstar != null) components zu0..zu0+2 are Z*(R) u (Z_u_R, dipoFFT.F:
 // 36-44).  SRC_FIELD: component c of src.
 // MC, LYC > 0 select the compile-time transforms for m = Lx/2 = MC and
-// Ly = LYC (launched with exactly kXYThreads threads); 0 = runtime plans.
-// The compile-time kernels run the y transforms on MC columns, not MC + 1:
-// the kx = 0 and kx = Lx/2 columns are real before the y pass (transforms of
-// real rows), so X(0) + i X(Lx/2) travels as one complex column and is split
-// by Hermitian symmetry after the pass (y_split); the inverse joins them the
-// same way before its y pass (y_join).  posm + m and posm + m + Ly hold the
-// y slot maps (slot -> ky, ky -> slot) that pair ky with -ky.
+// Ly = LYC (xy_fwd_ct / xy_inv_ct, launched with XyCT::NT threads); 0 =
+// runtime plans (512 threads).  The compile-time kernels run the y transforms
+// on MC columns, not MC + 1: the kx = 0 and kx = Lx/2 columns are real before
+// the y pass (transforms of real rows), so X(0) + i X(Lx/2) travels as one
+// complex column and is split by Hermitian symmetry after the pass (y_split);
+// the inverse joins them the same way before its y pass (y_join).  posm + m
+// and posm + m + Ly hold the y slot maps (slot -> ky, ky -> slot) that pair
+// ky with -ky.
 constexpr int kXYThreads = 512;
 
 // Column kx = 0 after the forward y pass holds C = Y0 + i Ym, Y0 and Ym the
@@ -297,167 +298,484 @@ __device__ __forceinline__ C y_join(C a0, C b0, C am, C bm) {
   return mk<C>(h0x - hmy, h0y + hmx);
 }
 
+// Shapes of the compile-time x-y transforms of a plane, on elements of W
+// transforms (fft_lane.cuh).
+//   x: rows q + NQ (2 l + h) of the plane (l < W, h < 2) form one group: rows
+//      h = 0 and 1 are the real and imaginary part of one complex transform of
+//      length Lx, and the W pairs its lanes.  R1 x R2 stages; the second stage
+//      takes the butterflies of k and -k in one thread (R1/2 tasks per group),
+//      which separates the two rows' half spectra in registers: no pass of its
+//      own for the real transform, no twiddles for it.
+//   y: W neighbouring x slots form one element; RY1 x RY2 stages.
+// A plane thus takes three round trips through shared memory.  Groups are
+// stored [q][x] with a row of Lx + 1 elements, columns [j][y] with Ly + 1:
+// every stage's 8 neighbouring lanes touch 8 different 16-byte banks, and all
+// element offsets of a thread are compile-time constants.  NT threads hold
+// one second-stage task each (at most 16 elements = 64 registers of data);
+// 512 threads of them fill an SM's registers.
 template <typename T, int MC, int LYC>
-__device__ __forceinline__ void xy_twiddles_to_smem(cplx<T>* tm, cplx<T>* ty, cplx<T>* tx, const cplx<T>* twm,
-                                                    const cplx<T>* twy, const cplx<T>* twx) {
-  if constexpr (MC > 0) {
-    for (int i = threadIdx.x; i < MC; i += blockDim.x) tm[i] = twm[i];
-    for (int i = threadIdx.x; i < LYC; i += blockDim.x) ty[i] = twy[i];
-    for (int i = threadIdx.x; i <= MC; i += blockDim.x) tx[i] = twx[i];
+struct XyCT {
+  static constexpr int W = kLanes<T>;
+  static constexpr int LX = 2 * MC, R1 = ct_radix(MC, 0), R2 = LX / R1;
+  static constexpr int RY1 = ct_radix(LYC, 0), RY2 = LYC / RY1;
+  static constexpr int NQ = LYC / (2 * W), NJ = MC / W;
+  static constexpr int QS = LX + 1, JS = LYC + 1;
+  // First x stage (and last inverse one): the butterfly of offset b reads
+  // x = b + R2 s.  Group q takes the same butterfly from offset
+  // bg = b + R2 (q % G) on, wrapping around the row (the transform of a
+  // rotated sequence, whose twiddles are those of offset bg), so that the
+  // lanes of a warp, R2 offsets of 32 / R2 rows, are spread over a row's
+  // 128-byte lines instead of hitting one 32-byte bank group in each row.
+  static constexpr int G = 32 / R2 < R1 ? 32 / R2 : R1;
+  static constexpr int NB = R2 * G;
+  static constexpr int T2 = (R1 / 2) * NQ;  // tasks of the second x stage
+  static constexpr int NT = (T2 + 31) / 32 * 32;
+  static __device__ __forceinline__ int wrap(int x) { return x < LX ? x : x - LX; }
+  static_assert(R1 % 2 == 0 && (R2 / 2) % W == 0 && 32 % R2 == 0 && LYC % (2 * W) == 0 && ct_nst(MC) == 2 && ct_nst(LYC) == 2, "");
+};
+template <typename T, int MC, int LYC>
+constexpr int xy_threads() {
+  if constexpr (MC > 0) return XyCT<T, MC, LYC>::NT;
+  else return kXYThreads;
+}
+template <typename T, int MC, int LYC>
+constexpr int xy_min_blocks() {
+  if constexpr (MC > 0) return 512 / XyCT<T, MC, LYC>::NT;
+  else return sizeof(T) == 4 ? 2 : 1;
+}
+
+// Real fields of a plane as the lanes and parts of a group (row offsets in
+// elements of T from the group's first row).
+template <typename T, int NQ, int LX>
+__device__ __forceinline__ CV<T> group_ld(const T* p) {
+  return CV<T>{vpack(p[0], sizeof(T) == 4 ? p[2 * NQ * LX] : (T)0),
+               vpack(p[NQ * LX], sizeof(T) == 4 ? p[3 * NQ * LX] : (T)0)};
+}
+template <int L, int NQ, int LX, typename T>
+__device__ __forceinline__ void group_st(T* p, const CV<T>& v) {
+  p[2 * L * NQ * LX] = vget<L>(v.re);
+  p[(2 * L + 1) * NQ * LX] = vget<L>(v.im);
+}
+
+// The second x stage pairs class a (k = a + R1 t) with class R1 - a; class 0
+// and class R1/2 pair with themselves and share a task.  For that task this
+// moves the partners to where the other tasks have them: the upper half of
+// v1 becomes the partners of class 0's lower half (with Z(Lx/2) in the last
+// place, opposite Z(0)), the upper half of v0 those of class R1/2.
+template <typename T, int R2>
+__device__ __forceinline__ void self_partners(CV<T>* v0, CV<T>* v1) {
+  const CV<T> nyq = v0[R2 / 2];
+#pragma unroll
+  for (int s = R2 / 2; s < R2; ++s) {
+    const CV<T> p = s + 1 < R2 ? v0[s + 1 < R2 ? s + 1 : 0] : nyq;
+    v0[s] = v1[s];
+    v1[s] = p;
+  }
+}
+template <typename T, int R2>
+__device__ __forceinline__ void self_partners_undo(CV<T>* v0, CV<T>* v1) {
+  CV<T> up[R2 / 2];
+#pragma unroll
+  for (int s = R2 / 2; s < R2; ++s) up[s - R2 / 2] = v1[s];
+#pragma unroll
+  for (int s = R2 / 2; s < R2; ++s) v1[s] = v0[s];
+#pragma unroll
+  for (int s = R2 / 2; s + 1 < R2; ++s) v0[s + 1] = up[s - R2 / 2];
+  v0[R2 / 2] = up[R2 / 2 - 1];
+}
+
+// Lane L of group q: the columns t and t+1 (one W-wide element; W = 1: column
+// t) of rows h = 0, 1 from Z(k) = A and Z(-k) = B, already halved:
+// X0 = Z(k) + conj Z(-k), X1 = -i (Z(k) - conj Z(-k)).  dc: A, B hold Z(0) and
+// Z(Lx/2); the column is X(0) + i X(Lx/2).
+template <int L, typename T>
+__device__ __forceinline__ void unpack_rows(const CV<T>& A, const CV<T>& B, bool dc, T* x0, T* x1) {
+  const T ar = vget<L>(A.re), ai = vget<L>(A.im), br = vget<L>(B.re), bi = vget<L>(B.im);
+  if (dc) {
+    x0[0] = ar + ar;
+    x0[1] = br + br;
+    x1[0] = ai + ai;
+    x1[1] = bi + bi;
+  } else {
+    x0[0] = ar + br;
+    x0[1] = ai - bi;
+    x1[0] = ai + bi;
+    x1[1] = br - ar;
+  }
+}
+// and back: Z(k) = X0 + i X1, Z(-k) = conj X0 + i conj X1.
+template <typename T>
+__device__ __forceinline__ void pack_rows(const T* x0, const T* x1, bool dc, T* z, T* zm) {
+  if (dc) {
+    z[0] = x0[0];
+    z[1] = x1[0];
+    zm[0] = x0[1];
+    zm[1] = x1[1];
+  } else {
+    z[0] = x0[0] - x1[1];
+    z[1] = x0[1] + x1[0];
+    zm[0] = x0[0] + x1[1];
+    zm[1] = x1[0] - x0[1];
   }
 }
 
+// Stores / loads of the columns of one class (R2/2 columns from slot0) of
+// group q in the [j][y] layout.
+template <typename T, int MC, int LYC, int L>
+__device__ __forceinline__ void class_to_columns(CV<T>* buf, const CV<T>* lo, const CV<T>* up, int slot0, int q, bool dc0) {
+  using C = XyCT<T, MC, LYC>;
+  constexpr int H = C::R2 / 2, W = C::W;
+#pragma unroll
+  for (int t = 0; t < H; t += W) {
+    T a0[2], a1[2], b0[2], b1[2];
+    unpack_rows<L>(lo[t], up[C::R2 - 1 - t], dc0 && t == 0, a0, a1);
+    if (W == 2) unpack_rows<L>(lo[t + W - 1], up[C::R2 - t - W], false, b0, b1);
+    CV<T>* d = buf + (slot0 + t) / W * C::JS + q + 2 * L * C::NQ;
+    cv_st(d, CV<T>{vpack(a0[0], W == 2 ? b0[0] : (T)0), vpack(a0[1], W == 2 ? b0[1] : (T)0)});
+    cv_st(d + C::NQ, CV<T>{vpack(a1[0], W == 2 ? b1[0] : (T)0), vpack(a1[1], W == 2 ? b1[1] : (T)0)});
+  }
+}
+template <typename T, int MC, int LYC>
+__device__ __forceinline__ void columns_to_class(const CV<T>* buf, CV<T>* lo, CV<T>* up, int slot0, int q, bool dc0) {
+  using C = XyCT<T, MC, LYC>;
+  constexpr int H = C::R2 / 2, W = C::W;
+#pragma unroll
+  for (int t = 0; t < H; t += W) {
+    const CV<T>* d = buf + (slot0 + t) / W * C::JS + q;
+    CV<T> x[2 * W];  // rows h + 2 l
+#pragma unroll
+    for (int r = 0; r < 2 * W; ++r) x[r] = cv_ld(d + r * C::NQ);
+    T z[W][W][2], zm[W][W][2];  // [column][lane]
+#pragma unroll
+    for (int l = 0; l < W; ++l) {
+      {
+        const T x0[2] = {vget<0>(x[2 * l].re), vget<0>(x[2 * l].im)}, x1[2] = {vget<0>(x[2 * l + 1].re), vget<0>(x[2 * l + 1].im)};
+        pack_rows(x0, x1, dc0 && t == 0, z[0][l], zm[0][l]);
+      }
+      if (W == 2) {
+        const T x0[2] = {vget<1>(x[2 * l].re), vget<1>(x[2 * l].im)}, x1[2] = {vget<1>(x[2 * l + 1].re), vget<1>(x[2 * l + 1].im)};
+        pack_rows(x0, x1, false, z[W - 1][l], zm[W - 1][l]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      lo[t + k] = CV<T>{vpack(z[k][0][0], z[k][W - 1][0]), vpack(z[k][0][1], z[k][W - 1][1])};
+      up[C::R2 - 1 - t - k] = CV<T>{vpack(zm[k][0][0], zm[k][W - 1][0]), vpack(zm[k][0][1], zm[k][W - 1][1])};
+    }
+  }
+}
+
+// Forward transform of one plane: pa (and, for products, pb) the real rows,
+// dst the plane's spectrum rows.  128^2 FP32: 256 threads, 2 CTAs per SM.
+enum { PLANE_PLAIN = 0, PLANE_SQUARE = 1, PLANE_PRODUCT = 2 };
+template <typename T, int MC, int LYC>
+__device__ __forceinline__ void xy_fwd_ct(const T* __restrict__ pa, const T* __restrict__ pb, int kind,
+                                          cplx<T>* __restrict__ dst, int kxp, unsigned char* smem,
+                                          const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twy,
+                                          const int* __restrict__ posm) {
+  using C = XyCT<T, MC, LYC>;
+  constexpr int NT = C::NT, R1 = C::R1, R2 = C::R2, RY1 = C::RY1, RY2 = C::RY2, W = C::W;
+  CV<T>* buf = reinterpret_cast<CV<T>*>(smem);
+  __shared__ cplx<T> tabx[R1 * C::NB], taby[LYC], col0[LYC];
+  stage_twiddles<T, C::LX, R1, C::NB>(tabx, twx, (T)0.5);  // halved: see unpack_rows
+  stage_twiddles<T, LYC, RY1, RY2>(taby, twy, (T)1);
+  __syncthreads();
+  // first x stage, from the real rows
+  lane_tasks<C::NQ * R2, NT>((int)threadIdx.x, [&](int t) {
+    const int b = t % R2, q = t / R2, bg = b + R2 * (q % C::G);
+    const T* r = pa + q * C::LX;
+    CV<T> v[R1];
+#pragma unroll
+    for (int s = 0; s < R1; ++s) v[s] = group_ld<T, C::NQ, C::LX>(r + C::wrap(bg + s * R2));
+    if (kind == PLANE_PRODUCT) {
+      const T* r2 = pb + q * C::LX;
+#pragma unroll
+      for (int s = 0; s < R1; ++s) {
+        const CV<T> w = group_ld<T, C::NQ, C::LX>(r2 + C::wrap(bg + s * R2));
+        v[s] = CV<T>{vmul(v[s].re, w.re), vmul(v[s].im, w.im)};
+      }
+    } else if (kind == PLANE_SQUARE) {
+#pragma unroll
+      for (int s = 0; s < R1; ++s) v[s] = CV<T>{vmul(v[s].re, v[s].re), vmul(v[s].im, v[s].im)};
+    }
+    DftV<T, R1, false>::run(v);
+    CV<T>* d = buf + q * C::QS + b;
+    const lane_t<T> half = vall((T)0.5);
+    cv_st(d, CV<T>{vmul(v[0].re, half), vmul(v[0].im, half)});
+#pragma unroll
+    for (int s = 1; s < R1; ++s) cv_st(d + s * R2, cvtw<T, false>(v[s], tabx[s * C::NB + bg]));
+  });
+  __syncthreads();
+  // second x stage with the separation of the rows
+  {
+    const bool on = threadIdx.x < C::T2;
+    const int q = threadIdx.x % C::NQ, al = on ? threadIdx.x / C::NQ : 0;
+    const int a1 = al == 0 ? R1 / 2 : R1 - al;
+    CV<T> v0[R2], v1[R2];
+    if (on) {
+      const CV<T>* r = buf + q * C::QS;
+#pragma unroll
+      for (int t = 0; t < R2; ++t) v0[t] = cv_ld(r + al * R2 + t);
+#pragma unroll
+      for (int t = 0; t < R2; ++t) v1[t] = cv_ld(r + a1 * R2 + t);
+      DftV<T, R2, false>::run(v0);
+      DftV<T, R2, false>::run(v1);
+      if (al == 0) self_partners<T, R2>(v0, v1);
+    }
+    __syncthreads();
+    if (on) {
+      class_to_columns<T, MC, LYC, 0>(buf, v0, v1, al * (R2 / 2), q, al == 0);
+      class_to_columns<T, MC, LYC, 0>(buf, v1, v0, a1 * (R2 / 2), q, false);
+      if constexpr (W == 2) {
+        class_to_columns<T, MC, LYC, 1>(buf, v0, v1, al * (R2 / 2), q, al == 0);
+        class_to_columns<T, MC, LYC, 1>(buf, v1, v0, a1 * (R2 / 2), q, false);
+      }
+    }
+  }
+  __syncthreads();
+  // first y stage
+  lane_tasks<C::NJ * RY2, NT>((int)threadIdx.x, [&](int t) {
+    const int j = t % C::NJ, b = t / C::NJ;
+    CV<T>* d = buf + j * C::JS + b;
+    CV<T> v[RY1];
+#pragma unroll
+    for (int s = 0; s < RY1; ++s) v[s] = cv_ld(d + s * RY2);
+    DftV<T, RY1, false>::run(v);
+    cv_st(d, v[0]);
+#pragma unroll
+    for (int s = 1; s < RY1; ++s) cv_st(d + s * RY2, cvtw<T, false>(v[s], taby[s * RY2 + b]));
+  });
+  __syncthreads();
+  // second y stage, to the spectrum rows; column 0 to shared memory first
+  lane_tasks<C::NJ * RY1, NT>((int)threadIdx.x, [&](int t) {
+    const int j = t % C::NJ, a = t / C::NJ;
+    const CV<T>* d = buf + j * C::JS + a * RY2;
+    CV<T> v[RY2];
+#pragma unroll
+    for (int s = 0; s < RY2; ++s) v[s] = cv_ld(d + s);
+    DftV<T, RY2, false>::run(v);
+    cplx<T>* o = dst + (long long)(a * RY2) * kxp + W * j;
+    if (j == 0) {
+#pragma unroll
+      for (int s = 0; s < RY2; ++s) {
+        col0[a * RY2 + s] = mk<cplx<T>>(vget<0>(v[s].re), vget<0>(v[s].im));
+        if constexpr (W == 2) o[(long long)s * kxp + 1] = mk<cplx<T>>(vget<1>(v[s].re), vget<1>(v[s].im));
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < RY2; ++s) cv_row(reinterpret_cast<rowvec<T>*>(o + (long long)s * kxp), v[s]);
+    }
+  });
+  __syncthreads();
+  const int *revy = posm + MC, *posy = posm + MC + LYC;
+  for (int sl = threadIdx.x; sl < LYC; sl += NT) {
+    const int sp = __ldg(&posy[(LYC - __ldg(&revy[sl])) % LYC]);
+    cplx<T> y0, ym;
+    y_split(col0[sl], col0[sp], y0, ym);
+    dst[(long long)sl * kxp] = y0;
+    dst[(long long)sl * kxp + MC] = ym;
+  }
+}
+
+// Inverse transform of one plane: src its spectrum rows (consumed: evict
+// first), out its real rows.
+template <typename T, int MC, int LYC>
+__device__ __forceinline__ void xy_inv_ct(const cplx<T>* __restrict__ src, T* __restrict__ out, int kxp,
+                                          unsigned char* smem, const cplx<T>* __restrict__ twx,
+                                          const cplx<T>* __restrict__ twy, const int* __restrict__ posm) {
+  using C = XyCT<T, MC, LYC>;
+  constexpr int NT = C::NT, R1 = C::R1, R2 = C::R2, RY1 = C::RY1, RY2 = C::RY2, W = C::W;
+  CV<T>* buf = reinterpret_cast<CV<T>*>(smem);
+  __shared__ cplx<T> tabx[R1 * C::NB], taby[LYC], col0[LYC];
+  const unsigned long long pol = l2_evict_first();
+  auto ldc = [&](const cplx<T>* a) {
+    if constexpr (sizeof(T) == 4 || FG_L2_HINT_FP64) return ld_first(a, pol);
+    else return *a;
+  };
+  // columns 0 and Lx/2 joined (y_join)
+  const int *revy = posm + MC, *posy = posm + MC + LYC;
+  for (int sl = threadIdx.x; sl < LYC; sl += NT) {
+    const int sp = __ldg(&posy[(LYC - __ldg(&revy[sl])) % LYC]);
+    const cplx<T>*r = src + (long long)sl * kxp, *rm = src + (long long)sp * kxp;
+    col0[sl] = y_join(ldc(r), ldc(rm), ldc(r + MC), ldc(rm + MC));
+  }
+  stage_twiddles<T, C::LX, R1, C::NB>(tabx, twx, (T)1);
+  stage_twiddles<T, LYC, RY1, RY2>(taby, twy, (T)1);
+  __syncthreads();
+  // y: the last forward stage (no twiddles) from the spectrum rows
+  lane_tasks<C::NJ * RY1, NT>((int)threadIdx.x, [&](int t) {
+    const int j = t % C::NJ, a = t / C::NJ;
+    const cplx<T>* r = src + (long long)(a * RY2) * kxp + W * j;
+    CV<T> v[RY2];
+#pragma unroll
+    for (int s = 0; s < RY2; ++s) {
+      if constexpr (sizeof(T) == 4) v[s] = cv_of(ld_first(reinterpret_cast<const float4*>(r + (long long)s * kxp), pol));
+      else v[s] = cv_of(ldc(r + (long long)s * kxp));
+    }
+    if (j == 0) {
+#pragma unroll
+      for (int s = 0; s < RY2; ++s) {
+        const cplx<T> c = col0[a * RY2 + s];
+        if constexpr (W == 2) v[s] = CV<T>{vpack(c.x, vget<1>(v[s].re)), vpack(c.y, vget<1>(v[s].im))};
+        else v[s] = CV<T>{vpack(c.x, c.x), vpack(c.y, c.y)};
+      }
+    }
+    DftV<T, RY2, true>::run(v);
+    CV<T>* d = buf + j * C::JS + a * RY2;
+#pragma unroll
+    for (int s = 0; s < RY2; ++s) cv_st(d + s, v[s]);
+  });
+  __syncthreads();
+  lane_tasks<C::NJ * RY2, NT>((int)threadIdx.x, [&](int t) {
+    const int j = t % C::NJ, b = t / C::NJ;
+    CV<T>* d = buf + j * C::JS + b;
+    CV<T> v[RY1];
+    v[0] = cv_ld(d);
+#pragma unroll
+    for (int s = 1; s < RY1; ++s) v[s] = cvtw<T, true>(cv_ld(d + s * RY2), taby[s * RY2 + b]);
+    DftV<T, RY1, true>::run(v);
+#pragma unroll
+    for (int s = 0; s < RY1; ++s) cv_st(d + s * RY2, v[s]);
+  });
+  __syncthreads();
+  // x: rows joined in pairs, the last forward stage
+  {
+    const bool on = threadIdx.x < C::T2;
+    const int q = threadIdx.x % C::NQ, al = on ? threadIdx.x / C::NQ : 0;
+    const int a1 = al == 0 ? R1 / 2 : R1 - al;
+    CV<T> v0[R2], v1[R2];
+    if (on) {
+      columns_to_class<T, MC, LYC>(buf, v0, v1, al * (R2 / 2), q, al == 0);
+      columns_to_class<T, MC, LYC>(buf, v1, v0, a1 * (R2 / 2), q, false);
+      if (al == 0) self_partners_undo<T, R2>(v0, v1);
+      DftV<T, R2, true>::run(v0);
+      DftV<T, R2, true>::run(v1);
+    }
+    __syncthreads();
+    if (on) {
+      CV<T>* r = buf + q * C::QS;
+#pragma unroll
+      for (int t = 0; t < R2; ++t) cv_st(r + al * R2 + t, v0[t]);
+#pragma unroll
+      for (int t = 0; t < R2; ++t) cv_st(r + a1 * R2 + t, v1[t]);
+    }
+  }
+  __syncthreads();
+  lane_tasks<C::NQ * R2, NT>((int)threadIdx.x, [&](int t) {
+    const int b = t % R2, q = t / R2, bg = b + R2 * (q % C::G);
+    const CV<T>* d = buf + q * C::QS + b;
+    CV<T> v[R1];
+    v[0] = cv_ld(d);
+#pragma unroll
+    for (int s = 1; s < R1; ++s) v[s] = cvtw<T, true>(cv_ld(d + s * R2), tabx[s * C::NB + bg]);
+    DftV<T, R1, true>::run(v);
+    T* r = out + q * C::LX;
+#pragma unroll
+    for (int s = 0; s < R1; ++s) {
+      const int x = C::wrap(bg + s * R2);
+      group_st<0, C::NQ, C::LX>(r + x, v[s]);
+      if constexpr (W == 2) group_st<1, C::NQ, C::LX>(r + x, v[s]);
+    }
+  });
+}
+
 template <typename T, int MODE, int MC = 0, int LYC = 0>
-__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_xy_fwd(const T* __restrict__ src, cplx<T>* __restrict__ spec, Geom g,
-                                                FftPlan px, FftPlan py, const cplx<T>* __restrict__ twx,
-                                                const cplx<T>* __restrict__ twm, const cplx<T>* __restrict__ twy,
-                                                const int* __restrict__ posm, int out_comp0,
-                                                const T* __restrict__ zstar = nullptr, int zu0 = 0,
-                                                const RepArgs* __restrict__ grp = nullptr) {
+__global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC, LYC>())
+    k_xy_fwd(const T* __restrict__ src, cplx<T>* __restrict__ spec, Geom g, FftPlan px, FftPlan py,
+             const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twm, const cplx<T>* __restrict__ twy,
+             const int* __restrict__ posm, int out_comp0, const T* __restrict__ zstar = nullptr, int zu0 = 0,
+             const RepArgs* __restrict__ grp = nullptr) {
   pdl_enter();
   if (grp) {
     src = (const T*)grp[blockIdx.z].u;
     spec = (cplx<T>*)grp[blockIdx.z].spec;
   }
   FG_DYN_SMEM(smem_raw);
-  cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
-  __shared__ cplx<T> tws_m[MC > 0 ? MC : 1], tws_y[LYC > 0 ? LYC : 1], tws_x[MC > 0 ? MC + 1 : 1];
   using T2 = typename RT2<T>::type;
   const int z = blockIdx.x, c = blockIdx.y;
-  const int m = MC > 0 ? MC : g.m, Ly = LYC > 0 ? LYC : g.Ly;
-  const int RS = m + 1, Lx = 2 * m;
-  const int buf_len = Ly * RS;
-  xy_twiddles_to_smem<T, MC, LYC>(tws_m, tws_y, tws_x, twm, twy, twx);
-  const cplx<T>* twx_u = MC > 0 ? tws_x : twx;
   const long long plane_off = (long long)z * g.plane_r;
-  const int total = Ly * m;
-  const bool zu = MODE == SRC_U9 && zstar != nullptr && c >= zu0;  // Z*(R) u_(c - zu0)
+  // what component c is: Z*(R) u_(c - zu0), a plain field, or u_ca u_cb
+  const bool zu = MODE == SRC_U9 && zstar != nullptr && c >= zu0;
+  const bool plain = !zu && (MODE == SRC_FIELD || c < 3 || c >= 9);
+  const int ca = zu ? c - zu0
+                    : plain ? (c >= 9 && MODE == SRC_U9 ? c - 6 : c) : (c == 3 || c == 8) ? 0 : (c == 4 || c == 6) ? 1 : 2;
+  const int cb = (c == 3) ? 0 : (c == 4) ? 1 : (c == 5) ? 2 : (c == 6) ? 2 : (c == 7) ? 0 : 1;
+  const T* pa = src + (long long)ca * g.nsite + plane_off;
+  const T* pb = zu ? zstar + plane_off : src + (long long)cb * g.nsite + plane_off;
+  cplx<T>* dst = spec + (long long)(out_comp0 + c) * g.ncplx + (long long)z * g.plane_c;
   if constexpr (MC > 0) {
-    // First x stage straight from the real rows (packed (x even, x odd)
-    // pairs, products formed on load), then the rest of the x pass.
-    const bool plain = !zu && (MODE == SRC_FIELD || c < 3 || c >= 9);
-    const int ca = zu ? c - zu0
-                      : plain ? (c >= 9 && MODE == SRC_U9 ? c - 6 : c) : (c == 3 || c == 8) ? 0 : (c == 4 || c == 6) ? 1 : 2;
-    const int cb = plain || zu ? -1 : (c == 3) ? 0 : (c == 4) ? 1 : (c == 5) ? 2 : (c == 6) ? 2 : (c == 7) ? 0 : 1;
-    const T* pa = src + (long long)ca * g.nsite + plane_off;
-    const T* pb = zu ? zstar + plane_off : src + (long long)(cb < 0 ? ca : cb) * g.nsite + plane_off;
-    auto st = [&](int y, int e, const cplx<T>& v) { buf[y * (MC + 1) + e] = v; };
-    if (plain) {
-      auto ld = [&](int y, int e) {
-        const T2 a = *reinterpret_cast<const T2*>(pa + (long long)y * (2 * MC) + 2 * e);
-        return mk<cplx<T>>(a.x, a.y);
-      };
-      ct_stage_io<T, MC, 0, false, kXYThreads, LYC, true>(ld, st, twm);
-    } else {
-      auto ld = [&](int y, int e) {
-        const long long o = (long long)y * (2 * MC) + 2 * e;
-        const T2 a = *reinterpret_cast<const T2*>(pa + o), b = *reinterpret_cast<const T2*>(pb + o);
-        return mk<cplx<T>>(a.x * b.x, a.y * b.y);
-      };
-      ct_stage_io<T, MC, 0, false, kXYThreads, LYC, true>(ld, st, twm);
-    }
-    __syncthreads();
-    ct_forward_range<T, MC, 1, ct_nst(MC), kXYThreads, BatchCT<LYC, 1, 0, MC + 1, 1>>(buf, tws_m);
-  } else if (!zu && (MODE == SRC_FIELD || c < 3 || c >= 9)) {
-    // plain component: asynchronous copies of packed (x even, x odd) pairs
-    const T* sp = src + (long long)(c >= 9 && MODE == SRC_U9 ? c - 6 : c) * g.nsite + plane_off;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-      const int y = idx / m, jx = idx - y * m;
-      cp_async<(int)sizeof(cplx<T>)>(&buf[y * RS + jx], sp + (long long)y * Lx + 2 * jx);
-    }
-    cp_async_wait();
+    const int kind = plain ? PLANE_PLAIN : (!zu && c < 6) ? PLANE_SQUARE : PLANE_PRODUCT;
+    xy_fwd_ct<T, MC, LYC>(pa, pb, kind, dst, g.KXP, smem_raw, twx, twy, posm);
   } else {
-    // products: kLB independent loads in flight per thread, then compute
-    constexpr int kLB = 4;
-    for (int base = threadIdx.x; base < total; base += kLB * blockDim.x) {
-      T2 va[kLB], vb[kLB];
-#pragma unroll
-      for (int r = 0; r < kLB; ++r) {
-        const int idx = base + r * blockDim.x;
-        if (idx < total) {
-          const int y = idx / m, jx = idx - y * m;
-          const long long o = plane_off + (long long)y * Lx + 2 * jx;
-          const int ca = zu ? c - zu0 : (c == 3 || c == 8) ? 0 : (c == 4 || c == 6) ? 1 : 2;
-          const int cb = (c == 3) ? 0 : (c == 4) ? 1 : (c == 5) ? 2 : (c == 6) ? 2 : (c == 7) ? 0 : 1;
-          va[r] = *reinterpret_cast<const T2*>(src + (long long)ca * g.nsite + o);
-          vb[r] = *reinterpret_cast<const T2*>(zu ? zstar + o : src + (long long)cb * g.nsite + o);
-        }
+    cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
+    const int m = g.m, Ly = g.Ly, RS = m + 1, Lx = 2 * m;
+    const int buf_len = Ly * RS;
+    const int total = Ly * m;
+    if (plain) {
+      // asynchronous copies of packed (x even, x odd) pairs
+      for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+        const int y = idx / m, jx = idx - y * m;
+        cp_async<(int)sizeof(cplx<T>)>(&buf[y * RS + jx], pa + (long long)y * Lx + 2 * jx);
       }
+      cp_async_wait();
+    } else {
+      // products: kLB independent loads in flight per thread, then compute
+      constexpr int kLB = 4;
+      for (int base = threadIdx.x; base < total; base += kLB * blockDim.x) {
+        T2 va[kLB], vb[kLB];
 #pragma unroll
-      for (int r = 0; r < kLB; ++r) {
-        const int idx = base + r * blockDim.x;
-        if (idx < total) {
-          const int y = idx / m, jx = idx - y * m;
-          buf[y * RS + jx] = mk<cplx<T>>(va[r].x * vb[r].x, va[r].y * vb[r].y);
+        for (int r = 0; r < kLB; ++r) {
+          const int idx = base + r * blockDim.x;
+          if (idx < total) {
+            const int y = idx / m, jx = idx - y * m;
+            const long long o = (long long)y * Lx + 2 * jx;
+            va[r] = *reinterpret_cast<const T2*>(pa + o);
+            vb[r] = *reinterpret_cast<const T2*>(pb + o);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < kLB; ++r) {
+          const int idx = base + r * blockDim.x;
+          if (idx < total) {
+            const int y = idx / m, jx = idx - y * m;
+            buf[y * RS + jx] = mk<cplx<T>>(va[r].x * vb[r].x, va[r].y * vb[r].y);
+          }
         }
       }
     }
-  }
-  // X pass; row stride RS = m+1 keeps the row-interleaved mapping bank-conflict free
-  if constexpr (MC == 0) {
+    // X pass; row stride RS = m+1 keeps the row-interleaved mapping bank-conflict free
     __syncthreads();
     Batch B{Ly, 1, 0, RS, 1, true};
     fft_forward<T>(buf, B, px, twm, buf_len);
-  }
-  // unpack: slot posm[k] holds Z(k) of the packed row; X(k) = E(k) + w^k O(k)
-  const int half = m / 2 + 1;
-  // lanes run along y (same k): conflict-free rows, uniform posm and twiddle
-  for (int idx = threadIdx.x; idx < Ly * half; idx += blockDim.x) {
-    const int k = idx / Ly, y = idx - k * Ly;
-    cplx<T>* row = buf + y * RS;
-    if (k == 0) {
-      const cplx<T> z0 = row[0];
-      if constexpr (MC > 0) {
-        row[0] = mk<cplx<T>>(z0.x + z0.y, z0.x - z0.y);  // X(0) + i X(m)
-      } else {
+    // unpack: slot posm[k] holds Z(k) of the packed row; X(k) = E(k) + w^k O(k)
+    const int half = m / 2 + 1;
+    // lanes run along y (same k): conflict-free rows, uniform posm and twiddle
+    for (int idx = threadIdx.x; idx < Ly * half; idx += blockDim.x) {
+      const int k = idx / Ly, y = idx - k * Ly;
+      cplx<T>* row = buf + y * RS;
+      if (k == 0) {
+        const cplx<T> z0 = row[0];
         row[0] = mk<cplx<T>>(z0.x + z0.y, (T)0);
         row[m] = mk<cplx<T>>(z0.x - z0.y, (T)0);
+      } else {
+        const int k2 = m - k;
+        const int s1 = __ldg(&posm[k]), s2 = __ldg(&posm[k2]);
+        const cplx<T> a = row[s1], b = row[s2];
+        const cplx<T> w1 = twx[k], w2 = twx[k2];
+        // X(k) = 1/2 (a + conj b) - i/2 w1 (a - conj b)
+        const cplx<T> e1 = mk<cplx<T>>(a.x + b.x, a.y - b.y), d1 = mk<cplx<T>>(a.x - b.x, a.y + b.y);
+        const cplx<T> wd1 = cmul(w1, d1);
+        const cplx<T> X1 = mk<cplx<T>>((T)0.5 * (e1.x + wd1.y), (T)0.5 * (e1.y - wd1.x));
+        const cplx<T> e2 = mk<cplx<T>>(b.x + a.x, b.y - a.y), d2 = mk<cplx<T>>(b.x - a.x, b.y + a.y);
+        const cplx<T> wd2 = cmul(w2, d2);
+        const cplx<T> X2 = mk<cplx<T>>((T)0.5 * (e2.x + wd2.y), (T)0.5 * (e2.y - wd2.x));
+        row[s1] = X1;
+        if (s2 != s1) row[s2] = X2;
       }
-    } else {
-      const int k2 = m - k;
-      const int s1 = __ldg(&posm[k]), s2 = __ldg(&posm[k2]);
-      const cplx<T> a = row[s1], b = row[s2];
-      const cplx<T> w1 = twx_u[k], w2 = twx_u[k2];
-      // X(k) = 1/2 (a + conj b) - i/2 w1 (a - conj b)
-      const cplx<T> e1 = mk<cplx<T>>(a.x + b.x, a.y - b.y), d1 = mk<cplx<T>>(a.x - b.x, a.y + b.y);
-      const cplx<T> wd1 = cmul(w1, d1);
-      const cplx<T> X1 = mk<cplx<T>>((T)0.5 * (e1.x + wd1.y), (T)0.5 * (e1.y - wd1.x));
-      const cplx<T> e2 = mk<cplx<T>>(b.x + a.x, b.y - a.y), d2 = mk<cplx<T>>(b.x - a.x, b.y + a.y);
-      const cplx<T> wd2 = cmul(w2, d2);
-      const cplx<T> X2 = mk<cplx<T>>((T)0.5 * (e2.x + wd2.y), (T)0.5 * (e2.y - wd2.x));
-      row[s1] = X1;
-      if (s2 != s1) row[s2] = X2;
     }
-  }
-  __syncthreads();
-  cplx<T>* dst = spec + (long long)(out_comp0 + c) * g.ncplx + (long long)z * g.plane_c;
-  if constexpr (MC > 0) {
-    // y pass over the MC columns (kx = Lx/2 rides in column 0); its last
-    // stage writes the spectrum rows directly, except column 0, which stays
-    // in shared memory for the Hermitian split
-    constexpr int NSY = ct_nst(LYC);
-    ct_forward_range<T, LYC, 0, NSY - 1, kXYThreads, BatchCT<MC, MC, 1, 0, MC + 1>>(buf, tws_y);
-    const long long kxp = g.KXP;
-    auto ld = [&](int col, int e) { return buf[col + e * (MC + 1)]; };
-    auto st = [&](int col, int e, const cplx<T>& v) {
-      if (col == 0) buf[e * (MC + 1)] = v;
-      else dst[(long long)e * kxp + col] = v;
-    };
-    ct_stage_io<T, LYC, NSY - 1, false, kXYThreads, MC, false>(ld, st, tws_y);
     __syncthreads();
-    const int* revy = posm + MC;
-    const int* posy = posm + MC + LYC;
-    for (int sl = threadIdx.x; sl < LYC; sl += kXYThreads) {
-      const int ky = __ldg(&revy[sl]);
-      const int sp = __ldg(&posy[(LYC - ky) % LYC]);
-      cplx<T> y0, ym;
-      y_split(buf[sl * (MC + 1)], buf[sp * (MC + 1)], y0, ym);
-      dst[(long long)sl * kxp] = y0;
-      dst[(long long)sl * kxp + MC] = ym;
-    }
-  } else {
-    Batch B{RS, RS, 1, 0, RS, true};
-    fft_forward<T>(buf, B, py, twy, buf_len);
+    Batch By{RS, RS, 1, 0, RS, true};
+    fft_forward<T>(buf, By, py, twy, buf_len);
     for (int idx = threadIdx.x; idx < Ly * RS; idx += blockDim.x) {
       const int y = idx / RS, col = idx - y * RS;
       dst[(long long)y * g.KXP + col] = buf[idx];
@@ -471,13 +789,11 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_xy_fwd(const T*
 // the half-complex convention of the reference's c2r), DIT along x, store
 // the real plane.  Output is unnormalised (Lx*Ly*Lz times the IDFT).
 template <typename T, int MC = 0, int LYC = 0>
-__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_xy_inv(const cplx<T>* __restrict__ spec, T* __restrict__ out, Geom g,
-                                                FftPlan px, FftPlan py, const cplx<T>* __restrict__ twx,
-                                                const cplx<T>* __restrict__ twm, const cplx<T>* __restrict__ twy,
-                                                const int* __restrict__ posm, int in_comp0,
-                                                const Phys* __restrict__ ph, DevScalars* sc,
-                                                const double* __restrict__ part_k, int nblk_k,
-                                                const RepArgs* __restrict__ grp = nullptr) {
+__global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC, LYC>())
+    k_xy_inv(const cplx<T>* __restrict__ spec, T* __restrict__ out, Geom g, FftPlan px, FftPlan py,
+             const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twm, const cplx<T>* __restrict__ twy,
+             const int* __restrict__ posm, int in_comp0, const Phys* __restrict__ ph, DevScalars* sc,
+             const double* __restrict__ part_k, int nblk_k, const RepArgs* __restrict__ grp = nullptr) {
   pdl_enter();
   if (grp) {
     const RepArgs& a = grp[blockIdx.z];
@@ -492,57 +808,16 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_xy_inv(const cp
   // (nothing in this kernel needs them; k_assemble does).
   if (ph != nullptr && blockIdx.x == 0 && blockIdx.y == 0) homo_strain_tail(ph, sc, part_k, nblk_k);
   FG_DYN_SMEM(smem_raw);
-  cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
-  __shared__ cplx<T> tws_m[MC > 0 ? MC : 1], tws_y[LYC > 0 ? LYC : 1], tws_x[MC > 0 ? MC + 1 : 1];
   using T2 = typename RT2<T>::type;
   const int z = blockIdx.x, c = blockIdx.y;
-  const int m = MC > 0 ? MC : g.m, Ly = LYC > 0 ? LYC : g.Ly;
-  const int RS = m + 1, Lx = 2 * m;
-  const int buf_len = Ly * RS;
-  xy_twiddles_to_smem<T, MC, LYC>(tws_m, tws_y, tws_x, twm, twy, twx);
-  const cplx<T>* twx_u = MC > 0 ? tws_x : twx;
   const cplx<T>* srcp = spec + (long long)(in_comp0 + c) * g.ncplx + (long long)z * g.plane_c;
+  T* dst = out + (long long)c * g.nsite + (long long)z * g.plane_r;
   if constexpr (MC > 0) {
-    // y pass; its first stage (the last forward one, no twiddles) reads the
-    // spectrum rows directly
-    constexpr int NSY = ct_nst(LYC);
-    const long long kxp = g.KXP;
-    // the spectrum is consumed here (evict_first)
-    const unsigned long long pol = l2_evict_first();
-    auto ld = [&](int col, int e) {
-      const cplx<T>* a = srcp + (long long)e * kxp + col;
-      if constexpr (sizeof(T) == 4) {
-        const float2 v = ld_first(reinterpret_cast<const float2*>(a), pol);
-        return mk<cplx<T>>(v.x, v.y);
-      } else if constexpr (FG_L2_HINT_FP64) {
-        const double2 v = ld_first(reinterpret_cast<const double2*>(a), pol);
-        return mk<cplx<T>>(v.x, v.y);
-      } else {
-        return *a;
-      }
-    };
-    // column 0 carries the kx = 0 and kx = Lx/2 columns joined (y_join),
-    // formed by LYC threads into shared memory while all threads run the
-    // first stage of columns 1 .. MC-1 straight from the spectrum (the join's
-    // loads overlap that stage); column 0's first stage then runs on the
-    // joined column in place
-    const int* revy = posm + MC;
-    const int* posy = posm + MC + LYC;
-    for (int sl = threadIdx.x; sl < LYC; sl += kXYThreads) {
-      const int sp = __ldg(&posy[(LYC - __ldg(&revy[sl])) % LYC]);
-      buf[sl * (MC + 1)] = y_join(ld(0, sl), ld(0, sp), ld(MC, sl), ld(MC, sp));
-    }
-    auto st = [&](int col, int e, const cplx<T>& v) { buf[col + e * (MC + 1)] = v; };
-    auto ld1 = [&](int t, int e) { return ld(t + 1, e); };
-    auto st1 = [&](int t, int e, const cplx<T>& v) { st(t + 1, e, v); };
-    ct_stage_io<T, LYC, NSY - 1, true, kXYThreads, MC - 1, false>(ld1, st1, tws_y);
-    __syncthreads();
-    auto ld0 = [&](int, int e) { return buf[e * (MC + 1)]; };
-    auto st0 = [&](int, int e, const cplx<T>& v) { st(0, e, v); };
-    ct_stage_io<T, LYC, NSY - 1, true, kXYThreads, 1, false>(ld0, st0, tws_y);
-    __syncthreads();
-    ct_inverse_range<T, LYC, NSY - 2, -1, kXYThreads, BatchCT<MC, MC, 1, 0, MC + 1>>(buf, tws_y);
+    xy_inv_ct<T, MC, LYC>(srcp, dst, g.KXP, smem_raw, twx, twy, posm);
   } else {
+    cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
+    const int m = g.m, Ly = g.Ly, RS = m + 1, Lx = 2 * m;
+    const int buf_len = Ly * RS;
     for (int idx = threadIdx.x; idx < Ly * RS; idx += blockDim.x) {
       const int y = idx / RS, col = idx - y * RS;
       cp_async<(int)sizeof(cplx<T>)>(&buf[idx], srcp + (long long)y * g.KXP + col);
@@ -551,48 +826,33 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_xy_inv(const cp
     __syncthreads();
     Batch B{RS, RS, 1, 0, RS, true};
     fft_inverse<T>(buf, B, py, twy, buf_len);
-  }
-  const int half = m / 2 + 1;
-  // lanes run along y (same k): conflict-free rows, uniform posm and twiddle
-  for (int idx = threadIdx.x; idx < Ly * half; idx += blockDim.x) {
-    const int k = idx / Ly, y = idx - k * Ly;
-    cplx<T>* row = buf + y * RS;
-    if (k == 0) {
-      // compile-time kernels: x(kx = Lx/2) came back as the imaginary part
-      const T X0 = row[0].x, Xm = MC > 0 ? row[0].y : row[m].x;
-      row[0] = mk<cplx<T>>(X0 + Xm, X0 - Xm);
-    } else {
-      const int k2 = m - k;
-      const int s1 = __ldg(&posm[k]), s2 = __ldg(&posm[k2]);
-      const cplx<T> a = row[s1], b = row[s2];
-      const cplx<T> w1 = twx_u[k], w2 = twx_u[k2];
-      // Z(k) = (a + conj b) + i conj(w1) (a - conj b)
-      const cplx<T> e1 = mk<cplx<T>>(a.x + b.x, a.y - b.y), d1 = mk<cplx<T>>(a.x - b.x, a.y + b.y);
-      const cplx<T> wd1 = cmulc(d1, w1);
-      const cplx<T> Z1 = mk<cplx<T>>(e1.x - wd1.y, e1.y + wd1.x);
-      const cplx<T> e2 = mk<cplx<T>>(b.x + a.x, b.y - a.y), d2 = mk<cplx<T>>(b.x - a.x, b.y + a.y);
-      const cplx<T> wd2 = cmulc(d2, w2);
-      const cplx<T> Z2 = mk<cplx<T>>(e2.x - wd2.y, e2.y + wd2.x);
-      row[s1] = Z1;
-      if (s2 != s1) row[s2] = Z2;
+    const int half = m / 2 + 1;
+    // lanes run along y (same k): conflict-free rows, uniform posm and twiddle
+    for (int idx = threadIdx.x; idx < Ly * half; idx += blockDim.x) {
+      const int k = idx / Ly, y = idx - k * Ly;
+      cplx<T>* row = buf + y * RS;
+      if (k == 0) {
+        const T X0 = row[0].x, Xm = row[m].x;
+        row[0] = mk<cplx<T>>(X0 + Xm, X0 - Xm);
+      } else {
+        const int k2 = m - k;
+        const int s1 = __ldg(&posm[k]), s2 = __ldg(&posm[k2]);
+        const cplx<T> a = row[s1], b = row[s2];
+        const cplx<T> w1 = twx[k], w2 = twx[k2];
+        // Z(k) = (a + conj b) + i conj(w1) (a - conj b)
+        const cplx<T> e1 = mk<cplx<T>>(a.x + b.x, a.y - b.y), d1 = mk<cplx<T>>(a.x - b.x, a.y + b.y);
+        const cplx<T> wd1 = cmulc(d1, w1);
+        const cplx<T> Z1 = mk<cplx<T>>(e1.x - wd1.y, e1.y + wd1.x);
+        const cplx<T> e2 = mk<cplx<T>>(b.x + a.x, b.y - a.y), d2 = mk<cplx<T>>(b.x - a.x, b.y + a.y);
+        const cplx<T> wd2 = cmulc(d2, w2);
+        const cplx<T> Z2 = mk<cplx<T>>(e2.x - wd2.y, e2.y + wd2.x);
+        row[s1] = Z1;
+        if (s2 != s1) row[s2] = Z2;
+      }
     }
-  }
-  __syncthreads();
-  T* dst = out + (long long)c * g.nsite + (long long)z * g.plane_r;
-  if constexpr (MC > 0) {
-    // x pass; its last stage (stage 0, DIT) writes the real rows directly
-    ct_inverse_range<T, MC, ct_nst(MC) - 1, 0, kXYThreads, BatchCT<LYC, 1, 0, MC + 1, 1>>(buf, tws_m);
-    auto ld = [&](int y, int e) { return buf[y * (MC + 1) + e]; };
-    auto st = [&](int y, int e, const cplx<T>& v) {
-      T2 w;
-      w.x = v.x;
-      w.y = v.y;
-      *reinterpret_cast<T2*>(dst + (long long)y * (2 * MC) + 2 * e) = w;
-    };
-    ct_stage_io<T, MC, 0, true, kXYThreads, LYC, true>(ld, st, tws_m);
-  } else {
-    Batch B{Ly, 1, 0, RS, 1, true};
-    fft_inverse<T>(buf, B, px, twm, buf_len);
+    __syncthreads();
+    Batch Bx{Ly, 1, 0, RS, 1, true};
+    fft_inverse<T>(buf, Bx, px, twm, buf_len);
     for (int idx = threadIdx.x; idx < Ly * m; idx += blockDim.x) {
       const int y = idx / m, jx = idx - y * m;
       const cplx<T> v = buf[y * RS + jx];
