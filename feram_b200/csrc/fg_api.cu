@@ -135,6 +135,8 @@ struct fg_ctx {
   double2* trz = nullptr;
   double2* trz_s = nullptr;  // trz and kvz in kz-slot order
   double* kvz_s = nullptr;
+  double2 *trx_s = nullptr, *try_s = nullptr;  // the same of x and y
+  double *kvx_s = nullptr, *kvy_s = nullptr;
   double* layer_minv = nullptr;
   unsigned char* layer_sump = nullptr;
   // acoustic-displacement MD (acoustic mass > 0): u, p and F hold three more
@@ -222,7 +224,8 @@ int fail(fg_ctx* c, int code, const std::string& msg) {
 
 template <typename T>
 KMaps kmaps(const fg_ctx* c) {
-  return KMaps{c->revx, c->revy, c->revz, c->kvx, c->kvy, c->kvz, c->trx, c->try_, c->trz, c->trz_s, c->kvz_s};
+  return KMaps{c->revx, c->revy, c->revz, c->kvx, c->kvy, c->kvz, c->trx, c->try_, c->trz, c->trz_s, c->kvz_s,
+               c->trx_s, c->try_s, c->kvx_s, c->kvy_s};
 }
 
 int check_device_error(fg_ctx* ctx) {
@@ -267,28 +270,39 @@ void with_xy_inv(int m, int Ly, F f) {
 }
 template <typename T>
 constexpr int z_cw_cap() { return sizeof(T) == 4 ? 8 : 4; }
+// The k-space pass: f(kernel, shape) with k_z_lane for the compile-time
+// lengths at tiles of 4 or 2 elements (cw = 8, 4 kx slots in FP32, 4, 2 in
+// FP64); false for what k_z_kspace takes (other lengths and widths, per-site
+// Z*).
+template <typename T, int PW, bool ACOU, class F>
+bool with_z_lane_pw(int Lz, F f) {
+  switch (Lz) {
+    case 128: f(k_z_lane<T, 128, PW, ACOU>, ZCT<T, 128, PW, ACOU>()); return true;
+    case 64: f(k_z_lane<T, 64, PW, ACOU>, ZCT<T, 64, PW, ACOU>()); return true;
+    case 48: f(k_z_lane<T, 48, PW, ACOU>, ZCT<T, 48, PW, ACOU>()); return true;
+    case 32: f(k_z_lane<T, 32, PW, ACOU>, ZCT<T, 32, PW, ACOU>()); return true;
+    case 24: f(k_z_lane<T, 24, PW, ACOU>, ZCT<T, 24, PW, ACOU>()); return true;
+    case 16: f(k_z_lane<T, 16, PW, ACOU>, ZCT<T, 16, PW, ACOU>()); return true;
+    default: return false;
+  }
+}
 template <typename T, class F>
-void with_z_kspace(int Lz, int cw, bool acou, bool zsite, F f) {
-  constexpr int C = z_cw_cap<T>();
-  if (zsite) {  // per-site Z*: runtime transforms
-    if (acou) f(k_z_kspace<T, 0, 0, true, true>);
-    else f(k_z_kspace<T, 0, 0, false, true>);
+bool with_z_lane(int Lz, int cw, bool acou, bool zsite, F f) {
+  constexpr int W = kLanes<T>;
+  if (zsite || (cw != 4 * W && cw != 2 * W)) return false;
+  if (acou) return cw == 4 * W ? with_z_lane_pw<T, 4, true>(Lz, f) : with_z_lane_pw<T, 2, true>(Lz, f);
+  return cw == 4 * W ? with_z_lane_pw<T, 4, false>(Lz, f) : with_z_lane_pw<T, 2, false>(Lz, f);
+}
+template <typename T, class F>
+void with_z_kspace(bool acou, bool zsite, F f) {
+  if (zsite) {  // per-site Z*
+    if (acou) f(k_z_kspace<T, true, true>);
+    else f(k_z_kspace<T, false, true>);
   } else if (acou) {
-    if (cw == C && Lz == 128) f(k_z_kspace<T, 128, C, true>);
-    else if (cw == C && Lz == 64) f(k_z_kspace<T, 64, C, true>);
-    else if (cw == C && Lz == 32) f(k_z_kspace<T, 32, C, true>);
-    else if (cw == C && Lz == 16) f(k_z_kspace<T, 16, C, true>);
-    else if (cw == C && Lz == 48) f(k_z_kspace<T, 48, C, true>);
-    else if (cw == 4 && Lz == 24) f(k_z_kspace<T, 24, 4, true>);
-    else f(k_z_kspace<T, 0, 0, true>);
-  } else if (cw == C && Lz == 128) f(k_z_kspace<T, 128, C>);
-  else if (sizeof(T) == 4 && cw == 4 && Lz == 128) f(k_z_kspace<T, 128, 4>);
-  else if (cw == C && Lz == 64) f(k_z_kspace<T, 64, C>);
-  else if (cw == C && Lz == 32) f(k_z_kspace<T, 32, C>);
-  else if (cw == C && Lz == 16) f(k_z_kspace<T, 16, C>);
-  else if (cw == C && Lz == 48) f(k_z_kspace<T, 48, C>);
-  else if (cw == 4 && Lz == 24) f(k_z_kspace<T, 24, 4>);
-  else f(k_z_kspace<T, 0, 0>);
+    f(k_z_kspace<T, true>);
+  } else {
+    f(k_z_kspace<T>);
+  }
 }
 
 // The standalone z pass of the 3-component FFT entry points (fg_fft_r2c3,
@@ -312,7 +326,7 @@ inline int zu_comp(const fg_ctx* ctx) { return ctx->acou ? 12 : 9; }
 
 // Kernel launch that, while ctx->pdl is set, lets the kernel be scheduled
 // before its predecessor on the stream has finished (programmatic stream
-// serialization).  Only kernels that start with pdl_enter() go through it.
+// serialization).  Only kernels that call pdl_wait() go through it.
 template <typename... KArgs, typename... Args>
 void launch_dep(fg_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -366,16 +380,39 @@ int launch_xy_inv(fg_ctx* ctx, const cplx<T>* spec, T* out, int ncomp, bool stra
 }
 
 // The k-space partials are finished by the next k_xy_inv (strain prologue).
+// nrep replicas (grp != null) or the context's own.
 template <typename T>
-int launch_z_kspace(fg_ctx* ctx, cplx<T>* acouK_out) {
+int launch_z_kspace(fg_ctx* ctx, cplx<T>* acouK_out, int nrep = 1, const RepArgs* grp = nullptr) {
   const Geom& g = ctx->g;
-  with_z_kspace<T>(g.Lz, ctx->zt.CW, ctx->acou, ctx->zsite, [&](auto kern) {
-    launch_dep(ctx, kern, ctx->zt.nreg + ctx->zt.nnyq, kThreadsZ, ctx->smem_z,
-        (cplx<T>*)ctx->spec, (const T*)ctx->dtab, (const cplx<T>*)ctx->ckmod, acouK_out, g, ctx->pz,
-        (const cplx<T>*)ctx->twz, kmaps<T>(ctx), ctx->ph, ctx->part_k, ctx->sc, ctx->zt, nullptr,
-        (const T*)ctx->ltab, (const RepArgs*)nullptr);
-  });
+  auto go = [&](auto kern, int nt, int smem) {
+    launch_dep(ctx, kern, dim3(ctx->zt.nreg + ctx->zt.nnyq, nrep), nt, smem, (cplx<T>*)ctx->spec, (const T*)ctx->dtab,
+               (const cplx<T>*)ctx->ckmod, acouK_out, g, ctx->pz, (const cplx<T>*)ctx->twz, kmaps<T>(ctx), ctx->ph,
+               ctx->part_k, ctx->sc, ctx->zt, (const T*)ctx->ltab, grp);
+  };
+  if (!with_z_lane<T>(g.Lz, ctx->zt.CW, ctx->acou, ctx->zsite,
+                      [&](auto kern, auto shape) { go(kern, decltype(shape)::NT, decltype(shape)::SMEM); }))
+    with_z_kspace<T>(ctx->acou, ctx->zsite, [&](auto kern) { go(kern, kZThreads, ctx->smem_z); });
   CKL();
+  return FG_OK;
+}
+
+// Dynamic shared-memory limit of the k-space kernel of tiles zt (smem_z: the
+// runtime kernel's).
+template <typename T>
+int prepare_z(fg_ctx* ctx, const ZTiles& zt, bool zsite, int smem_z, int smem_optin) {
+  cudaError_t ea = cudaSuccess;
+  auto setattr = [&](auto kern, int bytes) {
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+    const int cap = smem_optin - (int)fa.sharedSizeBytes;
+    if (e == cudaSuccess && bytes > cap) e = cudaErrorInvalidValue;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+    if (e != cudaSuccess) ea = e;
+  };
+  if (!with_z_lane<T>(ctx->g.Lz, zt.CW, ctx->acou, zsite,
+                      [&](auto kern, auto shape) { setattr(kern, decltype(shape)::SMEM); }))
+    with_z_kspace<T>(ctx->acou, zsite, [&](auto kern) { setattr(kern, smem_z); });
+  if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
   return FG_OK;
 }
 
@@ -610,13 +647,10 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
                c0->posm, 0, (const T*)nullptr, 0, grp);
   });
   CKL();
-  with_z_kspace<T>(g.Lz, c0->zt.CW, false, false, [&](auto kern) {
-    launch_dep(c0, kern, dim3(c0->zt.nreg + c0->zt.nnyq, nrep), kThreadsZ, c0->smem_z, (cplx<T>*)nullptr,
-               (const T*)nullptr, (const cplx<T>*)c0->ckmod, (cplx<T>*)nullptr, g, c0->pz, (const cplx<T>*)c0->twz,
-               kmaps<T>(c0), (const Phys*)nullptr, (double*)nullptr, (DevScalars*)nullptr, c0->zt,
-               (unsigned int*)nullptr, (const T*)nullptr, grp);
-  });
-  CKL();
+  {
+    const int rc = launch_z_kspace<T>(c0, nullptr, nrep, grp);
+    if (rc) return rc;
+  }
   with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
     launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), nt, c0->smem_xy, (const cplx<T>*)nullptr, (T*)nullptr, g,
                c0->px, c0->py, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm, (const cplx<T>*)c0->twy, c0->posm,
@@ -779,10 +813,17 @@ int validate(const fg_params* p, std::string* why) {
   return FG_OK;
 }
 
-// The widest z tile the context's plan allows.
+// The widest z tile the context's plan allows.  By default 4 elements of 16
+// bytes (64-byte rows), or 2 where that leaves SMs without a tile (32^3 mixed:
+// z pass 14.6 us with 68 tiles, 12.6 with 136) and for acoustic 128-layer
+// supercells, whose wider tiles do not fit the ring (with_z_lane).
 template <typename T>
-int plan_cw(const fg_ctx* ctx) {
-  return ctx->plan_zcw > 0 ? std::min(ctx->plan_zcw, z_cw_cap<T>()) : z_cw_cap<T>();
+int plan_cw(const fg_ctx* ctx, int nsm) {
+  constexpr int cap = z_cw_cap<T>();
+  if (ctx->plan_zcw > 0) return std::min(ctx->plan_zcw, cap);
+  const Geom& g = ctx->g;
+  if (g.m % cap == 0 && g.m / cap * g.Ly < nsm) return cap / 2;
+  return cap;
 }
 
 // z tiles: CW is the largest power of two <= cwmax dividing Lx/2 whose
@@ -849,12 +890,12 @@ int create_impl(fg_ctx* ctx) {
   auto tiles = [&](int nc, size_t esz, int cwmax) { return z_tiles(g, nc, esz, cwmax, smem_max); };
   ctx->acou = P.mass_acou[0] > 0.0;
   ctx->ncx = ctx->acou ? 12 : 9;
-  ctx->zt = tiles(ctx->ncx, sizeof(cplx<T>), plan_cw<T>(ctx));
+  ctx->zt = tiles(ctx->ncx, sizeof(cplx<T>), plan_cw<T>(ctx, nsm));
   ctx->zt6 = tiles(6, sizeof(cplx<double>), 8);
   ctx->zt1 = tiles(1, sizeof(cplx<double>), 8);
   if ((size_t)ctx->ncx * g.Lz * ctx->zt.CW * sizeof(cplx<T>) > (size_t)smem_max)
     return fail(ctx, FG_ERR_UNSUPPORTED, "a z pencil of the supercell does not fit in shared memory");
-  ctx->smem_z = (int)(ctx->ncx * ((size_t)g.Lz * ctx->zt.CW + kZPad<T>) * sizeof(cplx<T>));
+  ctx->smem_z = (int)(ctx->ncx * ((size_t)g.Lz * ctx->zt.CW) * sizeof(cplx<T>));
   ctx->smem_z3 = (int)(3 * (size_t)g.Lz * ctx->zt.CW * sizeof(cplx<T>));
   ctx->smem_z6 = (int)(6 * (size_t)g.Lz * ctx->zt6.CW * sizeof(cplx<double>));
   ctx->smem_z1 = (int)(1 * (size_t)g.Lz * ctx->zt1.CW * sizeof(cplx<double>));
@@ -878,7 +919,6 @@ int create_impl(fg_ctx* ctx) {
     with_xy_fwd<T, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
     with_xy_fwd<double, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy64); });
     with_xy_inv<T>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
-    with_z_kspace<T>(g.Lz, ctx->zt.CW, ctx->acou, false, [&](auto k) { setattr(k, ctx->smem_z); });
     with_z_pass<T, false>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
     with_z_pass<T, true>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
     setattr(k_z_ewald_pack<T>, ctx->smem_z6);
@@ -946,6 +986,19 @@ int create_impl(fg_ctx* ctx) {
       }
       if ((rc = upload(ctx, (void**)&ctx->trz_s, tzs))) return rc;
       if ((rc = upload(ctx, (void**)&ctx->kvz_s, kzs))) return rc;
+      auto in_slots = [](auto& to, const auto& from, const std::vector<int>& rev) {
+        for (int k : rev) to.push_back(from[k]);
+      };
+      std::vector<double2> txs, tys;
+      std::vector<double> kxs, kys;
+      in_slots(txs, trig(g.NKX, P.Lx), ctx->h_revx);
+      in_slots(tys, trig(g.Ly, P.Ly), ctx->h_revy);
+      in_slots(kxs, kx, ctx->h_revx);
+      in_slots(kys, ky, ctx->h_revy);
+      if ((rc = upload(ctx, (void**)&ctx->trx_s, txs))) return rc;
+      if ((rc = upload(ctx, (void**)&ctx->try_s, tys))) return rc;
+      if ((rc = upload(ctx, (void**)&ctx->kvx_s, kxs))) return rc;
+      if ((rc = upload(ctx, (void**)&ctx->kvy_s, kys))) return rc;
     }
   }
   // per-layer masses and masks (alloc_Coord, read_defects_u.F:52-69)
@@ -1077,7 +1130,7 @@ int create_impl(fg_ctx* ctx) {
     CK(cudaMemset(ctx->Flo, 0, 3 * ctx->real_bytes));
   }
   CK(cudaMalloc(&ctx->spec, (size_t)ctx->ncx * sizeof(cplx<T>) * (size_t)g.ncplx));
-  CK(cudaMemset(ctx->spec, 0, 9 * sizeof(cplx<T>) * (size_t)g.ncplx));
+  CK(cudaMemset(ctx->spec, 0, (size_t)ctx->ncx * sizeof(cplx<T>) * (size_t)g.ncplx));
   CK(cudaMalloc(&ctx->rwork, (size_t)ctx->ncx * ctx->real_bytes));
   CK(cudaMalloc(&ctx->dtab, 6 * es * (size_t)g.nkpos));
   CK(cudaMemset(ctx->dtab, 0, 6 * es * (size_t)g.nkpos));
@@ -1086,6 +1139,7 @@ int create_impl(fg_ctx* ctx) {
   CK(cudaMalloc(&ctx->acouK, 3 * sizeof(cplx<T>) * (size_t)g.nkpos));
   CK(cudaMemset(ctx->acouK, 0, 3 * sizeof(cplx<T>) * (size_t)g.nkpos));
   CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(ctx->zt.nreg + ctx->zt.nnyq)));
+  if (const int rc2 = prepare_z<T>(ctx, ctx->zt, false, ctx->smem_z, smem_optin)) return rc2;
   CK(cudaMalloc(&ctx->part_r, sizeof(double) * NQ_R * (size_t)ctx->grid_elem));
   CK(cudaMalloc(&ctx->part_ke, sizeof(double) * 3 * (size_t)ctx->grid_elem));
   CK(cudaMalloc(&ctx->part_avg, sizeof(double) * 6 * (size_t)ctx->grid_elem));
@@ -1187,7 +1241,7 @@ int upload_tables_impl(fg_ctx* ctx, const double* sr, const double* lr) {
           const double l = lr[ftab(ctx, 3, qa[q], qb[q], kx, ky, kz)];
           smax = std::max(smax, std::fabs(s));
           sdiff = std::max(sdiff, std::fabs(s - S[q]));
-          D[tpos * 6 + q] = (T)((s + z2 * l) * P.Ninv);
+          D[(size_t)tab_index<T>((long long)tpos, q)] = (T)((s + z2 * l) * P.Ninv);
           L[tpos * 6 + q] = l;
         }
       }
@@ -1408,21 +1462,14 @@ int set_zsite(fg_ctx* ctx, bool on) {
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const int smem_max = smem_optin - 8192;
+  int nsm = 0;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int ncx = (ctx->acou ? 12 : 9) + (on ? 3 : 0);
-  const ZTiles zt = z_tiles(g, ncx, sizeof(cplx<T>), plan_cw<T>(ctx), smem_max);
+  const ZTiles zt = z_tiles(g, ncx, sizeof(cplx<T>), plan_cw<T>(ctx, nsm), smem_max);
   if ((size_t)ncx * g.Lz * zt.CW * sizeof(cplx<T>) > (size_t)smem_max)
     return fail(ctx, FG_ERR_UNSUPPORTED, "a z pencil of the supercell does not fit in shared memory");
-  const int smem_z = (int)(ncx * ((size_t)g.Lz * zt.CW + kZPad<T>) * sizeof(cplx<T>));
-  cudaError_t ea = cudaSuccess;
-  with_z_kspace<T>(g.Lz, zt.CW, ctx->acou, on, [&](auto kern) {
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, kern);
-    const int cap = smem_optin - (int)fa.sharedSizeBytes;
-    if (e == cudaSuccess && smem_z > cap) e = cudaErrorInvalidValue;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-    ea = e;
-  });
-  if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
+  const int smem_z = (int)(ncx * ((size_t)g.Lz * zt.CW) * sizeof(cplx<T>));
+  if (const int rc = prepare_z<T>(ctx, zt, on, smem_z, smem_optin)) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->broken = true;  // until every buffer below is allocated again
   for (void** b : {&ctx->spec, &ctx->rwork, (void**)&ctx->part_k, &ctx->ltab})
@@ -1687,7 +1734,7 @@ void fg_destroy(fg_ctx* ctx) {
   if (ctx->g_lf) cudaGraphExecDestroy(ctx->g_lf);
   if (ctx->g_vs) cudaGraphExecDestroy(ctx->g_vs);
   if (ctx->g_force) cudaGraphExecDestroy(ctx->g_force);
-  void* bufs[] = {ctx->u, ctx->p, ctx->F, ctx->Flo, ctx->spec, ctx->rwork, ctx->dtab, ctx->ckmod, ctx->acouK, ctx->twx,
+  void* bufs[] = {ctx->trx_s, ctx->try_s, ctx->kvx_s, ctx->kvy_s, ctx->u, ctx->p, ctx->F, ctx->Flo, ctx->spec, ctx->rwork, ctx->dtab, ctx->ckmod, ctx->acouK, ctx->twx,
                   ctx->twm, ctx->twy, ctx->twz, ctx->twx64, ctx->twm64, ctx->twy64, ctx->twz64, ctx->L64, ctx->ltab, ctx->revx,
                   ctx->revy, ctx->revz, ctx->posm, ctx->kvx, ctx->kvy, ctx->kvz, ctx->trx, ctx->try_, ctx->trz, ctx->trz_s, ctx->kvz_s,
                   ctx->layer_minv, ctx->layer_sump, ctx->ph, ctx->sc, ctx->part_k, ctx->part_r, ctx->part_ke,
@@ -2684,11 +2731,14 @@ int apply_plan_t(fg_ctx* ctx, int zcw, int waves) {
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int smem_max = smem_optin - 8192;
-  const int cwmax = zcw > 0 ? std::min(zcw, z_cw_cap<T>()) : z_cw_cap<T>();
+  const int old_zcw = ctx->plan_zcw;
+  ctx->plan_zcw = zcw;
+  const int cwmax = plan_cw<T>(ctx, nsm);
+  ctx->plan_zcw = old_zcw;
   const ZTiles zt = z_tiles(g, ctx->ncx, sizeof(cplx<T>), cwmax, smem_max);
   if ((size_t)ctx->ncx * g.Lz * zt.CW * sizeof(cplx<T>) > (size_t)smem_max)
     return fail(ctx, FG_ERR_UNSUPPORTED, "a z pencil of the supercell does not fit in shared memory");
-  const int smem_z = (int)(ctx->ncx * ((size_t)g.Lz * zt.CW + kZPad<T>) * sizeof(cplx<T>));
+  const int smem_z = (int)(ctx->ncx * ((size_t)g.Lz * zt.CW) * sizeof(cplx<T>));
   const int smem_z3 = (int)(3 * (size_t)g.Lz * zt.CW * sizeof(cplx<T>));
   cudaError_t ea = cudaSuccess;
   auto setattr = [&](auto kern, int bytes) {
@@ -2699,7 +2749,7 @@ int apply_plan_t(fg_ctx* ctx, int zcw, int waves) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     if (e != cudaSuccess) ea = e;
   };
-  with_z_kspace<T>(g.Lz, zt.CW, ctx->acou, ctx->zsite, [&](auto k) { setattr(k, smem_z); });
+  if (const int rc = prepare_z<T>(ctx, zt, ctx->zsite, smem_z, smem_optin)) return rc;
   with_z_pass<T, false>(g.Lz, zt.CW, [&](auto k) { setattr(k, smem_z3); });
   with_z_pass<T, true>(g.Lz, zt.CW, [&](auto k) { setattr(k, smem_z3); });
   if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));

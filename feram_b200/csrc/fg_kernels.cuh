@@ -19,6 +19,8 @@
 #pragma once
 #include "fft_lane.cuh"
 
+#include <type_traits>
+
 namespace fg {
 
 // energy slots, fg_energy member order (energy_module.F:7-23)
@@ -480,6 +482,7 @@ __device__ __forceinline__ void xy_fwd_ct(const T* __restrict__ pa, const T* __r
   stage_twiddles<T, C::LX, R1, C::NB>(tabx, twx, (T)0.5);  // halved: see unpack_rows
   stage_twiddles<T, LYC, RY1, RY2>(taby, twy, (T)1);
   __syncthreads();
+  pdl_wait();
   // first x stage, from the real rows
   lane_tasks<C::NQ * R2, NT>((int)threadIdx.x, [&](int t) {
     const int b = t % R2, q = t / R2, bg = b + R2 * (q % C::G);
@@ -546,6 +549,7 @@ __device__ __forceinline__ void xy_fwd_ct(const T* __restrict__ pa, const T* __r
     for (int s = 1; s < RY1; ++s) cv_st(d + s * RY2, cvtw<T, false>(v[s], taby[s * RY2 + b]));
   });
   __syncthreads();
+  pdl_launch();
   // second y stage, to the spectrum rows; column 0 to shared memory first
   lane_tasks<C::NJ * RY1, NT>((int)threadIdx.x, [&](int t) {
     const int j = t % C::NJ, a = t / C::NJ;
@@ -661,6 +665,7 @@ __device__ __forceinline__ void xy_inv_ct(const cplx<T>* __restrict__ src, T* __
     }
   }
   __syncthreads();
+  pdl_launch();
   lane_tasks<C::NQ * R2, NT>((int)threadIdx.x, [&](int t) {
     const int b = t % R2, q = t / R2, bg = b + R2 * (q % C::G);
     const CV<T>* d = buf + q * C::QS + b;
@@ -685,7 +690,6 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
              const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twm, const cplx<T>* __restrict__ twy,
              const int* __restrict__ posm, int out_comp0, const T* __restrict__ zstar = nullptr, int zu0 = 0,
              const RepArgs* __restrict__ grp = nullptr) {
-  pdl_enter();
   if (grp) {
     src = (const T*)grp[blockIdx.z].u;
     spec = (cplx<T>*)grp[blockIdx.z].spec;
@@ -707,6 +711,7 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
     const int kind = plain ? PLANE_PLAIN : (!zu && c < 6) ? PLANE_SQUARE : PLANE_PRODUCT;
     xy_fwd_ct<T, MC, LYC>(pa, pb, kind, dst, g.KXP, smem_raw, twx, twy, posm);
   } else {
+    pdl_wait();
     cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
     const int m = g.m, Ly = g.Ly, RS = m + 1, Lx = 2 * m;
     const int buf_len = Ly * RS;
@@ -776,6 +781,7 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
     __syncthreads();
     Batch By{RS, RS, 1, 0, RS, true};
     fft_forward<T>(buf, By, py, twy, buf_len);
+    pdl_launch();
     for (int idx = threadIdx.x; idx < Ly * RS; idx += blockDim.x) {
       const int y = idx / RS, col = idx - y * RS;
       dst[(long long)y * g.KXP + col] = buf[idx];
@@ -794,7 +800,7 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
              const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twm, const cplx<T>* __restrict__ twy,
              const int* __restrict__ posm, int in_comp0, const Phys* __restrict__ ph, DevScalars* sc,
              const double* __restrict__ part_k, int nblk_k, const RepArgs* __restrict__ grp = nullptr) {
-  pdl_enter();
+  pdl_wait();
   if (grp) {
     const RepArgs& a = grp[blockIdx.z];
     spec = (const cplx<T>*)a.spec;
@@ -853,6 +859,7 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
     __syncthreads();
     Batch Bx{Ly, 1, 0, RS, 1, true};
     fft_inverse<T>(buf, Bx, px, twm, buf_len);
+    pdl_launch();
     for (int idx = threadIdx.x; idx < Ly * m; idx += blockDim.x) {
       const int y = idx / m, jx = idx - y * m;
       const cplx<T> v = buf[y * RS + jx];
@@ -925,6 +932,15 @@ __device__ __forceinline__ void z_tile_store(const cplx<T>* buf, cplx<T>* __rest
     const int c = r / Lz, z = r - c * Lz;
     base[(long long)c * g.ncplx + (long long)z * g.plane_c] = buf[r * CW + cw];
   }
+}
+
+// Value q of the dipole table at position pos = (ky slot, kz slot, kx slot):
+// the 6 values of W neighbouring kx slots interleaved, [pos / W][6][W], as the
+// elements of k_z_lane read them (KXP is even).
+template <typename T>
+__host__ __device__ __forceinline__ long long tab_index(long long pos, int q) {
+  constexpr int W = 16 / (2 * (int)sizeof(T));
+  return (pos & ~(long long)(W - 1)) * 6 + q * W + (pos & (W - 1));
 }
 
 // ------------------------------------------------------------ scalar kernels
@@ -1162,6 +1178,10 @@ struct KMaps {
   const double2* trz;
   const double2* trz_s;  // trz and kvz in kz-slot order (no revz lookup first)
   const double* kvz_s;
+  const double2* trx_s;  // the same of x (slots 0 .. Lx/2) and y
+  const double2* try_s;
+  const double* kvx_s;
+  const double* kvy_s;
 };
 
 // Plain z pass of nc spectra in place: DIF (INV = false) or DIT (INV = true).
@@ -1202,26 +1222,16 @@ __global__ void __launch_bounds__(256) k_z_pass(cplx<T>* __restrict__ spec, Geom
 // ZSC (per-site Z*, dVddi-dipole-dipole.F:20-60): slots Z0..Z0+2 carry
 // FFT(Z*(R) u) in and the long-range part (L/N) FFT(Z* u) out, while slots
 // 0..2 return the short-range part (S/N) uK alone; L/N comes from ltab.
-// LZC, CWC > 0 select the compile-time z transforms (launched with exactly
-// kZThreads threads); 0 = runtime plan and tile width.
 constexpr int kZThreads = 256;
-// Resident CTAs per SM the z kernel is compiled for: FP32 tiles of 4 kx
-// columns (37 KB at Lz = 128) leave room for three CTAs, whose 85-register
-// budget the compiler then meets; wider tiles fit two.
-template <typename T>
-constexpr int kZMinBlocks(int cwc) { return (sizeof(T) == 4 && cwc == 4) ? 3 : 2; }
-// Component padding of the compile-time z tile, in complex values (64 bytes).
-template <typename T>
-constexpr int kZPad = 64 / (int)sizeof(cplx<T>);
 
-template <typename T, int LZC = 0, int CWC = 0, bool ACOU = false, bool ZSC = false>
-__global__ void __launch_bounds__(256, kZMinBlocks<T>(CWC)) k_z_kspace(cplx<T>* __restrict__ spec, const T* __restrict__ dtab,
+template <typename T, bool ACOU = false, bool ZSC = false>
+__global__ void __launch_bounds__(256, 2) k_z_kspace(cplx<T>* __restrict__ spec, const T* __restrict__ dtab,
                                                      const cplx<T>* __restrict__ ckmod, cplx<T>* __restrict__ acouK_out,
                                                      Geom g, FftPlan pz, const cplx<T>* __restrict__ twz, KMaps km,
                                                      const Phys* __restrict__ ph, double* __restrict__ part,
-                                                     DevScalars* sc, ZTiles zt, unsigned int* done,
-                                                     const T* __restrict__ ltab, const RepArgs* __restrict__ grp = nullptr) {
-  pdl_enter();
+                                                     DevScalars* sc, ZTiles zt, const T* __restrict__ ltab,
+                                                     const RepArgs* __restrict__ grp = nullptr) {
+  pdl_wait();
   if (grp) {
     const RepArgs& a = grp[blockIdx.y];
     spec = (cplx<T>*)a.spec;
@@ -1232,74 +1242,19 @@ __global__ void __launch_bounds__(256, kZMinBlocks<T>(CWC)) k_z_kspace(cplx<T>* 
   }
   FG_DYN_SMEM(smem_raw);
   cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
-  __shared__ cplx<T> tws_z[LZC > 0 ? LZC : 1];
-  const int Lz = LZC > 0 ? LZC : g.Lz, CW = CWC > 0 ? CWC : zt.CW;
+  const int Lz = g.Lz, CW = zt.CW;
   // ACOU: acoustic-displacement MD, three more components in and out
   // (FFT(acouR) in, dVdacK out; acouFFT.F:9-26, dVdac.F:11-63)
   constexpr int Z0 = ACOU ? 12 : 9;  // first Z* u slot (ZSC)
   constexpr int NC = Z0 + (ZSC ? 3 : 0);
   const int buf_len = NC * Lz * CW;
-  // component stride of the tile; the compile-time path pads it by 64 bytes
-  // so that the 4 components a warp spans fall on different banks
-  const int ZS = LZC > 0 ? LZC * CWC + kZPad<T> : Lz * CW;
-  // this thread's pencil: every butterfly it takes belongs to pencil
-  // threadIdx.x % CW (the batch and the block size are multiples of CW)
+  const int ZS = Lz * CW;  // component stride of the tile
   const int cwp = threadIdx.x % CW;
   int colp = 0, ysp = 0;
   const bool okp = tile_pencil(zt, g, cwp, &colp, &ysp);
-  cplx<T>* gp = spec + (okp ? (long long)ysp * g.KXP + colp : 0);
-  using BZ = BatchCT<NC * (CWC > 0 ? CWC : 1), (CWC > 0 ? CWC : 1), 1,
-                     (LZC > 0 ? LZC : 1) * (CWC > 0 ? CWC : 1) + kZPad<T>, (CWC > 0 ? CWC : 1)>;
-  if constexpr (LZC > 0) {
-    for (int i = threadIdx.x; i < LZC; i += blockDim.x) tws_z[i] = twz[i];
-    // first z stage straight from the spectrum (zeros for the pencils past
-    // Ly of the last Nyquist tile)
-    // (an evict_first policy on these FP64 loads measured slower: 156 against 140 us)
-    auto ld = [&](int t, int e) {
-      return okp ? gp[(long long)(t / CWC) * g.ncplx + (long long)e * g.plane_c] : mk<cplx<T>>((T)0, (T)0);
-    };
-    auto st = [&](int t, int e, const cplx<T>& v) { buf[(t / CWC) * ZS + (t % CWC) + e * CWC] = v; };
-    if constexpr (sizeof(T) == 4) {
-      // FP32: the whole tile by cp.async first (every copy in flight at
-      // once; regular tiles in 16-byte pencil pairs), then all stages
-      if (blockIdx.x >= zt.nnyq) {
-        int col0 = 0, ys0 = 0;
-        tile_pencil(zt, g, 0, &col0, &ys0);
-        const cplx<T>* base = spec + (long long)ys0 * g.KXP + col0;
-        constexpr int PP = 16 / (int)sizeof(cplx<T>);
-        const unsigned long long pol = l2_evict_first();  // the input spectrum is consumed
-        for (int r = threadIdx.x; r < NC * LZC * (CWC / PP); r += kZThreads) {
-          const int pp = r % (CWC / PP), rz = r / (CWC / PP);
-          const int c = rz / LZC, z = rz - c * LZC;
-          cp_async16_first(&buf[c * ZS + z * CWC + pp * PP],
-                           base + (long long)c * g.ncplx + (long long)z * g.plane_c + pp * PP, pol);
-        }
-      } else {
-        for (int r = threadIdx.x; r < NC * LZC * CWC; r += kZThreads) {
-          const int cw = r % CWC, rz = r / CWC;
-          const int c = rz / LZC, z = rz - c * LZC;
-          int col = 0, ys = 0;
-          cplx<T>* d = &buf[c * ZS + z * CWC + cw];
-          if (tile_pencil(zt, g, cw, &col, &ys))
-            cp_async<(int)sizeof(cplx<T>)>(
-                d, spec + (long long)ys * g.KXP + col + (long long)c * g.ncplx + (long long)z * g.plane_c);
-          else
-            *d = mk<cplx<T>>((T)0, (T)0);
-        }
-      }
-      cp_async_wait();
-      __syncthreads();
-      ct_forward_range<T, LZC, 0, ct_nst(LZC), kZThreads, BZ>(buf, tws_z);
-    } else {
-      ct_stage_io<T, LZC, 0, false, kZThreads, NC * CWC, false>(ld, st, twz);
-      __syncthreads();
-      ct_forward_range<T, LZC, 1, ct_nst(LZC), kZThreads, BZ>(buf, tws_z);
-    }
-  } else {
-    z_tile_load<T, LZC, CWC>(buf, spec, g, zt, NC);
-    Batch B{NC * CW, CW, 1, Lz * CW, CW, true};
-    fft_forward<T>(buf, B, pz, twz, buf_len);
-  }
+  z_tile_load<T>(buf, spec, g, zt, NC);
+  const Batch B{NC * CW, CW, 1, Lz * CW, CW, true};
+  fft_forward<T>(buf, B, pz, twz, buf_len);
   const double Ninv = ph->Ninv;
   // Energy sums: the per-k products in T (FP32 in the mixed path, whose
   // spectra are FP32), accumulated per thread in FP64
@@ -1349,15 +1304,9 @@ __global__ void __launch_bounds__(256, kZMinBlocks<T>(CWC)) k_z_kspace(cplx<T>* 
     }
     // ---- dipole-dipole
     const long long tpos = tpos0 + (long long)zs * g.KXP;
-    using T2 = typename RT2<T>::type;
-    const T2* Dp = reinterpret_cast<const T2*>((ZSC ? ltab : dtab) + tpos * 6);  // 6 T per k: 2 T-aligned pairs
     T D[6];  // D = (S + Z*^2 L)/N; ZSC: L/N
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const T2 v = __ldg(&Dp[q]);
-      D[2 * q] = v.x;
-      D[2 * q + 1] = v.y;
-    }
+    for (int q = 0; q < 6; ++q) D[q] = __ldg((ZSC ? ltab : dtab) + tab_index<T>(tpos, q));
     T qv[6];  // Re(conj(u_a) u_b): xx, yy, zz, yz, zx, xy
     qv[0] = u[0].x * u[0].x + u[0].y * u[0].y;
     qv[1] = u[1].x * u[1].x + u[1].y * u[1].y;
@@ -1530,21 +1479,402 @@ __global__ void __launch_bounds__(256, kZMinBlocks<T>(CWC)) k_z_kspace(cplx<T>* 
     for (int i = 0; i < 6; ++i) buf[(3 + i) * ZS + zs * CW + cw] = d[i];
   }
   __syncthreads();
-  if constexpr (LZC > 0) {
-    ct_inverse_range<T, LZC, ct_nst(LZC) - 1, 0, kZThreads, BZ>(buf, tws_z);
-    // last z stage straight to the spectrum
-    auto ld = [&](int t, int e) { return buf[(t / CWC) * ZS + (t % CWC) + e * CWC]; };
-    auto st = [&](int t, int e, const cplx<T>& v) {
-      if (okp) gp[(long long)(t / CWC) * g.ncplx + (long long)e * g.plane_c] = v;
-    };
-    ct_stage_io<T, LZC, 0, true, kZThreads, NC * CWC, false>(ld, st, tws_z);
-  } else {
-    Batch B{NC * CW, CW, 1, Lz * CW, CW, true};
-    fft_inverse<T>(buf, B, pz, twz, buf_len);
-    z_tile_store<T, LZC, CWC>(buf, spec, g, zt, NC);
-  }
+  fft_inverse<T>(buf, B, pz, twz, buf_len);
+  pdl_launch();
+  z_tile_store<T>(buf, spec, g, zt, NC);
   block_partials<NQ_K>(acc, part, blockIdx.x);
-  if (done != nullptr && is_last_block(done)) homo_strain_tail(ph, sc, part, gridDim.x);
+}
+
+// ------------------------------------------------------------------- k_z_lane
+// k_z_kspace for the compile-time lengths Lz, on elements of W neighbouring kx
+// slots (fft_lane.cuh).  A tile holds PW elements (PW W pencils) of all z and
+// components as buf[c][z'][pw], z' = z ^ (z / R2 & 1): with that swap of
+// neighbours the second stage's lanes (pw, a) fall on different banks.  The
+// stages have compile-time offsets; the k-space step works on W wavevectors
+// at a time.  Nyquist tiles (kx = Lx/2): the lanes of an element are ky slots.
+template <typename T, int LZ, int PW, bool ACOU>
+struct ZCT {
+  static constexpr int W = kLanes<T>, NC = ACOU ? 12 : 9;
+  static constexpr int R1 = ct_radix(LZ, 0), R2 = LZ / R1;
+  static constexpr int T1 = NC * PW * R2, T2 = NC * PW * R1;
+  // Threads: one first-stage butterfly each, up to 288.  128 x 4 elements:
+  // 288 threads at 96 registers in FP32 (74.1 us at 128^3; 256 threads 76.8),
+  // 256 at 128 in FP64 (131.8 us; 288 threads 133.6, spilling); three tiles per
+  // SM at 160 threads each took 96 and 166 us, the pass before this kernel
+  // 81.5 and 143.
+  static constexpr int NT = T1 > 256 && (ACOU || sizeof(T) == 8) ? 256 : (T1 + 31) / 32 * 32;
+  static constexpr int SMEM = NC * LZ * PW * 16;
+  static constexpr int MINB = NT >= 576 ? 1 : 576 / NT;
+  static_assert(ct_nst(LZ) == 2 && R2 % 2 == 0 && NT % PW == 0, "");
+};
+
+template <typename T, int LZ, int PW, bool ACOU = false>
+__global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>::MINB)
+    k_z_lane(cplx<T>* __restrict__ spec, const T* __restrict__ dtab, const cplx<T>* __restrict__ ckmod,
+             cplx<T>* __restrict__ acouK_out, Geom g, FftPlan, const cplx<T>* __restrict__ twz, KMaps km,
+             const Phys* __restrict__ ph, double* __restrict__ part, DevScalars* sc, ZTiles zt,
+             const T* __restrict__, const RepArgs* __restrict__ grp = nullptr) {
+  using Z = ZCT<T, LZ, PW, ACOU>;
+  using V = lane_t<T>;
+  constexpr int W = Z::W, NC = Z::NC, R1 = Z::R1, R2 = Z::R2, NT = Z::NT, ZS = LZ * PW;
+  if (grp) {
+    const RepArgs& a = grp[blockIdx.y];
+    spec = (cplx<T>*)a.spec;
+    dtab = (const T*)a.dtab;
+    ph = a.ph;
+    part = a.part_k;
+    sc = a.sc;
+  }
+  FG_DYN_SMEM(smem_raw);
+  CV<T>* const buf = reinterpret_cast<CV<T>*>(smem_raw);
+  __shared__ cplx<T> tab[LZ];
+  __shared__ double sAB[PW][W][10];  // S(k) along a pencil: A_q + B_q cos kz (sin kz for yz, zx)
+  __shared__ double reds[NT / 32][NQ_K];
+  const int tid = threadIdx.x;
+  const int pw = tid % PW, tile = blockIdx.x;
+  stage_twiddles<T, LZ, R1, R2>(tab, twz, (T)1);
+  // this thread's element: slots (ys, col) and (ys, col + 1), of a Nyquist
+  // tile (ys, m) and (ys + 1, m)
+  const bool nyq = tile < zt.nnyq;
+  int col, ys;
+  {
+    const int r = tile - zt.nnyq;
+    ys = nyq ? tile * zt.CW + W * pw : r / zt.ntx;
+    col = nyq ? g.m : (r - ys * zt.ntx) * zt.CW + W * pw;
+  }
+  const bool ok = ys < g.Ly, okb = nyq && W == 2 ? ys + 1 < g.Ly : ok;
+  if (!ok) ys = 0;
+  const int colb = W == 2 && !nyq ? col + 1 : col, ysb = W == 2 && nyq && okb ? ys + 1 : ys;
+  V k1, k2, w1;
+  bool has_k0;
+  {
+    k1 = vpack((T)__ldg(&km.kvx_s[col]), (T)__ldg(&km.kvx_s[colb]));
+    k2 = vpack((T)__ldg(&km.kvy_s[ys]), (T)__ldg(&km.kvy_s[ysb]));
+    // full-spectrum multiplicity: kx = 0 is slot 0, kx = Lx/2 slot m
+    w1 = vpack(!ok ? (T)0 : (col == 0 || nyq) ? (T)1 : (T)2, !okb ? (T)0 : nyq ? (T)1 : (T)2);
+    has_k0 = !nyq && col == 0 && ys == 0;  // lane 0 (ky = 0 is slot 0)
+    // S(k) of a pencil: one thread per pencil, each in a warp of its own
+    if (tid % 32 < PW && tid / 32 < W) {
+      const double* j = ph->j;
+      const double kap = ph->kap2x2;
+      const double2 ty = __ldg(&km.try_s[tid / 32 == 0 ? ys : ysb]), tx = __ldg(&km.trx_s[tid / 32 == 0 ? col : colb]);
+      const double c0 = tx.x, c1 = ty.x, s0 = tx.y, s1 = ty.y;
+      double* a = sAB[pw][tid / 32];
+      {
+        a[0] = kap + 2 * j[1] * c0 + 2 * j[0] * c1 + 4 * j[2] * c0 * c1;
+        a[1] = kap + 2 * j[1] * c1 + 2 * j[0] * c0 + 4 * j[2] * c1 * c0;
+        a[2] = kap + 2 * j[0] * (c0 + c1) + 4 * j[3] * c0 * c1;
+        a[3] = -4 * j[4] * s1 - 8 * j[6] * s1 * c0;  // yz, times sin kz
+        a[4] = -4 * j[4] * s0 - 8 * j[6] * s0 * c1;  // zx, times sin kz
+        a[5] = -4 * j[4] * s0 * s1;
+        a[6] = 2 * j[0] + 4 * j[3] * c1 + 4 * j[2] * c0 + 8 * j[5] * c0 * c1;
+        a[7] = 2 * j[0] + 4 * j[3] * c0 + 4 * j[2] * c1 + 8 * j[5] * c0 * c1;
+        a[8] = 2 * j[1] + 4 * j[2] * (c0 + c1) + 8 * j[5] * c0 * c1;
+        a[9] = -8 * j[6] * s0 * s1;
+      }
+    }
+  }
+  __syncthreads();
+  pdl_wait();
+  // Byte offset of this thread's element from the spectrum; a tile of a
+  // compile-time Lz spans less than 2 GB
+  constexpr unsigned ES = sizeof(cplx<T>);
+  const unsigned zstep = (unsigned)g.plane_c * ES, cstep = (unsigned)g.ncplx * ES;
+  const unsigned o0 = (unsigned)(ys * g.KXP + col) * ES, o1 = (unsigned)(ysb * g.KXP + colb) * ES;
+  const unsigned long long pol = l2_evict_first();  // the input spectrum is consumed
+  // forward: first stage from the spectrum
+  auto first = [&](auto nyqt) {
+    lane_tasks<Z::T1, NT>(tid, [&](int t) {
+      const int b = t / PW % R2, c = t / (PW * R2);
+      unsigned off = c * cstep + b * zstep;
+      CV<T> v[R1];
+#pragma unroll
+      for (int s = 0; s < R1; ++s, off += R2 * zstep) {
+        const char* q = reinterpret_cast<const char*>(spec) + off;
+        if constexpr (!decltype(nyqt)::value) {
+          const rowvec<T>* r = reinterpret_cast<const rowvec<T>*>(q + o0);
+          if constexpr (sizeof(T) == 4) v[s] = cv_of(ld_first(r, pol));
+          else v[s] = cv_of(*r);
+        } else {
+          const cplx<T> zero = mk<cplx<T>>((T)0, (T)0);
+          const cplx<T> x = ok ? *reinterpret_cast<const cplx<T>*>(q + o0) : zero;
+          const cplx<T> y = okb ? *reinterpret_cast<const cplx<T>*>(q + o1) : zero;
+          v[s] = CV<T>{vpack(x.x, y.x), vpack(x.y, y.y)};
+        }
+      }
+      DftV<T, R1, false>::run(v);
+      CV<T>* d = buf + c * ZS + pw;
+      cv_st(d + b * PW, v[0]);
+#pragma unroll
+      for (int s = 1; s < R1; ++s)
+        cv_st(d + (((s & 1) ? b ^ 1 : b) + R2 * s) * PW, cvtw<T, false>(v[s], tab[s * R2 + b]));
+    });
+  };
+  if (nyq) first(std::true_type());
+  else first(std::false_type());
+  // The dipole table's 6 values of W neighbouring slots, [slot / W][6][W], of
+  // this thread's k-space element e: the next one's are loaded while the
+  // strain part of the present one is computed
+  V D[6];
+  auto load_D = [&](int e) {
+    const unsigned tz = (unsigned)(e / PW) * g.KXP;
+    if (!nyq) {
+      const CV<T>* Dp = reinterpret_cast<const CV<T>*>(dtab + ((size_t)(ys * LZ * g.KXP) + tz + col) * 6);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const CV<T> v = cv_stream(Dp + q);
+        D[2 * q] = v.re;
+        D[2 * q + 1] = v.im;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        D[q] = vpack(dtab[tab_index<T>((long long)ys * LZ * g.KXP + tz + col, q)],
+                     dtab[tab_index<T>((long long)ysb * LZ * g.KXP + tz + colb, q)]);
+    }
+  };
+  if (tid < LZ * PW) load_D(tid);
+  __syncthreads();
+  auto second = [&](auto inv) {
+    lane_tasks<Z::T2, NT>(tid, [&](int t) {
+      const int a = t / PW % R1, c = t / (PW * R1), x = a & 1;
+      CV<T>*d0 = buf + c * ZS + pw + (a * R2 + x) * PW, *d1 = d0 - 2 * x * PW;  // z even / odd of the block
+      CV<T> v[R2];
+#pragma unroll
+      for (int q = 0; q < R2; ++q) v[q] = cv_ld(((q & 1) ? d1 : d0) + q * PW);
+      DftV<T, R2, decltype(inv)::value>::run(v);
+#pragma unroll
+      for (int q = 0; q < R2; ++q) cv_st(((q & 1) ? d1 : d0) + q * PW, v[q]);
+    });
+  };
+  second(std::false_type());
+  __syncthreads();
+  // ---- k space
+  const double Ninv = ph->Ninv;
+  const T ni = (T)Ninv;
+  const T B11 = (T)ph->B11, B12 = (T)ph->B12, B44 = (T)ph->B44;
+  const T hx = (T)(ph->HC2[0][0]), hy = (T)(ph->HC2[0][1]), h4 = (T)(ph->HC2[3][3]);
+  const bool mod = ph->modulation_on != 0;
+  double acc[NQ_K] = {0, 0, 0, 0, 0};
+#pragma unroll 1
+  for (int e = tid; e < LZ * PW; e += NT) {
+    const int zs = e / PW, zx = zs ^ (zs / R2 & 1);
+    CV<T>* el = buf + zx * PW + pw;
+    CV<T> u[3], d[6];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) u[a] = cv_ld(el + a * ZS);
+    const long long tz = (long long)zs * g.KXP;  // table positions of the element's lanes
+    {
+      // Re(conj(u_a) u_b): xx, yy, zz, yz, zx, xy
+      const V qv[6] = {vfma(u[0].re, u[0].re, vmul(u[0].im, u[0].im)), vfma(u[1].re, u[1].re, vmul(u[1].im, u[1].im)),
+                       vfma(u[2].re, u[2].re, vmul(u[2].im, u[2].im)), vfma(u[1].re, u[2].re, vmul(u[1].im, u[2].im)),
+                       vfma(u[2].re, u[0].re, vmul(u[2].im, u[0].im)), vfma(u[0].re, u[1].re, vmul(u[0].im, u[1].im))};
+      // short-range and total dipole energies in FP64 from the same products,
+      // so that their difference (the long-range energy) keeps its digits
+      const double2 tzc = __ldg(&km.trz_s[zs]);
+      auto lane_energy = [&](auto lane) {
+        constexpr int L = decltype(lane)::value;
+        const double* a = sAB[pw][L];
+        double qd[6], dd[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+          qd[q] = (double)vget<L>(qv[q]);
+          dd[q] = (double)vget<L>(D[q]);
+        }
+        const double w = (double)vget<L>(w1);
+        acc[0] += w * ((a[0] + a[6] * tzc.x) * qd[0] + (a[1] + a[7] * tzc.x) * qd[1] + (a[2] + a[8] * tzc.x) * qd[2] +
+                       2.0 * (a[3] * tzc.y * qd[3] + a[4] * tzc.y * qd[4] + (a[5] + a[9] * tzc.x) * qd[5]));
+        acc[1] += w * (dd[0] * qd[0] + dd[1] * qd[1] + dd[2] * qd[2] + 2.0 * (dd[3] * qd[3] + dd[4] * qd[4] + dd[5] * qd[5]));
+      };
+      lane_energy(std::integral_constant<int, 0>());
+      if constexpr (W == 2) lane_energy(std::integral_constant<int, 1>());
+    }
+    // F = D u
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int b = (a + 1) % 3, c = (a + 2) % 3;  // off-diagonal slots: yz 3, zx 4, xy 5
+      const V dab = D[a == 0 ? 5 : a == 1 ? 3 : 4], dac = D[a == 0 ? 4 : a == 1 ? 5 : 3];
+      cv_st(el + a * ZS, CV<T>{vfma(D[a], u[a].re, vfma(dab, u[b].re, vmul(dac, u[c].re))),
+                               vfma(D[a], u[a].im, vfma(dab, u[b].im, vmul(dac, u[c].im)))});
+    }
+    if (e + NT < LZ * PW) load_D(e + NT);
+    // ---- inhomogeneous strain
+#pragma unroll
+    for (int i = 0; i < 6; ++i) d[i] = cv_ld(el + (3 + i) * ZS);
+    const bool k0 = has_k0 && zs == 0;  // slot 0 holds kz = 0
+    if (k0) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) sc->didiK0[i] = (double)vget<0>(d[i].re);
+      __threadfence();  // read by homo_strain_tail in another kernel
+    }
+    const V k3 = vall((T)__ldg(&km.kvz_s[zs]));
+    // the elastic matrix K(k)
+    const V b11 = vall(B11), b44 = vall(B44), bxy = vall(B12 + B44);
+    const V k11 = vmul(k1, k1), k22 = vmul(k2, k2), k33 = vmul(k3, k3);
+    const V K00 = vfma(b11, k11, vmul(b44, vadd(k22, k33))), K11 = vfma(b11, k22, vmul(b44, vadd(k11, k33)));
+    const V K22 = vfma(b11, k33, vmul(b44, vadd(k11, k22)));
+    const V K01 = vmul(bxy, vmul(k1, k2)), K02 = vmul(bxy, vmul(k1, k3)), K12 = vmul(bxy, vmul(k2, k3));
+    // coup2 . didiK with coup2(a, i) of elastic.F:156-180
+    CV<T> cs[3], ck[3], acou[3];
+    {
+      const V vx = vall(hx), vy = vall(hy), v4 = vall(h4);
+      auto comb = [&](const V& ka, int ia, int ib, int ic, const V& kb, int sb, const V& kc, int sc_) {
+        // ka (hx d_ia + hy (d_ib + d_ic)) + h4 (kb d_sb + kc d_sc)
+        return CV<T>{vfma(ka, vfma(vx, d[ia].re, vmul(vy, vadd(d[ib].re, d[ic].re))),
+                          vmul(v4, vfma(kb, d[sb].re, vmul(kc, d[sc_].re)))),
+                     vfma(ka, vfma(vx, d[ia].im, vmul(vy, vadd(d[ib].im, d[ic].im))),
+                          vmul(v4, vfma(kb, d[sb].im, vmul(kc, d[sc_].im))))};
+      };
+      cs[0] = comb(k1, 0, 1, 2, k3, 4, k2, 5);
+      cs[1] = comb(k2, 1, 0, 2, k3, 3, k1, 5);
+      cs[2] = comb(k3, 2, 0, 1, k2, 3, k1, 4);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      cplx<T> m[2] = {mk<cplx<T>>((T)0, (T)0), mk<cplx<T>>((T)0, (T)0)};
+      if (mod) {
+#pragma unroll
+        for (int l = 0; l < W; ++l)
+          m[l] = ckmod[((long long)(l == 0 ? ys : ysb) * LZ * g.KXP + tz + (l == 0 ? col : colb)) * 3 + a];
+      }
+      ck[a] = CV<T>{vpack(m[0].x, m[1].x), vpack(m[0].y, m[1].y)};
+    }
+    const V w2 = vmul(vall((T)0.5), w1);  // energy_module.F weights: 1/2 at kx = 0, Lx/2
+    auto dot = [&](const CV<T>* x) {
+      V s = vmul(acou[0].re, x[0].re);
+      s = vfma(acou[0].im, x[0].im, s);
+#pragma unroll
+      for (int a = 1; a < 3; ++a) s = vfma(acou[a].im, x[a].im, vfma(acou[a].re, x[a].re, s));
+      return s;
+    };
+    auto add = [&](double& to, const V& v) {
+      to += (double)vget<0>(v);
+      if constexpr (W == 2) to += (double)vget<1>(v);
+    };
+    if constexpr (ACOU) {
+      // dynamic acoustic field: acouK = i FFT(acouR) (acouFFT.F:22);
+      // dVdacK = -i (c_k + coup2 didiK + K acouK) / N (dVdac.F:30-60);
+      // energies with the K acouK of this field (energy_module.F:150-240)
+      CV<T> KA[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const CV<T> X = cv_ld(el + (9 + a) * ZS);
+        acou[a] = CV<T>{vneg(X.im), X.re};
+      }
+      KA[0] = CV<T>{vfma(K00, acou[0].re, vfma(K01, acou[1].re, vmul(K02, acou[2].re))),
+                    vfma(K00, acou[0].im, vfma(K01, acou[1].im, vmul(K02, acou[2].im)))};
+      KA[1] = CV<T>{vfma(K01, acou[0].re, vfma(K11, acou[1].re, vmul(K12, acou[2].re))),
+                    vfma(K01, acou[0].im, vfma(K11, acou[1].im, vmul(K12, acou[2].im)))};
+      KA[2] = CV<T>{vfma(K02, acou[0].re, vfma(K12, acou[1].re, vmul(K22, acou[2].re))),
+                    vfma(K02, acou[0].im, vfma(K12, acou[1].im, vmul(K22, acou[2].im)))};
+      add(acc[2], vmul(w2, dot(KA)));
+      add(acc[3], vmul(w2, dot(cs)));
+      add(acc[4], vmul(w2, dot(ck)));
+      const V n = vall(ni);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const CV<T> v = cvadd(cvadd(ck[a], cs[a]), KA[a]);
+        cv_st(el + (9 + a) * ZS, CV<T>{vmul(v.im, n), vneg(vmul(v.re, n))});
+      }
+    } else {
+      // K acou = rhs = -(c_k + coup2 didiK) with K symmetric positive
+      // definite: adjugate over the determinant (the reference factorises K by
+      // Cholesky, elastic.F:110-125; the same up to rounding)
+      const V c00 = vfma(K11, K22, vneg(vmul(K12, K12))), c11 = vfma(K00, K22, vneg(vmul(K02, K02)));
+      const V c22 = vfma(K00, K11, vneg(vmul(K01, K01))), c01 = vfma(K02, K12, vneg(vmul(K01, K22)));
+      const V c02 = vfma(K01, K12, vneg(vmul(K02, K11))), c12 = vfma(K01, K02, vneg(vmul(K00, K12)));
+      const V det = vfma(K00, c00, vfma(K01, c01, vmul(K02, c02)));
+      // inhomo_K_G(:,:,0,0,0) = 0: no acoustic field at k = 0
+      const T i0 = k0 ? (T)0 : (T)-1 / vget<0>(det);
+      V inv = vpack(i0, (T)0);
+      if constexpr (W == 2) inv = vpack(i0, (T)-1 / vget<W - 1>(det));
+      CV<T> r[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) r[a] = CV<T>{vmul(vadd(ck[a].re, cs[a].re), inv), vmul(vadd(ck[a].im, cs[a].im), inv)};
+      acou[0] = CV<T>{vfma(c00, r[0].re, vfma(c01, r[1].re, vmul(c02, r[2].re))),
+                      vfma(c00, r[0].im, vfma(c01, r[1].im, vmul(c02, r[2].im)))};
+      acou[1] = CV<T>{vfma(c01, r[0].re, vfma(c11, r[1].re, vmul(c12, r[2].re))),
+                      vfma(c01, r[0].im, vfma(c11, r[1].im, vmul(c12, r[2].im)))};
+      acou[2] = CV<T>{vfma(c02, r[0].re, vfma(c12, r[1].re, vmul(c22, r[2].re))),
+                      vfma(c02, r[0].im, vfma(c12, r[1].im, vmul(c22, r[2].im)))};
+      // coupling Re(acou* . coup2 didiK), modulation Re(acou* . c_k); the
+      // strain energy Re(acou* K acou) = -(coupling + modulation) because
+      // K acou = -(c_k + coup2 didiK)
+      double x = 0.0, y = 0.0;
+      add(x, vmul(w2, dot(cs)));
+      if (mod) add(y, vmul(w2, dot(ck)));
+      acc[2] -= x + y;
+      acc[3] += x;
+      acc[4] += y;
+    }
+    if (acouK_out) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (ok) acouK_out[((long long)ys * LZ * g.KXP + tz + col) * 3 + a] = mk<cplx<T>>(vget<0>(acou[a].re), vget<0>(acou[a].im));
+        if (W == 2 && okb)
+          acouK_out[((long long)ysb * LZ * g.KXP + tz + colb) * 3 + a] = mk<cplx<T>>(vget<W - 1>(acou[a].re), vget<W - 1>(acou[a].im));
+      }
+    }
+    // inhoK = k (x) acou / N
+    {
+      const V n = vall(ni);
+      CV<T> an[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) an[a] = CV<T>{vmul(acou[a].re, n), vmul(acou[a].im, n)};
+      auto prod = [&](const V& ka, int a) { return CV<T>{vmul(ka, an[a].re), vmul(ka, an[a].im)}; };
+      auto prod2 = [&](const V& ka, int a, const V& kb, int b) {
+        return CV<T>{vfma(ka, an[a].re, vmul(kb, an[b].re)), vfma(ka, an[a].im, vmul(kb, an[b].im))};
+      };
+      cv_st(el + 3 * ZS, prod(k1, 0));
+      cv_st(el + 4 * ZS, prod(k2, 1));
+      cv_st(el + 5 * ZS, prod(k3, 2));
+      cv_st(el + 6 * ZS, prod2(k3, 1, k2, 2));
+      cv_st(el + 7 * ZS, prod2(k1, 2, k3, 0));
+      cv_st(el + 8 * ZS, prod2(k2, 0, k1, 1));
+    }
+  }
+  // this tile's energies: warps by shuffles, warps in order
+#pragma unroll
+  for (int q = 0; q < NQ_K; ++q) {
+    const double s = warp_sum(acc[q]);
+    if (tid % 32 == 0) reds[tid / 32][q] = s;
+  }
+  __syncthreads();
+  // inverse: the last forward stage first, the first one to the spectrum
+  second(std::true_type());
+  if (tid < NQ_K) {
+    double s = 0.0;
+    for (int w = 0; w < NT / 32; ++w) s += reds[w][tid];
+    part[(long long)tile * NQ_K + tid] = s;
+  }
+  __syncthreads();
+  pdl_launch();
+  auto last = [&](auto nyqt) {
+    lane_tasks<Z::T1, NT>(tid, [&](int t) {
+      const int b = t / PW % R2, c = t / (PW * R2);
+      const CV<T>* d = buf + c * ZS + pw;
+      CV<T> v[R1];
+      v[0] = cv_ld(d + b * PW);
+#pragma unroll
+      for (int s = 1; s < R1; ++s)
+        v[s] = cvtw<T, true>(cv_ld(d + (((s & 1) ? b ^ 1 : b) + R2 * s) * PW), tab[s * R2 + b]);
+      DftV<T, R1, true>::run(v);
+      unsigned off = c * cstep + b * zstep;
+#pragma unroll
+      for (int s = 0; s < R1; ++s, off += R2 * zstep) {
+        char* q = reinterpret_cast<char*>(spec) + off;
+        if constexpr (!decltype(nyqt)::value) {
+          cv_row(reinterpret_cast<rowvec<T>*>(q + o0), v[s]);
+        } else {
+          if (ok) *reinterpret_cast<cplx<T>*>(q + o0) = mk<cplx<T>>(vget<0>(v[s].re), vget<0>(v[s].im));
+          if (W == 2 && okb)
+            *reinterpret_cast<cplx<T>*>(q + o1) = mk<cplx<T>>(vget<W - 1>(v[s].re), vget<W - 1>(v[s].im));
+        }
+      }
+    });
+  };
+  if (nyq) last(std::true_type());
+  else last(std::false_type());
 }
 
 // ------------------------------------------------------------------ k_assemble
@@ -1688,7 +2018,8 @@ __global__ void __launch_bounds__(256, 2)
                const unsigned char* __restrict__ layer_sump, const T* __restrict__ site_minv,
                const unsigned char* __restrict__ site_sump, double* __restrict__ part_ke, T* __restrict__ Flo,
                const AsmConst k, const RepArgs* __restrict__ grp = nullptr) {
-  pdl_enter();
+  pdl_launch();  // one resident wave: nothing of this grid is left to schedule
+  pdl_wait();
   if (grp) {
     const RepArgs& a = grp[blockIdx.y];
     rw = (const T*)a.rwork;
@@ -2049,7 +2380,8 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
                                                     const double* __restrict__ layer_minv,
                                                     const T* __restrict__ site_minv = nullptr,
                                                     const RepArgs* __restrict__ grp = nullptr) {
-  pdl_enter();
+  pdl_launch();  // one resident wave: nothing of this grid is left to schedule
+  pdl_wait();
   if (grp) {
     const RepArgs& a = grp[blockIdx.y];
     p = (T*)a.p;
@@ -2110,7 +2442,8 @@ __global__ void __launch_bounds__(256) k_kick_close(T* __restrict__ p, const T* 
                                                     const double* __restrict__ part_r, int nblk_r,
                                                     const T* __restrict__ site_minv = nullptr,
                                                     const unsigned char* __restrict__ site_sump = nullptr) {
-  pdl_enter();
+  pdl_launch();  // one resident wave: nothing of this grid is left to schedule
+  pdl_wait();
   if (!PREP && blockIdx.x == 0) force_energies_tail(ph, sc, part_r, nblk_r, true);
   const long long ns = g.nsite;
   // pend_kick_f is not changed by block 0's commit
@@ -2456,7 +2789,7 @@ __global__ void __launch_bounds__(256) k_z_ewald_pack(const cplx<double>* __rest
     const long long tpos = ((long long)yslot * Lz + zs) * g.KXP + col;
     const double z2 = ph->Zstar * ph->Zstar;
     for (int q = 0; q < 6; ++q) {
-      dtab[tpos * 6 + q] = (T)((S[q] + z2 * Lt[q]) * ph->Ninv);
+      dtab[tab_index<T>(tpos, q)] = (T)((S[q] + z2 * Lt[q]) * ph->Ninv);
       if (L64) L64[tpos * 6 + q] = Lt[q];
     }
   }
@@ -2467,7 +2800,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_table_scale(T* __restrict__ dst, const double* __restrict__ src, double scale,
                                                      long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = (T)(src[i] * scale);
+    dst[tab_index<T>(i / 6, (int)(i % 6))] = (T)(src[i] * scale);
 }
 
 // c_k_modulation_k = modulation_constant * k * r2c(modulation_R) (elastic.F:212-225)
