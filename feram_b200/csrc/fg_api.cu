@@ -364,13 +364,13 @@ int launch_xy_fwd(fg_ctx* ctx, const T* src, cplx<T>* spec, int ncomp, int smem,
   return FG_OK;
 }
 
-// strain_prologue: block (0, 0) also runs the k-space energies and the
-// homogeneous strain from the partials of the preceding k_z_kspace.
+// strain_prologue: a block of its own also runs the k-space energies and the
+// homogeneous strain from the partials of the preceding k-space pass.
 template <typename T>
 int launch_xy_inv(fg_ctx* ctx, const cplx<T>* spec, T* out, int ncomp, bool strain_prologue = false) {
   const Geom& g = ctx->g;
   with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
-    launch_dep(ctx, kern, dim3(g.Lz, ncomp), nt, ctx->smem_xy,
+    launch_dep(ctx, kern, dim3(g.Lz, ncomp + (strain_prologue ? 1 : 0)), nt, ctx->smem_xy,
         spec, out, g, ctx->px, ctx->py, (const cplx<T>*)ctx->twx, (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy,
         ctx->posm, 0, strain_prologue ? ctx->ph : nullptr, ctx->sc, ctx->part_k, ctx->zt.nreg + ctx->zt.nnyq,
         (const RepArgs*)nullptr);
@@ -652,7 +652,7 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
     if (rc) return rc;
   }
   with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
-    launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), nt, c0->smem_xy, (const cplx<T>*)nullptr, (T*)nullptr, g,
+    launch_dep(c0, kern, dim3(g.Lz, c0->ncx + 1, nrep), nt, c0->smem_xy, (const cplx<T>*)nullptr, (T*)nullptr, g,
                c0->px, c0->py, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm, (const cplx<T>*)c0->twy, c0->posm,
                0, (const Phys*)c0->ph, (DevScalars*)nullptr, (const double*)nullptr, c0->zt.nreg + c0->zt.nnyq, grp);
   });

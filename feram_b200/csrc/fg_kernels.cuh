@@ -147,6 +147,27 @@ __device__ void block_partials(double* v, double* part, long long blockid) {
   __syncthreads();
 }
 
+// The same for two sets of sums with arrays of their own, in one pass.
+template <int NA, int NB>
+__device__ void block_partials2(const double* va, const double* vb, double* pa, double* pb, long long blockid) {
+  __shared__ double red[32][NA + NB];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int q = 0; q < NA + NB; ++q) {
+    const double s = warp_sum(q < NA ? va[q < NA ? q : 0] : vb[q < NA ? 0 : q - NA]);
+    if (lane == 0) red[wid][q] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < NA + NB; ++q) {
+      double s = 0.0;
+      for (int w = 0; w < nw; ++w) s += red[w][q];
+      (q < NA ? pa[blockid * NA + q] : pb[blockid * NB + q - NA]) = s;
+    }
+  }
+  __syncthreads();
+}
+
 // Sum of part[b*NQ + q] over b in fixed order by one RED_THREADS block.
 __device__ double reduce_partials(const double* part, int nblk, int NQ, int q) {
   __shared__ double red[RED_THREADS];
@@ -163,54 +184,53 @@ __device__ double reduce_partials(const double* part, int nblk, int NQ, int q) {
   return r;
 }
 
-// The same sums for all NQ columns in one pass: each thread adds its
-// blocks in a fixed order, warps combine with shuffles, warps in order.
-// Every thread receives the NQ totals.
-template <int NQ>
-__device__ void reduce_partials_all(const double* __restrict__ part, int nblk, double (&out)[NQ]) {
-  __shared__ double red[32][NQ];
-  double s[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) s[q] = 0.0;
-#pragma unroll 4
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) s[q] += __ldcg(&part[(long long)b * NQ + q]);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    const double t = warp_sum(s[q]);
-    if (lane == 0) red[wid][q] = t;
-  }
-  __syncthreads();
-  const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += red[w][q];
-    out[q] = t;
-  }
-  __syncthreads();
-}
-
 // Scalar work of a tail: thread 0 runs body on shared-memory copies of the
 // constants and scalars, loaded and stored back by the whole block in one
 // round trip each (instead of a chain of dependent global loads and stores
 // by one thread).
 static_assert(sizeof(DevScalars) % 8 == 0, "DevScalars is copied as doubles");
 static_assert(sizeof(Phys) % 8 == 0, "Phys is copied as doubles");
-template <class F>
-__device__ __forceinline__ void scalar_tail(const Phys* __restrict__ ph, DevScalars* sc, F&& body) {
+// The reduction of one or two sets of block partials (columns 0 .. NA-1 from
+// pa, then NB from pb) and the scalar work on the totals v[NA + NB]: the loads
+// of the constants and scalars are in flight with those of the partials, so a
+// tail costs one round trip to the L2, not two.
+template <int NA, int NB, class F>
+__device__ __forceinline__ void reduced_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ pa,
+                                             const double* __restrict__ pb, int nblk, F&& body) {
+  constexpr int NQ = NA + NB;
   __shared__ Phys sph;
   __shared__ DevScalars ssc;
+  __shared__ double red[32][NQ];
+  __shared__ double tot[NQ];
   constexpr int NP = (int)(sizeof(Phys) / 8), NS = (int)(sizeof(DevScalars) / 8);
   for (int i = threadIdx.x; i < NP; i += blockDim.x)
     reinterpret_cast<double*>(&sph)[i] = __ldg(reinterpret_cast<const double*>(ph) + i);
   for (int i = threadIdx.x; i < NS; i += blockDim.x)
     reinterpret_cast<double*>(&ssc)[i] = __ldcg(reinterpret_cast<const double*>(sc) + i);
+  double s[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) s[q] = 0.0;
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+#pragma unroll
+    for (int q = 0; q < NA; ++q) s[q] += __ldcg(&pa[(long long)b * NA + q]);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) s[NA + q] += __ldcg(&pb[(long long)b * NB + q]);
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const double t = warp_sum(s[q]);
+    if (lane == 0) red[wid][q] = t;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) body(static_cast<const Phys*>(&sph), &ssc);
+  if (threadIdx.x < NQ) {
+    double t = 0.0;
+    for (int w = 0; w < nw; ++w) t += red[w][threadIdx.x];
+    tot[threadIdx.x] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) body(static_cast<const Phys*>(&sph), &ssc, tot);
   __syncthreads();
   for (int i = threadIdx.x; i < NS; i += blockDim.x)
     reinterpret_cast<double*>(sc)[i] = reinterpret_cast<const double*>(&ssc)[i];
@@ -809,13 +829,17 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
     sc = a.sc;
     part_k = a.part_k;
   }
-  // Block (0, 0) first finishes the k-space pass that wrote spec: its
-  // energies and the homogeneous strain, from k_z_kspace's block partials
-  // (nothing in this kernel needs them; k_assemble does).
-  if (ph != nullptr && blockIdx.x == 0 && blockIdx.y == 0) homo_strain_tail(ph, sc, part_k, nblk_k);
+  // ph != null: the first row of blocks is no plane; its block 0 finishes the
+  // k-space pass that wrote spec: its energies and the homogeneous strain,
+  // from that pass's block partials (nothing in this kernel needs them;
+  // k_assemble does), beside the transforms instead of ahead of a plane's.
+  if (ph != nullptr && blockIdx.y == 0) {
+    if (blockIdx.x == 0) homo_strain_tail(ph, sc, part_k, nblk_k);
+    return;
+  }
   FG_DYN_SMEM(smem_raw);
   using T2 = typename RT2<T>::type;
-  const int z = blockIdx.x, c = blockIdx.y;
+  const int z = blockIdx.x, c = blockIdx.y - (ph != nullptr ? 1 : 0);
   const cplx<T>* srcp = spec + (long long)(in_comp0 + c) * g.ncplx + (long long)z * g.plane_c;
   T* dst = out + (long long)c * g.nsite + (long long)z * g.plane_r;
   if constexpr (MC > 0) {
@@ -972,9 +996,7 @@ __device__ __forceinline__ void check_finite(DevScalars* sc, const double* v, in
 // (optimize-homo-strain.F:27-186) and w_hom for k_assemble.
 __device__ __noinline__ void homo_strain_tail(const Phys* __restrict__ ph, DevScalars* sc,
                                               const double* __restrict__ part_k, int nblk) {
-  double v[NQ_K];
-  reduce_partials_all<NQ_K>(part_k, nblk, v);
-  scalar_tail(ph, sc, [&](const Phys* P, DevScalars* S) {
+  reduced_tail<NQ_K, 0>(ph, sc, part_k, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
     double* e = S->e;
     const double es = v[0] * P->Ninv / 2;  // (1/2N) sum w' Re(uK* S uK)
     const double edd = v[1] / 2;           // (1/2)  sum w' Re(uK* D uK), D = (S + Z*^2 L)/N
@@ -1044,40 +1066,29 @@ __device__ __noinline__ void homo_strain_tail(const Phys* __restrict__ ph, DevSc
 // kinetic_energy_dipo.F:106 from the kick partials
 __device__ __forceinline__ double ke_from(const Phys* ph, double sum) { return sum * ph->ke_scale; }
 
-// Nose-Poincare after the force (nose-poincare.F:60-66): H_NP, (35e).
-// Thread 0 only.
-__device__ void np_post_body(const Phys* __restrict__ ph, DevScalars* sc) {
-  const double inv_s = 1.0 / sc->s, inv_s2 = inv_s * inv_s;
-  np_hamiltonian(ph, sc, inv_s2, log(sc->s));
-  const double delta_H = sc->e[E_HNP] * inv_s;
-  sc->pi = sc->pi + ph->dt_2 * (2 * sc->e[E_DIPO] * inv_s2 - ph->nf_kT) - ph->dt_2 * delta_H;
+// After k_assemble: real-space energies from the totals v of its partials.
+__device__ __forceinline__ void force_energies_body(const Phys* P, DevScalars* S, const double* v) {
+  S->e[E_UNH] = v[0];
+  S->e[E_DIPE] = P->E_on ? -v[1] : 0.0;
+  check_finite(S, S->e + E_SHORT, 9);
 }
-
-// After k_assemble: real-space energies.  With np_close also the commit of
-// the prepared half step ((38), (35c): s, pi, KE at the half step) and the
-// (35e) update of pi, as the closing kick of a Nose-Poincare step needs.
-__device__ __noinline__ void force_energies_tail(const Phys* __restrict__ ph, DevScalars* sc,
-                                                 const double* __restrict__ part_r, int nblk, bool np_close) {
-  double v[NQ_R];
-  reduce_partials_all<NQ_R>(part_r, nblk, v);
-  scalar_tail(ph, sc, [&](const Phys* P, DevScalars* S) {
-    S->e[E_UNH] = v[0];
-    S->e[E_DIPE] = P->E_on ? -v[1] : 0.0;
-    check_finite(S, S->e + E_SHORT, 9);
-    if (np_close) {
-      S->s_old = S->s;
-      S->s = S->pend_s;
-      S->pi = S->pend_pi;
-      S->ke_sum = S->pend_ke_sum;
-      S->e[E_DIPO] = S->pend_ke;
-      S->drift_coef = S->pend_drift;
-      np_post_body(P, S);
-    }
-  });
+// A Nose-Poincare step after its force (nose-poincare.F:60-66): the commit of
+// the prepared half step ((38), (35c): s, pi, KE at the half step), H_NP and
+// the (35e) update of pi.
+__device__ __forceinline__ void np_post_body(const Phys* P, DevScalars* S, double inv_s, double log_s) {
+  S->s_old = S->s;
+  S->s = S->pend_s;
+  S->pi = S->pend_pi;
+  S->ke_sum = S->pend_ke_sum;
+  S->e[E_DIPO] = S->pend_ke;
+  S->drift_coef = S->pend_drift;
+  const double inv_s2 = inv_s * inv_s;
+  np_hamiltonian(P, S, inv_s2, log_s);
+  const double delta_H = S->e[E_HNP] * inv_s;
+  S->pi = S->pi + P->dt_2 * (2 * S->e[E_DIPO] * inv_s2 - P->nf_kT) - P->dt_2 * delta_H;
 }
-
-// Closing tail of a Nose-Poincare step.  part holds per block the masked
-// sums of p^2/m, p.F/m and F^2/m after the closing kick (35f).
+// End of a Nose-Poincare step from the masked sums v of p^2/m, p.F/m and
+// F^2/m after the closing kick (35f).
 //  - step_done: KE, H_NP and total of the finished step (nose-poincare.F:
 //    74-75, molecular-dynamics.F:293);
 //  - always: the first half of the next step (nose-poincare.F:24-41) as far
@@ -1085,39 +1096,59 @@ __device__ __noinline__ void force_energies_tail(const Phys* __restrict__ ph, De
 //    sum  sum p^2/m - 2 c sum p.F/m + c^2 sum F^2/m,  which gives (38) pi,
 //    s_{n+1} and the drift coefficient of (35c) before any site is touched.
 //    They are kept pending (s and pi still report the finished step).
+// One thread's serial FP64 chain: three divisions and a square root.
+__device__ __forceinline__ void np_close_body(const Phys* P, DevScalars* S, const double* v, double inv_s, double log_s,
+                                              bool step_done) {
+  const double s = S->s, inv_s2 = inv_s * inv_s;
+  const double epot = sum_potential(S->e);
+  if (step_done) {
+    S->ke_sum = v[0];
+    S->e[E_DIPO] = ke_from(P, v[0]);
+    np_hamiltonian(P, S, inv_s2, log_s);
+    S->e[E_TOT] = S->e[E_DIPO] * inv_s2 + S->e[E_ACOU] + epot;
+    check_finite(S, S->e, E_COUNT);
+  }
+  const double ca = P->dt_2 * s;
+  const double kh = v[0] - 2 * ca * v[1] + ca * ca * v[2];
+  const double ke = ke_from(P, kh);
+  double CB = P->nf_kT * (1.0 + log_s) - ke * inv_s2 + epot - S->H0;
+  CB = P->dt_2 * CB - S->pi;
+  const double r = CB * P->dt * P->Qinv;
+  if (1.0 - r < 0.0) S->status = 10;  // (38) has no real root: Q_Nose too small
+  const double pih = -2 * CB / (1.0 + sqrt(1.0 - r));
+  const double a = P->dt_2 * pih * P->Qinv;
+  const double sn = s * (1.0 + a) / (1.0 - a);
+  S->kick_coef = ca;
+  S->pend_ke_sum = kh;
+  S->pend_ke = ke;
+  S->pend_pi = pih;
+  S->pend_s = sn;
+  S->pend_drift = P->dt_2 * (1.0 / sn + inv_s);
+  S->pend_kick_f = P->dt_2 * sn;
+}
+
+__device__ __noinline__ void force_energies_tail(const Phys* __restrict__ ph, DevScalars* sc,
+                                                 const double* __restrict__ part_r, int nblk, bool np_close) {
+  reduced_tail<NQ_R, 0>(ph, sc, part_r, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+    force_energies_body(P, S, v);
+    if (np_close) np_post_body(P, S, 1.0 / S->pend_s, log(S->pend_s));
+  });
+}
 __device__ __noinline__ void np_close_tail(const Phys* __restrict__ ph, DevScalars* sc,
                                            const double* __restrict__ part, int nblk, bool step_done) {
-  double v[3];
-  reduce_partials_all<3>(part, nblk, v);
-  scalar_tail(ph, sc, [&](const Phys* P, DevScalars* S) {
-    // one thread's serial FP64 chain: one log, four divisions, one sqrt
-    const double s = S->s;
-    const double inv_s = 1.0 / s, inv_s2 = inv_s * inv_s, log_s = log(s);
-    const double epot = sum_potential(S->e);
-    if (step_done) {
-      S->ke_sum = v[0];
-      S->e[E_DIPO] = ke_from(P, v[0]);
-      np_hamiltonian(P, S, inv_s2, log_s);
-      S->e[E_TOT] = S->e[E_DIPO] * inv_s2 + S->e[E_ACOU] + epot;
-      check_finite(S, S->e, E_COUNT);
-    }
-    const double ca = P->dt_2 * s;
-    const double kh = v[0] - 2 * ca * v[1] + ca * ca * v[2];
-    const double ke = ke_from(P, kh);
-    double CB = P->nf_kT * (1.0 + log_s) - ke * inv_s2 + epot - S->H0;
-    CB = P->dt_2 * CB - S->pi;
-    const double r = CB * P->dt * P->Qinv;
-    if (1.0 - r < 0.0) S->status = 10;  // (38) has no real root: Q_Nose too small
-    const double pih = -2 * CB / (1.0 + sqrt(1.0 - r));
-    const double a = P->dt_2 * pih * P->Qinv;
-    const double sn = s * (1.0 + a) / (1.0 - a);
-    S->kick_coef = ca;
-    S->pend_ke_sum = kh;
-    S->pend_ke = ke;
-    S->pend_pi = pih;
-    S->pend_s = sn;
-    S->pend_drift = P->dt_2 * (1.0 / sn + inv_s);
-    S->pend_kick_f = P->dt_2 * sn;
+  reduced_tail<3, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+    np_close_body(P, S, v, 1.0 / S->s, log(S->s), step_done);
+  });
+}
+// Both for k_assemble with the fused closing kick, in one tail.
+__device__ __noinline__ void np_step_tail(const Phys* __restrict__ ph, DevScalars* sc,
+                                          const double* __restrict__ part_r, const double* __restrict__ part_ke,
+                                          int nblk) {
+  reduced_tail<NQ_R, 3>(ph, sc, part_r, part_ke, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+    const double inv_s = 1.0 / S->pend_s, log_s = log(S->pend_s);
+    force_energies_body(P, S, v);
+    np_post_body(P, S, inv_s, log_s);
+    np_close_body(P, S, v + NQ_R, inv_s, log_s, true);
   });
 }
 
@@ -1125,9 +1156,7 @@ __device__ __noinline__ void np_close_tail(const Phys* __restrict__ ph, DevScala
 // momenta, the factor sqrt(target / KE) for k_scale, total.  The reported
 // dipo_kinetic is the value before rescaling, as in the reference.
 __device__ void vs_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk) {
-  double v[1];
-  reduce_partials_all<1>(part, nblk, v);
-  scalar_tail(ph, sc, [&](const Phys* P, DevScalars* S) {
+  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
     S->ke_sum = v[0];
     S->e[E_DIPO] = ke_from(P, v[0]);
     S->vs_scale = sqrt(P->target_ke / S->e[E_DIPO]);
@@ -1141,9 +1170,7 @@ __device__ void vs_tail(const Phys* __restrict__ ph, DevScalars* sc, const doubl
 // with vs also the rescale factor (velocity_scaling.F:86-98) and the total.
 __device__ void acou_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk,
                           bool vs) {
-  double v[1];
-  reduce_partials_all<1>(part, nblk, v);
-  scalar_tail(ph, sc, [&](const Phys* P, DevScalars* S) {
+  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
     S->e[E_ACOU] = v[0] / 2;
     if (vs) {
       S->vs_scale_acou = sqrt(P->target_ke / S->e[E_ACOU]);
@@ -1155,9 +1182,7 @@ __device__ void acou_tail(const Phys* __restrict__ ph, DevScalars* sc, const dou
 
 // Leapfrog closing reduction (leapfrog.F:151) and total.
 __device__ void lf_final_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk) {
-  double v[1];
-  reduce_partials_all<1>(part, nblk, v);
-  scalar_tail(ph, sc, [&](const Phys* P, DevScalars* S) {
+  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
     S->ke_sum = v[0];
     S->e[E_DIPO] = ke_from(P, v[0]);
     S->e[E_TOT] = S->e[E_DIPO] / (S->s * S->s) + S->e[E_ACOU] + sum_potential(S->e);
@@ -2191,15 +2216,12 @@ __global__ void __launch_bounds__(256, 2)
       }
     }
   }
-  block_partials<NQ_R>(acc, part, blockIdx.x);
   if constexpr (CLOSE) {
-    block_partials<3>(ke, part_ke, blockIdx.x);
-    if (is_last_block(done)) {
-      force_energies_tail(ph, sc, part, gridDim.x, true);
-      np_close_tail(ph, sc, part_ke, gridDim.x, true);
-    }
-  } else if (tail == TAIL_ENERGIES && is_last_block(done)) {
-    force_energies_tail(ph, sc, part, gridDim.x, false);
+    block_partials2<NQ_R, 3>(acc, ke, part, part_ke, blockIdx.x);
+    if (is_last_block(done)) np_step_tail(ph, sc, part, part_ke, gridDim.x);
+  } else {
+    block_partials<NQ_R>(acc, part, blockIdx.x);
+    if (tail == TAIL_ENERGIES && is_last_block(done)) force_energies_tail(ph, sc, part, gridDim.x, false);
   }
 }
 
