@@ -17,6 +17,8 @@
 #pragma once
 #include "fft_smem.cuh"
 
+#include <type_traits>
+
 namespace fg {
 
 #ifdef FG_HOST_EMU
@@ -209,6 +211,30 @@ template <typename T, bool INV> struct DftV<T, 4, INV> {
   }
 };
 
+template <typename T, bool INV> struct DftV<T, 1, INV> {
+  static __device__ __forceinline__ void run(CV<T>*) {}
+};
+
+template <typename T, bool INV> struct DftV<T, 5, INV> {
+  static __device__ __forceinline__ void run(CV<T>* v) {
+    const lane_t<T> c1 = vall((T)0.30901699437494742410), c2 = vall((T)-0.80901699437494742410);
+    const lane_t<T> s1 = vall((T)0.95105651629515357212), s2 = vall((T)0.58778525229247312917);
+    const CV<T> t1 = cvadd(v[1], v[4]), t2 = cvadd(v[2], v[3]), t3 = cvsub(v[1], v[4]), t4 = cvsub(v[2], v[3]);
+    const CV<T> a1{vfma(t1.re, c1, vfma(t2.re, c2, v[0].re)), vfma(t1.im, c1, vfma(t2.im, c2, v[0].im))};
+    const CV<T> a2{vfma(t1.re, c2, vfma(t2.re, c1, v[0].re)), vfma(t1.im, c2, vfma(t2.im, c1, v[0].im))};
+    const CV<T> b1{vfma(t3.re, s1, vmul(t4.re, s2)), vfma(t3.im, s1, vmul(t4.im, s2))};
+    const CV<T> b2{vfma(t3.re, s2, vneg(vmul(t4.re, s1))), vfma(t3.im, s2, vneg(vmul(t4.im, s1)))};
+    v[0] = cvadd(v[0], cvadd(t1, t2));
+    // y = a -+ i b
+    const CV<T> p1{vadd(a1.re, b1.im), vsub(a1.im, b1.re)}, n1{vsub(a1.re, b1.im), vadd(a1.im, b1.re)};
+    const CV<T> p2{vadd(a2.re, b2.im), vsub(a2.im, b2.re)}, n2{vsub(a2.re, b2.im), vadd(a2.im, b2.re)};
+    v[1] = INV ? n1 : p1;
+    v[4] = INV ? p1 : n1;
+    v[2] = INV ? n2 : p2;
+    v[3] = INV ? p2 : n2;
+  }
+};
+
 // 6 = 2 x 3 by the Chinese remainder map: no twiddles.
 template <typename T, bool INV> struct DftV<T, 6, INV> {
   static __device__ __forceinline__ void run(CV<T>* v) {
@@ -283,6 +309,126 @@ template <typename T, bool INV> struct DftV<T, 16, INV> {
     }
   }
 };
+
+// 9, 10, 12 and 15 as Dft of fft_smem.cuh.
+template <typename T, int N1, int N2, bool INV> struct DftVCrt {
+  static __device__ __forceinline__ void run(CV<T>* v) {
+    constexpr int N = N1 * N2;
+    constexpr int c1 = N2 * (N2 % N1 == 1 ? 1 : N1 - 1), c2 = N1 * (N1 % N2 == 1 ? 1 : N1 * 2 % N2 == 1 ? 2 : N1 * 3 % N2 == 1 ? 3 : 4);
+    static_assert(c1 % N1 == 1 && c2 % N2 == 1, "");
+    CV<T> a[N1][N2];
+#pragma unroll
+    for (int i = 0; i < N1; ++i) {
+#pragma unroll
+      for (int j = 0; j < N2; ++j) a[i][j] = v[(N2 * i + N1 * j) % N];
+      DftV<T, N2, INV>::run(a[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < N2; ++j) {
+      CV<T> b[N1];
+#pragma unroll
+      for (int i = 0; i < N1; ++i) b[i] = a[i][j];
+      DftV<T, N1, INV>::run(b);
+#pragma unroll
+      for (int i = 0; i < N1; ++i) v[(c1 * i + c2 * j) % N] = b[i];
+    }
+  }
+};
+template <typename T, bool INV> struct DftV<T, 10, INV> : DftVCrt<T, 2, 5, INV> {};
+template <typename T, bool INV> struct DftV<T, 12, INV> : DftVCrt<T, 3, 4, INV> {};
+template <typename T, bool INV> struct DftV<T, 15, INV> : DftVCrt<T, 3, 5, INV> {};
+template <typename T, bool INV> struct DftV<T, 9, INV> {
+  static __device__ __forceinline__ void run(CV<T>* v) {
+    const T sg = INV ? (T)1 : (T)-1;
+    const T c[3] = {(T)0.76604444311897803520, (T)0.17364817766693034885, (T)-0.93969262078590838405};
+    const T s[3] = {(T)0.64278760968653932632, (T)0.98480775301220805937, (T)0.34202014332566873304};
+    CV<T> a[3][3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) a[q][r] = v[q + 3 * r];
+      DftV<T, 3, INV>::run(a[q]);
+    }
+    auto tw = [&](const CV<T>& x, int k) { return cvtw<T, false>(x, mk<cplx<T>>(c[k], sg * s[k])); };
+    a[1][1] = tw(a[1][1], 0);
+    a[1][2] = tw(a[1][2], 1);
+    a[2][1] = tw(a[2][1], 1);
+    a[2][2] = tw(a[2][2], 2);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      CV<T> b[3] = {a[0][r], a[1][r], a[2][r]};
+      DftV<T, 3, INV>::run(b);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) v[r + 3 * q] = b[q];
+    }
+  }
+};
+
+// ------------------------------------------------ lengths known at run time
+// Two stages n = r1 r2, r1 >= r2, r1 <= 16 and r2 <= 10: every n <= 100 of
+// factors 2, 3, 5 and most up to 160.  even: r1 even (the x pass, whose r2 may
+// then be the larger one).  False: no such split (125, an x length 150).
+__host__ __device__ inline bool lane_radix(int r) {
+  return (r >= 2 && r <= 6) || r == 8 || r == 9 || r == 10 || r == 12 || r == 15 || r == 16;
+}
+inline bool lane_split(int n, bool even, int* r1, int* r2) {
+  int best = 0;
+  for (int a = 2; a <= 16; ++a) {
+    if (n % a != 0 || !lane_radix(a) || (even && a % 2 != 0)) continue;
+    const int b = n / a;
+    if (b > 10 || (b > 1 && !lane_radix(b)) || (!even && b > a)) continue;
+    const int larger = a > b ? a : b;  // the most even split
+    if (best == 0 || larger < best) {
+      best = larger;
+      *r1 = a;
+      *r2 = b;
+    }
+  }
+  return best != 0;
+}
+// f(std::integral_constant<int, r>) for a radix known at run time
+template <class F>
+__device__ __forceinline__ void first_radix(int r, F&& f) {
+  switch (r) {
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 5: f(std::integral_constant<int, 5>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    case 9: f(std::integral_constant<int, 9>()); break;
+    case 10: f(std::integral_constant<int, 10>()); break;
+    case 12: f(std::integral_constant<int, 12>()); break;
+    case 15: f(std::integral_constant<int, 15>()); break;
+    case 16: f(std::integral_constant<int, 16>()); break;
+    default: break;
+  }
+}
+template <class F>
+__device__ __forceinline__ void second_radix(int r, F&& f) {
+  switch (r) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 5: f(std::integral_constant<int, 5>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    case 9: f(std::integral_constant<int, 9>()); break;
+    case 10: f(std::integral_constant<int, 10>()); break;
+    default: break;
+  }
+}
+// Quotients by a number known at launch, n d < 2^31: multiplication by
+// ceil(2^32 / d).
+struct FastDiv {
+  unsigned mul;  // 0: d = 1
+  int d;
+};
+inline FastDiv fast_div(int d) { return FastDiv{d == 1 ? 0u : (unsigned)((0x100000000ull + d - 1) / d), d}; }
+__device__ __forceinline__ int fdiv(int n, const FastDiv& f) {
+  return f.mul == 0 ? n : (int)(((unsigned long long)(unsigned)n * f.mul) >> 32);
+}
 
 // Twiddles of a first stage of radix R1 in the order its threads read them,
 // tab[s * NB + b] = scale w_n^(b s), b < NB: neighbouring butterflies b read

@@ -190,6 +190,64 @@ struct Dft<T, 5, INV> {
   }
 };
 
+// 10 = 2 x 5, 12 = 3 x 4 and 15 = 3 x 5 by the Chinese remainder map; 9 = 3 x 3
+// with the twiddles w9, w9^2, w9^4.
+template <typename T, int N1, int N2, bool INV>
+struct DftCrt {
+  static __device__ __forceinline__ void run(cplx<T>* v) {
+    constexpr int N = N1 * N2;
+    // k = k1 (mod N1), k2 (mod N2): k = c1 k1 + c2 k2
+    constexpr int c1 = N2 * (N2 % N1 == 1 ? 1 : N1 - 1), c2 = N1 * (N1 % N2 == 1 ? 1 : N1 * 2 % N2 == 1 ? 2 : N1 * 3 % N2 == 1 ? 3 : 4);
+    static_assert(c1 % N1 == 1 && c2 % N2 == 1, "");
+    cplx<T> a[N1][N2];
+#pragma unroll
+    for (int i = 0; i < N1; ++i) {
+#pragma unroll
+      for (int j = 0; j < N2; ++j) a[i][j] = v[(N2 * i + N1 * j) % N];
+      Dft<T, N2, INV>::run(a[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < N2; ++j) {
+      cplx<T> b[N1];
+#pragma unroll
+      for (int i = 0; i < N1; ++i) b[i] = a[i][j];
+      Dft<T, N1, INV>::run(b);
+#pragma unroll
+      for (int i = 0; i < N1; ++i) v[(c1 * i + c2 * j) % N] = b[i];
+    }
+  }
+};
+template <typename T, bool INV> struct Dft<T, 10, INV> : DftCrt<T, 2, 5, INV> {};
+template <typename T, bool INV> struct Dft<T, 12, INV> : DftCrt<T, 3, 4, INV> {};
+template <typename T, bool INV> struct Dft<T, 15, INV> : DftCrt<T, 3, 5, INV> {};
+template <typename T, bool INV>
+struct Dft<T, 9, INV> {
+  static __device__ __forceinline__ void run(cplx<T>* v) {
+    const T sg = INV ? (T)1 : (T)-1;
+    const T c[3] = {(T)0.76604444311897803520, (T)0.17364817766693034885, (T)-0.93969262078590838405};
+    const T s[3] = {(T)0.64278760968653932632, (T)0.98480775301220805937, (T)0.34202014332566873304};
+    cplx<T> a[3][3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) a[q][r] = v[q + 3 * r];
+      Dft<T, 3, INV>::run(a[q]);
+    }
+    auto tw = [&](cplx<T> x, int k) { return cmul(x, mk<cplx<T>>(c[k], sg * s[k])); };
+    a[1][1] = tw(a[1][1], 0);
+    a[1][2] = tw(a[1][2], 1);
+    a[2][1] = tw(a[2][1], 1);
+    a[2][2] = tw(a[2][2], 2);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      cplx<T> b[3] = {a[0][r], a[1][r], a[2][r]};
+      Dft<T, 3, INV>::run(b);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) v[r + 3 * q] = b[q];
+    }
+  }
+};
+
 template <typename T, int R, bool INV>
 __device__ __forceinline__ void fft_stage(cplx<T>* __restrict__ buf, const Batch& B, int n, int Ls,
                                           const cplx<T>* __restrict__ tw, int buf_len) {
@@ -242,6 +300,10 @@ __device__ __forceinline__ void fft_stage_rt(int R, cplx<T>* buf, const Batch& B
     case 5: fft_stage<T, 5, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 6: fft_stage<T, 6, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 8: fft_stage<T, 8, INV>(buf, B, n, Ls, tw, buf_len); break;
+    case 9: fft_stage<T, 9, INV>(buf, B, n, Ls, tw, buf_len); break;
+    case 10: fft_stage<T, 10, INV>(buf, B, n, Ls, tw, buf_len); break;
+    case 12: fft_stage<T, 12, INV>(buf, B, n, Ls, tw, buf_len); break;
+    case 15: fft_stage<T, 15, INV>(buf, B, n, Ls, tw, buf_len); break;
     case 16: fft_stage<T, 16, INV>(buf, B, n, Ls, tw, buf_len); break;
     default: break;
   }

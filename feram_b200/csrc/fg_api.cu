@@ -28,14 +28,21 @@ constexpr int kThreadsElem = 256;
 
 int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
-// DIF stage radices: the compile-time plans of fft_smem.cuh for powers of
-// two, otherwise largest first (8, 4, 2, then 3 and 5).
+// DIF stage radices: the compile-time plans of fft_smem.cuh, the two stages
+// of fft_lane.cuh's runtime kernels, otherwise largest first (8, 4, 2, then 3
+// and 5).
 bool make_plan(int n, FftPlan* P) {
   P->n = n;
   P->nst = 0;
   if (ct_supported(n)) {
     P->nst = ct_nst(n);
     for (int st = 0; st < P->nst; ++st) P->r[st] = ct_radix(n, st);
+    return true;
+  }
+  int r1 = 0, r2 = 0;
+  if (n <= kLaneMax && lane_split(n, false, &r1, &r2)) {
+    P->r[P->nst++] = r1;
+    if (r2 > 1) P->r[P->nst++] = r2;
     return true;
   }
   int m = n;
@@ -45,6 +52,33 @@ bool make_plan(int n, FftPlan* P) {
   while (m % 3 == 0) { if (P->nst >= FFT_MAX_STAGES) return false; P->r[P->nst++] = 3; m /= 3; }
   while (m % 5 == 0) { if (P->nst >= FFT_MAX_STAGES) return false; P->r[P->nst++] = 5; m /= 5; }
   return m == 1 && P->nst <= FFT_MAX_STAGES;
+}
+
+// A plane with compile-time x-y kernels (with_xy_fwd).
+bool xy_ct(int m, int Ly) {
+  return (m == 64 && Ly == 128) || (m == 32 && Ly == 64) || (m == 16 && Ly == 32) || (m == 8 && Ly == 16) ||
+         (m == 24 && Ly == 48) || (m == 12 && Ly == 24);
+}
+// Shapes of the runtime two-stage x-y kernels at W transforms per element;
+// false: the plane is left to the general kernels (a length without two
+// stages, more second-stage tasks than threads, or no room in shared memory).
+bool xy_geo(int Lx, int Ly, const FftPlan& py, int W, int smem_max, XyGeo* h) {
+  *h = XyGeo{};
+  if (xy_ct(Lx / 2, Ly) || Lx > kLaneMax || Ly > kLaneMax || py.nst > 2 || !lane_split(Lx, true, &h->R1, &h->R2)) return false;
+  h->RY1 = py.r[0];
+  h->RY2 = py.nst == 2 ? py.r[1] : 1;
+  if (!lane_radix(h->RY1) || (h->RY2 > 1 && (!lane_radix(h->RY2) || h->RY2 > 10))) return false;
+  h->NQ = div_up(Ly, 2 * W);
+  h->NJ = div_up(Lx / 2, W);
+  h->QS = Lx + 1;
+  h->JS = Ly | 1;
+  h->dR2 = fast_div(h->R2);
+  h->dNQ = fast_div(h->NQ);
+  h->dNJ = fast_div(h->NJ);
+  const int second = h->R1 / 2 * h->NQ;
+  h->nt = (std::max({second, std::min(256, h->NQ * h->R2), std::min(256, h->NJ * h->RY2)}) + 31) / 32 * 32;
+  h->smem = std::max(h->NQ * h->QS, h->NJ * h->JS) * 16;
+  return h->nt <= 512 && h->smem <= smem_max;
 }
 
 // slot -> frequency of the DIF output (digit reversal)
@@ -89,6 +123,9 @@ struct fg_ctx {
   std::string err;
   Geom g{};
   FftPlan px{}, py{}, pz{};
+  ZTiles zk{};  // tiles of the k-space pass (zt, or the runtime k_z_lane's)
+  ZGeo zg{};    // runtime k_z_lane; R1 = 0: not in use
+  XyGeo xyg{}, xyg64{};  // runtime two-stage x-y kernels (nt = 0: not in use) in the context's precision and in FP64
   ZTiles zt{}, zt6{}, zt1{};  // z tiles: MD k-space (9 comps, T), table build (6, FP64), modulation (1, FP64)
   int smem_xy = 0, smem_xy64 = 0, smem_z = 0, smem_z3 = 0, smem_z6 = 0, smem_z1 = 0;
   int grid_elem = 1;
@@ -351,15 +388,23 @@ void launch_dep(fg_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size
   cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// zstar: per-site Z*, transformed times u in components zu0..zu0+2
+// zstar: per-site Z*, transformed times u in components zu0..zu0+2; nrep
+// replicas (grp != null) or the context's own
 template <typename T, int MODE>
-int launch_xy_fwd(fg_ctx* ctx, const T* src, cplx<T>* spec, int ncomp, int smem, const cplx<T>* twx,
-                  const cplx<T>* twm, const cplx<T>* twy, const T* zstar = nullptr, int zu0 = 0) {
+int launch_xy_fwd(fg_ctx* ctx, const T* src, cplx<T>* spec, int ncomp, const cplx<T>* twx, const cplx<T>* twm,
+                  const cplx<T>* twy, const T* zstar = nullptr, int zu0 = 0, int nrep = 1, const RepArgs* grp = nullptr) {
   const Geom& g = ctx->g;
-  with_xy_fwd<T, MODE>(g.m, g.Ly, [&](auto kern, int nt) {
-    launch_dep(ctx, kern, dim3(g.Lz, ncomp), nt, smem, src, spec, g, ctx->px, ctx->py, twx, twm, twy,
-               ctx->posm, 0, zstar, zu0, (const RepArgs*)nullptr);
-  });
+  const bool own = (ctx->prec == FG_PREC_MIXED) == (sizeof(T) == 4);  // FP64 in a mixed context: the table build
+  const XyGeo& h = own ? ctx->xyg : ctx->xyg64;
+  if (h.nt > 0) {
+    launch_dep(ctx, k_xy_fwd_gen<T, MODE>, dim3(g.Lz, ncomp, nrep), h.nt, h.smem, src, spec, g, h, twx, twy,
+               ctx->posm, zstar, zu0, grp);
+  } else {
+    with_xy_fwd<T, MODE>(g.m, g.Ly, [&](auto kern, int nt) {
+      launch_dep(ctx, kern, dim3(g.Lz, ncomp, nrep), nt, own ? ctx->smem_xy : ctx->smem_xy64, src, spec, g, ctx->px,
+                 ctx->py, twx, twm, twy, ctx->posm, 0, zstar, zu0, grp);
+    });
+  }
   CKL();
   return FG_OK;
 }
@@ -367,39 +412,61 @@ int launch_xy_fwd(fg_ctx* ctx, const T* src, cplx<T>* spec, int ncomp, int smem,
 // strain_prologue: a block of its own also runs the k-space energies and the
 // homogeneous strain from the partials of the preceding k-space pass.
 template <typename T>
-int launch_xy_inv(fg_ctx* ctx, const cplx<T>* spec, T* out, int ncomp, bool strain_prologue = false) {
+int launch_xy_inv(fg_ctx* ctx, const cplx<T>* spec, T* out, int ncomp, bool strain_prologue = false, int nrep = 1,
+                  const RepArgs* grp = nullptr) {
   const Geom& g = ctx->g;
-  with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
-    launch_dep(ctx, kern, dim3(g.Lz, ncomp + (strain_prologue ? 1 : 0)), nt, ctx->smem_xy,
-        spec, out, g, ctx->px, ctx->py, (const cplx<T>*)ctx->twx, (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy,
-        ctx->posm, 0, strain_prologue ? ctx->ph : nullptr, ctx->sc, ctx->part_k, ctx->zt.nreg + ctx->zt.nnyq,
-        (const RepArgs*)nullptr);
-  });
+  const dim3 grid(g.Lz, ncomp + (strain_prologue ? 1 : 0), nrep);
+  const Phys* ph = strain_prologue ? ctx->ph : nullptr;
+  const int nblk = ctx->zk.nreg + ctx->zk.nnyq;
+  const XyGeo& h = ctx->xyg;
+  if (h.nt > 0) {
+    launch_dep(ctx, k_xy_inv_gen<T>, grid, h.nt, h.smem, spec, out, g, h, (const cplx<T>*)ctx->twx,
+               (const cplx<T>*)ctx->twy, ctx->posm, ph, ctx->sc, ctx->part_k, nblk, grp);
+  } else {
+    with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
+      launch_dep(ctx, kern, grid, nt, ctx->smem_xy, spec, out, g, ctx->px, ctx->py, (const cplx<T>*)ctx->twx,
+                 (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy, ctx->posm, 0, ph, ctx->sc, ctx->part_k, nblk, grp);
+    });
+  }
   CKL();
   return FG_OK;
 }
 
-// The k-space partials are finished by the next k_xy_inv (strain prologue).
 // nrep replicas (grp != null) or the context's own.
 template <typename T>
 int launch_z_kspace(fg_ctx* ctx, cplx<T>* acouK_out, int nrep = 1, const RepArgs* grp = nullptr) {
   const Geom& g = ctx->g;
-  auto go = [&](auto kern, int nt, int smem) {
-    launch_dep(ctx, kern, dim3(ctx->zt.nreg + ctx->zt.nnyq, nrep), nt, smem, (cplx<T>*)ctx->spec, (const T*)ctx->dtab,
-               (const cplx<T>*)ctx->ckmod, acouK_out, g, ctx->pz, (const cplx<T>*)ctx->twz, kmaps<T>(ctx), ctx->ph,
-               ctx->part_k, ctx->sc, ctx->zt, (const T*)ctx->ltab, grp);
+  const ZTiles& zk = ctx->zk;
+  const dim3 grid(zk.nreg + zk.nnyq, nrep);
+  auto lane = [&](auto kern, int nt, int smem) {
+    launch_dep(ctx, kern, grid, nt, smem, (cplx<T>*)ctx->spec, (const T*)ctx->dtab, (const cplx<T>*)ctx->ckmod,
+               acouK_out, g, ctx->zg, (const cplx<T>*)ctx->twz, kmaps<T>(ctx), ctx->ph, ctx->part_k, ctx->sc, zk, grp);
   };
-  if (!with_z_lane<T>(g.Lz, ctx->zt.CW, ctx->acou, ctx->zsite,
-                      [&](auto kern, auto shape) { go(kern, decltype(shape)::NT, decltype(shape)::SMEM); }))
-    with_z_kspace<T>(ctx->acou, ctx->zsite, [&](auto kern) { go(kern, kZThreads, ctx->smem_z); });
+  if (ctx->zg.R1 > 0) {
+    const int smem = (int)(ctx->ncx * (size_t)g.Lz * zk.CW * sizeof(cplx<T>));
+    if (ctx->acou) lane(k_z_lane<T, 0, 0, true>, ZCT<T, 0, 0, true>::NT, smem);
+    else lane(k_z_lane<T, 0, 0, false>, ZCT<T, 0, 0, false>::NT, smem);
+  } else if (!with_z_lane<T>(g.Lz, zk.CW, ctx->acou, ctx->zsite,
+                             [&](auto kern, auto shape) { lane(kern, decltype(shape)::NT, decltype(shape)::SMEM); })) {
+    with_z_kspace<T>(ctx->acou, ctx->zsite, [&](auto kern) {
+      launch_dep(ctx, kern, grid, kZThreads, ctx->smem_z, (cplx<T>*)ctx->spec, (const T*)ctx->dtab,
+                 (const cplx<T>*)ctx->ckmod, acouK_out, g, ctx->pz, (const cplx<T>*)ctx->twz, kmaps<T>(ctx), ctx->ph,
+                 ctx->part_k, ctx->sc, zk, (const T*)ctx->ltab, grp);
+    });
+  }
   CKL();
   return FG_OK;
 }
 
-// Dynamic shared-memory limit of the k-space kernel of tiles zt (smem_z: the
-// runtime kernel's).
+// How the k-space pass runs on tiles zt of ncx components: the compile-time
+// k_z_lane where with_z_lane has it, else its runtime form for lengths of two
+// stages, whose rows need not divide into tiles (as wide as zt's cap `cw`
+// allows: 1, 2 or 4 elements), else k_z_kspace (smem_z bytes).  Raises the
+// kernel's shared-memory limit; the caller stores the result.
 template <typename T>
-int prepare_z(fg_ctx* ctx, const ZTiles& zt, bool zsite, int smem_z, int smem_optin) {
+int plan_z(fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_z, int smem_optin, ZTiles* zk, ZGeo* zg) {
+  constexpr int W = kLanes<T>;
+  const Geom& g = ctx->g;
   cudaError_t ea = cudaSuccess;
   auto setattr = [&](auto kern, int bytes) {
     cudaFuncAttributes fa;
@@ -409,9 +476,33 @@ int prepare_z(fg_ctx* ctx, const ZTiles& zt, bool zsite, int smem_z, int smem_op
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     if (e != cudaSuccess) ea = e;
   };
-  if (!with_z_lane<T>(ctx->g.Lz, zt.CW, ctx->acou, zsite,
-                      [&](auto kern, auto shape) { setattr(kern, decltype(shape)::SMEM); }))
+  *zk = zt;
+  *zg = ZGeo{};
+  const FftPlan& pz = ctx->pz;
+  if (with_z_lane<T>(g.Lz, zt.CW, ctx->acou, zsite,
+                     [&](auto kern, auto shape) { setattr(kern, decltype(shape)::SMEM); })) {
+  } else if (!zsite && g.Lz <= kLaneMax && pz.nst <= 2 && (pz.nst == 1 || pz.r[1] <= 10)) {
+    int pw = std::max(1, cw / W);
+    while (pw > 1 && (size_t)ncx * g.Lz * pw * 16 > (size_t)(smem_optin - 8192) / 2) pw /= 2;  // two tiles per SM
+    zk->CW = pw * W;
+    zg->R1 = pz.r[0];
+    zg->R2 = pz.nst == 2 ? pz.r[1] : 1;
+    zg->lpw = pw == 4 ? 2 : pw == 2 ? 1 : 0;
+    zg->d1 = fast_div(zg->R1);
+    zg->d2 = fast_div(zg->R2);
+    // FP32 elements are pairs of slots: with an odd Lx/2 the last pair of a row
+    // ends with the Nyquist slot
+    const bool with_nyq = W == 2 && g.m % 2 != 0;
+    zg->ncol = g.m + (with_nyq ? 1 : 0);
+    zk->ntx = div_up(zg->ncol, zk->CW);
+    zk->nreg = zk->ntx * g.Ly;
+    zk->nnyq = with_nyq ? 0 : div_up(g.Ly, zk->CW);
+    const int smem = (int)((size_t)ncx * g.Lz * pw * 16);
+    if (ctx->acou) setattr(k_z_lane<T, 0, 0, true>, smem);
+    else setattr(k_z_lane<T, 0, 0, false>, smem);
+  } else {
     with_z_kspace<T>(ctx->acou, zsite, [&](auto kern) { setattr(kern, smem_z); });
+  }
   if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
   return FG_OK;
 }
@@ -461,7 +552,7 @@ int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false) {
     CKL();
   }
   int rc;
-  if ((rc = launch_xy_fwd<T, SRC_U9>(ctx, u, (cplx<T>*)ctx->spec, ctx->ncx, ctx->smem_xy, (const cplx<T>*)ctx->twx,
+  if ((rc = launch_xy_fwd<T, SRC_U9>(ctx, u, (cplx<T>*)ctx->spec, ctx->ncx, (const cplx<T>*)ctx->twx,
                                      (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy,
                                      ctx->zsite ? (const T*)ctx->site_zstar : nullptr, zu_comp(ctx))))
     return rc;
@@ -641,22 +732,11 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
              (const T*)nullptr, (const DevScalars*)nullptr, g, (const double*)nullptr, (const T*)nullptr, grp);
   CKL();
   c0->pdl = true;
-  with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto kern, int nt) {
-    launch_dep(c0, kern, dim3(g.Lz, c0->ncx, nrep), nt, c0->smem_xy, (const T*)nullptr, (cplx<T>*)nullptr,
-               g, c0->px, c0->py, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm, (const cplx<T>*)c0->twy,
-               c0->posm, 0, (const T*)nullptr, 0, grp);
-  });
-  CKL();
-  {
-    const int rc = launch_z_kspace<T>(c0, nullptr, nrep, grp);
-    if (rc) return rc;
-  }
-  with_xy_inv<T>(g.m, g.Ly, [&](auto kern, int nt) {
-    launch_dep(c0, kern, dim3(g.Lz, c0->ncx + 1, nrep), nt, c0->smem_xy, (const cplx<T>*)nullptr, (T*)nullptr, g,
-               c0->px, c0->py, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm, (const cplx<T>*)c0->twy, c0->posm,
-               0, (const Phys*)c0->ph, (DevScalars*)nullptr, (const double*)nullptr, c0->zt.nreg + c0->zt.nnyq, grp);
-  });
-  CKL();
+  int rc = launch_xy_fwd<T, SRC_U9>(c0, nullptr, nullptr, c0->ncx, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm,
+                                    (const cplx<T>*)c0->twy, nullptr, 0, nrep, grp);
+  if (!rc) rc = launch_z_kspace<T>(c0, nullptr, nrep, grp);
+  if (!rc) rc = launch_xy_inv<T>(c0, nullptr, nullptr, c0->ncx, true, nrep, grp);
+  if (rc) return rc;
   launch_dep(c0, k_assemble<T, true>, dim3(c0->grid_asc, nrep), kThreadsElem, 0, (const T*)nullptr,
              (const T*)nullptr, (T*)nullptr, g, (const Phys*)nullptr, (DevScalars*)nullptr, (double*)nullptr,
              (int)TAIL_NONE, (unsigned int*)nullptr, (const unsigned char*)nullptr, (const T*)nullptr,
@@ -678,7 +758,7 @@ bool groupable(const fg_ctx* c) {
 bool same_group(const fg_ctx* a, const fg_ctx* b) {
   if (a->prec != b->prec || a->g.Lx != b->g.Lx || a->g.Ly != b->g.Ly || a->g.Lz != b->g.Lz) return false;
   // one launch covers the group with the first replica's tiles and grids
-  if (a->zt.CW != b->zt.CW || a->grid_kd != b->grid_kd || a->grid_asc != b->grid_asc) return false;
+  if (a->zt.CW != b->zt.CW || a->zk.CW != b->zk.CW || a->grid_kd != b->grid_kd || a->grid_asc != b->grid_asc) return false;
   const AsmConst ka = asm_const(a), kb = asm_const(b);
   return std::memcmp(&ka, &kb, sizeof(AsmConst)) == 0;
 }
@@ -899,6 +979,10 @@ int create_impl(fg_ctx* ctx) {
   ctx->smem_z3 = (int)(3 * (size_t)g.Lz * ctx->zt.CW * sizeof(cplx<T>));
   ctx->smem_z6 = (int)(6 * (size_t)g.Lz * ctx->zt6.CW * sizeof(cplx<double>));
   ctx->smem_z1 = (int)(1 * (size_t)g.Lz * ctx->zt1.CW * sizeof(cplx<double>));
+  // FP64 too (the table build), so that both precisions leave the same slots
+  if (!xy_geo(g.Lx, g.Ly, ctx->py, kLanes<double>, smem_max, &ctx->xyg64) ||
+      !xy_geo(g.Lx, g.Ly, ctx->py, kLanes<T>, smem_max, &ctx->xyg))
+    ctx->xyg = ctx->xyg64 = XyGeo{};
   ctx->grid_elem = std::max(1, std::min(div_up(g.nsite, kThreadsElem), nsm * 8));
   plan_grids<T>(ctx, ctx->plan_waves, nsm);
   {
@@ -915,10 +999,17 @@ int create_impl(fg_ctx* ctx) {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
       if (e != cudaSuccess) ea = e;
     };
-    with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
-    with_xy_fwd<T, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
-    with_xy_fwd<double, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy64); });
-    with_xy_inv<T>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
+    if (ctx->xyg.nt > 0) {
+      setattr(k_xy_fwd_gen<T, SRC_U9>, ctx->xyg.smem);
+      setattr(k_xy_fwd_gen<T, SRC_FIELD>, ctx->xyg.smem);
+      setattr(k_xy_fwd_gen<double, SRC_FIELD>, ctx->xyg64.smem);
+      setattr(k_xy_inv_gen<T>, ctx->xyg.smem);
+    } else {
+      with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
+      with_xy_fwd<T, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
+      with_xy_fwd<double, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy64); });
+      with_xy_inv<T>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
+    }
     with_z_pass<T, false>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
     with_z_pass<T, true>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
     setattr(k_z_ewald_pack<T>, ctx->smem_z6);
@@ -931,6 +1022,8 @@ int create_impl(fg_ctx* ctx) {
   // posm: [0, m) the slot of each packed-x frequency; then the y maps of
   // the xy kernels, [m, m + Ly) slot -> ky and [m + Ly, m + 2 Ly) ky -> slot
   std::vector<int> revm = digit_reversal(ctx->px);
+  if (ctx->xyg.nt > 0)  // x slot = kx
+    for (int k = 0; k < g.m; ++k) revm[k] = k;
   ctx->h_revx.resize(g.NKX);
   for (int s = 0; s < g.m; ++s) ctx->h_revx[s] = revm[s];
   ctx->h_revx[g.m] = g.m;
@@ -1138,8 +1231,9 @@ int create_impl(fg_ctx* ctx) {
   CK(cudaMemset(ctx->ckmod, 0, 3 * sizeof(cplx<T>) * (size_t)g.nkpos));
   CK(cudaMalloc(&ctx->acouK, 3 * sizeof(cplx<T>) * (size_t)g.nkpos));
   CK(cudaMemset(ctx->acouK, 0, 3 * sizeof(cplx<T>) * (size_t)g.nkpos));
-  CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(ctx->zt.nreg + ctx->zt.nnyq)));
-  if (const int rc2 = prepare_z<T>(ctx, ctx->zt, false, ctx->smem_z, smem_optin)) return rc2;
+  if (const int rc2 = plan_z<T>(ctx, ctx->zt, plan_cw<T>(ctx, nsm), ctx->ncx, false, ctx->smem_z, smem_optin, &ctx->zk, &ctx->zg))
+    return rc2;
+  CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(ctx->zk.nreg + ctx->zk.nnyq)));
   CK(cudaMalloc(&ctx->part_r, sizeof(double) * NQ_R * (size_t)ctx->grid_elem));
   CK(cudaMalloc(&ctx->part_ke, sizeof(double) * 3 * (size_t)ctx->grid_elem));
   CK(cudaMalloc(&ctx->part_avg, sizeof(double) * 6 * (size_t)ctx->grid_elem));
@@ -1168,7 +1262,7 @@ int build_tables_impl(fg_ctx* ctx) {
   const int max_x = 24 / P.Lx, max_y = 24 / P.Ly, max_z = 24 / P.Lz;  // dipole-dipole-long-range.F:98-100
   k_ewald_real<<<std::max(1, div_up(g.nsite, 128)), 128, 0, ctx->stream>>>(real6, g, P.a0, P.kappa, max_x, max_y, max_z);
   CKL();
-  int rc0 = launch_xy_fwd<double, SRC_FIELD>(ctx, real6, spec6, 6, ctx->smem_xy64, ctx->twx64, ctx->twm64,
+  int rc0 = launch_xy_fwd<double, SRC_FIELD>(ctx, real6, spec6, 6, ctx->twx64, ctx->twm64,
                                              ctx->twy64);
   if (rc0) return rc0;
   k_z_ewald_pack<T><<<ctx->zt6.nreg + ctx->zt6.nnyq, kThreadsZ, ctx->smem_z6, ctx->stream>>>(
@@ -1196,7 +1290,7 @@ int set_modulation_R_impl(fg_ctx* ctx, const double* modR) {
   CK(cudaMemcpyAsync(ctx->staging, modR, sizeof(double) * nin, cudaMemcpyHostToDevice, ctx->stream));
   k_fortran_to_soa<double><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>(r1, ctx->staging, g, 1, ctx->NXP, ctx->NYP);
   CKL();
-  int rc0 = launch_xy_fwd<double, SRC_FIELD>(ctx, r1, s1, 1, ctx->smem_xy64, ctx->twx64, ctx->twm64, ctx->twy64);
+  int rc0 = launch_xy_fwd<double, SRC_FIELD>(ctx, r1, s1, 1, ctx->twx64, ctx->twm64, ctx->twy64);
   if (rc0) return rc0;
   k_z_modulation_pack<T><<<ctx->zt1.nreg + ctx->zt1.nnyq, kThreadsZ, ctx->smem_z1, ctx->stream>>>(
       s1, (cplx<T>*)ctx->ckmod, g, ctx->pz, ctx->twz64, kmaps<T>(ctx), ctx->P.modulation_constant, ctx->zt1);
@@ -1354,7 +1448,7 @@ int launch_z_pass(fg_ctx* ctx) {
 // the FFT entry points, on the device buffers only.
 template <typename T>
 int enqueue_fft_r2c3(fg_ctx* ctx) {
-  int rc = launch_xy_fwd<T, SRC_FIELD>(ctx, (const T*)ctx->rwork, (cplx<T>*)ctx->spec, 3, ctx->smem_xy,
+  int rc = launch_xy_fwd<T, SRC_FIELD>(ctx, (const T*)ctx->rwork, (cplx<T>*)ctx->spec, 3,
                                        (const cplx<T>*)ctx->twx, (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy);
   if (rc) return rc;
   return launch_z_pass<T, false>(ctx);
@@ -1401,7 +1495,7 @@ int fft_r2c3_impl(fg_ctx* ctx, const double* in, double* out) {
   const Geom& g = ctx->g;
   int rc = set_field<T>(ctx, ctx->rwork, in);
   if (rc) return rc;
-  if ((rc = launch_xy_fwd<T, SRC_FIELD>(ctx, (const T*)ctx->rwork, (cplx<T>*)ctx->spec, 3, ctx->smem_xy,
+  if ((rc = launch_xy_fwd<T, SRC_FIELD>(ctx, (const T*)ctx->rwork, (cplx<T>*)ctx->spec, 3,
                                         (const cplx<T>*)ctx->twx, (const cplx<T>*)ctx->twm,
                                         (const cplx<T>*)ctx->twy)))
     return rc;
@@ -1469,7 +1563,9 @@ int set_zsite(fg_ctx* ctx, bool on) {
   if ((size_t)ncx * g.Lz * zt.CW * sizeof(cplx<T>) > (size_t)smem_max)
     return fail(ctx, FG_ERR_UNSUPPORTED, "a z pencil of the supercell does not fit in shared memory");
   const int smem_z = (int)(ncx * ((size_t)g.Lz * zt.CW) * sizeof(cplx<T>));
-  if (const int rc = prepare_z<T>(ctx, zt, on, smem_z, smem_optin)) return rc;
+  ZTiles zk;
+  ZGeo zg;
+  if (const int rc = plan_z<T>(ctx, zt, plan_cw<T>(ctx, nsm), ncx, on, smem_z, smem_optin, &zk, &zg)) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->broken = true;  // until every buffer below is allocated again
   for (void** b : {&ctx->spec, &ctx->rwork, (void**)&ctx->part_k, &ctx->ltab})
@@ -1479,6 +1575,8 @@ int set_zsite(fg_ctx* ctx, bool on) {
     }
   ctx->ncx = ncx;
   ctx->zt = zt;
+  ctx->zk = zk;
+  ctx->zg = zg;
   ctx->smem_z = smem_z;
   ctx->smem_z3 = (int)(3 * (size_t)g.Lz * zt.CW * sizeof(cplx<T>));
   ctx->zsite = on;
@@ -1486,7 +1584,7 @@ int set_zsite(fg_ctx* ctx, bool on) {
   CK(cudaMalloc(&ctx->spec, (size_t)ncx * sizeof(cplx<T>) * (size_t)g.ncplx));
   CK(cudaMemsetAsync(ctx->spec, 0, (size_t)ncx * sizeof(cplx<T>) * (size_t)g.ncplx, ctx->stream));
   CK(cudaMalloc(&ctx->rwork, (size_t)ncx * ctx->real_bytes));
-  CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(zt.nreg + zt.nnyq)));
+  CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(zk.nreg + zk.nnyq)));
   if (on) CK(cudaMalloc(&ctx->ltab, 6 * sizeof(T) * (size_t)g.nkpos));
   ctx->broken = false;
   return FG_OK;
@@ -1675,7 +1773,7 @@ int profile_impl(fg_ctx* ctx, int reps, double* ms) {
     CK(cudaEventRecord(ev[k], st));
     rc |= enqueue_kick_drift<T>(ctx);
     CK(cudaEventRecord(ev[++k], st));
-    rc |= launch_xy_fwd<T, SRC_U9>(ctx, u, (cplx<T>*)ctx->spec, ctx->ncx, ctx->smem_xy, (const cplx<T>*)ctx->twx,
+    rc |= launch_xy_fwd<T, SRC_U9>(ctx, u, (cplx<T>*)ctx->spec, ctx->ncx, (const cplx<T>*)ctx->twx,
                                    (const cplx<T>*)ctx->twm, (const cplx<T>*)ctx->twy,
                                    ctx->zsite ? (const T*)ctx->site_zstar : nullptr, zu_comp(ctx));
     CK(cudaEventRecord(ev[++k], st));
@@ -2749,19 +2847,23 @@ int apply_plan_t(fg_ctx* ctx, int zcw, int waves) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     if (e != cudaSuccess) ea = e;
   };
-  if (const int rc = prepare_z<T>(ctx, zt, ctx->zsite, smem_z, smem_optin)) return rc;
+  ZTiles zk;
+  ZGeo zg;
+  if (const int rc = plan_z<T>(ctx, zt, cwmax, ctx->ncx, ctx->zsite, smem_z, smem_optin, &zk, &zg)) return rc;
   with_z_pass<T, false>(g.Lz, zt.CW, [&](auto k) { setattr(k, smem_z3); });
   with_z_pass<T, true>(g.Lz, zt.CW, [&](auto k) { setattr(k, smem_z3); });
   if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (zt.nreg + zt.nnyq > ctx->zt.nreg + ctx->zt.nnyq) {
+  if (zk.nreg + zk.nnyq > ctx->zk.nreg + ctx->zk.nnyq) {
     ctx->broken = true;  // until part_k is allocated again
     cudaFree(ctx->part_k);
     ctx->part_k = nullptr;
-    CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(zt.nreg + zt.nnyq)));
+    CK(cudaMalloc(&ctx->part_k, sizeof(double) * NQ_K * (size_t)(zk.nreg + zk.nnyq)));
     ctx->broken = false;
   }
   ctx->zt = zt;
+  ctx->zk = zk;
+  ctx->zg = zg;
   ctx->smem_z = smem_z;
   ctx->smem_z3 = smem_z3;
   ctx->plan_zcw = zcw;

@@ -895,6 +895,345 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
   }
 }
 
+constexpr int kLaneMax = 160;  // longest length of the runtime two-stage transforms
+
+// ------------------------------------------------------- k_xy_fwd_gen / inv_gen
+// The x-y passes of planes without a compile-time instance: the algorithm and
+// layouts of XyCT with the lengths, strides and counts known at run time and
+// the butterflies chosen by radix.  Any Lx = R1 R2 with R1 even (R2 may be
+// odd), Ly = RY1 RY2 (lane_split).  Rows of a group past Ly (the last one's
+// fourth, for Ly = 5 also its third) are zero;
+// with an odd Lx/2 the last column element's second lane is a dummy.  Columns
+// cross from the x to the y pass as complex values side by side, two per FP32
+// element, in natural order: x slot = kx.
+struct XyGeo {
+  int R1, R2, RY1, RY2;
+  int NQ, NJ, QS, JS;       // row groups, column elements, their strides
+  FastDiv dR2, dNQ, dNJ;
+  int nt, smem;             // threads, dynamic shared memory (this precision)
+};
+
+// f(k, A, B, dc) for every column k < Lx/2 of classes al and a1 held in v0, v1
+// with A = Z(k), B = Z(-k); dc: column 0 with A = Z(0), B = Z(Lx/2).
+template <int R2, class C, class F>
+__device__ __forceinline__ void class_columns(C* v0, C* v1, int al, int a1, int R1, F&& f) {
+  if (al != 0) {
+#pragma unroll
+    for (int t = 0; t < (R2 + 1) / 2; ++t) f(al + R1 * t, v0[t], v1[R2 - 1 - t], false);
+#pragma unroll
+    for (int t = 0; t < R2 / 2; ++t) f(a1 + R1 * t, v1[t], v0[R2 - 1 - t], false);
+  } else {
+    f(0, v0[0], R2 % 2 == 0 ? v0[R2 / 2] : v1[(R2 - 1) / 2], true);
+#pragma unroll
+    for (int t = 1; t < (R2 + 1) / 2; ++t) f(R1 * t, v0[t], v0[R2 - t], false);
+#pragma unroll
+    for (int t = 0; t < R2 / 2; ++t) f(a1 + R1 * t, v1[t], v1[R2 - 1 - t], false);
+  }
+}
+// complex value of column k, row y in the column layout
+template <typename T>
+__device__ __forceinline__ cplx<T>* column_at(CV<T>* buf, int JS, int k, int y) {
+  constexpr int W = kLanes<T>;
+  return reinterpret_cast<cplx<T>*>(buf + k / W * JS + y) + k % W;
+}
+
+template <typename T, int MODE>
+__global__ void __launch_bounds__(512, 1)
+    k_xy_fwd_gen(const T* __restrict__ src, cplx<T>* __restrict__ spec, Geom g, XyGeo h, const cplx<T>* __restrict__ twx,
+                 const cplx<T>* __restrict__ twy, const int* __restrict__ posm, const T* __restrict__ zstar, int zu0,
+                 const RepArgs* __restrict__ grp) {
+  constexpr int W = kLanes<T>;
+  if (grp) {
+    src = (const T*)grp[blockIdx.z].u;
+    spec = (cplx<T>*)grp[blockIdx.z].spec;
+  }
+  FG_DYN_SMEM(smem_raw);
+  CV<T>* const buf = reinterpret_cast<CV<T>*>(smem_raw);
+  __shared__ cplx<T> tabx[kLaneMax], taby[kLaneMax], col0[kLaneMax];
+  const int nt = blockDim.x, tid = threadIdx.x;
+  const int Lx = g.Lx, Ly = g.Ly, m = g.m;
+  const int z = blockIdx.x, c = blockIdx.y;
+  for (int k = tid; k < Lx; k += nt) tabx[k] = mk<cplx<T>>((T)0.5 * twx[k].x, (T)0.5 * twx[k].y);  // halved: unpack_rows
+  for (int k = tid; k < Ly; k += nt) taby[k] = twy[k];
+  __syncthreads();
+  pdl_wait();
+  const bool zu = MODE == SRC_U9 && zstar != nullptr && c >= zu0;
+  const bool plain = !zu && (MODE == SRC_FIELD || c < 3 || c >= 9);
+  const bool square = !zu && !plain && c < 6;
+  const int ca = zu ? c - zu0
+                    : plain ? (c >= 9 && MODE == SRC_U9 ? c - 6 : c) : (c == 3 || c == 8) ? 0 : (c == 4 || c == 6) ? 1 : 2;
+  const int cb = (c == 3) ? 0 : (c == 4) ? 1 : (c == 5) ? 2 : (c == 6) ? 2 : (c == 7) ? 0 : 1;
+  const long long plane_off = (long long)z * g.plane_r;
+  const T* const pa = src + (long long)ca * g.nsite + plane_off;
+  const T* const pb = zu ? zstar + plane_off : src + (long long)cb * g.nsite + plane_off;
+  cplx<T>* const dst = spec + (long long)c * g.ncplx + (long long)z * g.plane_c;
+  const int rows = h.NQ * Lx;  // elements between a group's rows
+  // first x stage
+  first_radix(h.R1, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+    for (int t = tid; t < h.NQ * h.R2; t += nt) {
+      const int q = fdiv(t, h.dR2), b = t - q * h.R2;
+      const bool full = q + h.NQ * (2 * W - 1) < Ly, third = q + 2 * h.NQ < Ly;
+      auto ld = [&](const T* r) {
+        return CV<T>{vpack(r[0], W == 2 && third ? r[2 * rows] : (T)0),
+                     vpack(W == 2 || full ? r[rows] : (T)0, W == 2 && full ? r[3 * rows] : (T)0)};
+      };
+      const T* r = pa + q * Lx + b;
+      CV<T> v[R];
+#pragma unroll
+      for (int s = 0; s < R; ++s) v[s] = ld(r + s * h.R2);
+      if (!plain) {
+        const T* r2 = pb + q * Lx + b;
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+          const CV<T> w = square ? v[s] : ld(r2 + s * h.R2);
+          v[s] = CV<T>{vmul(v[s].re, w.re), vmul(v[s].im, w.im)};
+        }
+      }
+      DftV<T, R, false>::run(v);
+      CV<T>* d = buf + q * h.QS + b;
+      const lane_t<T> half = vall((T)0.5);
+      cv_st(d, CV<T>{vmul(v[0].re, half), vmul(v[0].im, half)});
+#pragma unroll
+      for (int s = 1; s < R; ++s) cv_st(d + s * h.R2, cvtw<T, false>(v[s], tabx[s * b]));
+    }
+  });
+  __syncthreads();
+  // second x stage with the separation of the rows
+  second_radix(h.R2, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+    const int al = fdiv(tid, h.dNQ), q = tid - al * h.NQ;
+    const bool on = tid < (h.R1 / 2) * h.NQ;
+    const int a1 = al == 0 ? h.R1 / 2 : h.R1 - al;
+    CV<T> v0[R], v1[R];
+    if (on) {
+      const CV<T>* r = buf + q * h.QS;
+#pragma unroll
+      for (int t = 0; t < R; ++t) v0[t] = cv_ld(r + al * R + t);
+#pragma unroll
+      for (int t = 0; t < R; ++t) v1[t] = cv_ld(r + a1 * R + t);
+      DftV<T, R, false>::run(v0);
+      DftV<T, R, false>::run(v1);
+    }
+    __syncthreads();
+    if (on) {
+      const bool full = q + h.NQ * (2 * W - 1) < Ly, third = q + 2 * h.NQ < Ly;
+      class_columns<R>(v0, v1, al, a1, h.R1, [&](int k, const CV<T>& A, const CV<T>& B, bool dc) {
+        T x0[2], x1[2];
+        unpack_rows<0>(A, B, dc, x0, x1);
+        *column_at<T>(buf, h.JS, k, q) = mk<cplx<T>>(x0[0], x0[1]);
+        if (W == 2 || full) *column_at<T>(buf, h.JS, k, q + h.NQ) = mk<cplx<T>>(x1[0], x1[1]);
+        if constexpr (W == 2) {
+          unpack_rows<W - 1>(A, B, dc, x0, x1);
+          if (third) *column_at<T>(buf, h.JS, k, q + 2 * h.NQ) = mk<cplx<T>>(x0[0], x0[1]);
+          if (full) *column_at<T>(buf, h.JS, k, q + 3 * h.NQ) = mk<cplx<T>>(x1[0], x1[1]);
+        }
+      });
+    }
+  });
+  __syncthreads();
+  // first y stage
+  first_radix(h.RY1, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+    for (int t = tid; t < h.NJ * h.RY2; t += nt) {
+      const int b = fdiv(t, h.dNJ), j = t - b * h.NJ;
+      CV<T>* d = buf + j * h.JS + b;
+      CV<T> v[R];
+#pragma unroll
+      for (int s = 0; s < R; ++s) v[s] = cv_of(*reinterpret_cast<const rowvec<T>*>(d + s * h.RY2));
+      DftV<T, R, false>::run(v);
+      cv_st(d, v[0]);
+#pragma unroll
+      for (int s = 1; s < R; ++s) cv_st(d + s * h.RY2, cvtw<T, false>(v[s], taby[s * b]));
+    }
+  });
+  __syncthreads();
+  pdl_launch();
+  // second y stage, to the spectrum rows; column 0 to shared memory first
+  second_radix(h.RY2, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+    for (int t = tid; t < h.NJ * h.RY1; t += nt) {
+      const int a = fdiv(t, h.dNJ), j = t - a * h.NJ;
+      const CV<T>* d = buf + j * h.JS + a * R;
+      CV<T> v[R];
+#pragma unroll
+      for (int s = 0; s < R; ++s) v[s] = cv_ld(d + s);
+      DftV<T, R, false>::run(v);
+      cplx<T>* o = dst + (long long)(a * R) * g.KXP + W * j;
+      if (j > 0 && W * j + W <= m) {
+#pragma unroll
+        for (int s = 0; s < R; ++s) cv_row(reinterpret_cast<rowvec<T>*>(o + (long long)s * g.KXP), v[s]);
+      } else {
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+          const cplx<T> x = mk<cplx<T>>(vget<0>(v[s].re), vget<0>(v[s].im));
+          if (j == 0) col0[a * R + s] = x;
+          else o[(long long)s * g.KXP] = x;
+          if (W == 2 && W * j + 1 < m) o[(long long)s * g.KXP + 1] = mk<cplx<T>>(vget<W - 1>(v[s].re), vget<W - 1>(v[s].im));
+        }
+      }
+    }
+  });
+  __syncthreads();
+  const int *revy = posm + m, *posy = posm + m + Ly;
+  for (int sl = tid; sl < Ly; sl += nt) {
+    const int ky = __ldg(&revy[sl]), sp = __ldg(&posy[ky == 0 ? 0 : Ly - ky]);
+    cplx<T> y0, ym;
+    y_split(col0[sl], col0[sp], y0, ym);
+    dst[(long long)sl * g.KXP] = y0;
+    dst[(long long)sl * g.KXP + m] = ym;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(512, 1)
+    k_xy_inv_gen(const cplx<T>* __restrict__ spec, T* __restrict__ out, Geom g, XyGeo h, const cplx<T>* __restrict__ twx,
+                 const cplx<T>* __restrict__ twy, const int* __restrict__ posm, const Phys* __restrict__ ph,
+                 DevScalars* sc, const double* __restrict__ part_k, int nblk_k, const RepArgs* __restrict__ grp) {
+  constexpr int W = kLanes<T>;
+  pdl_wait();
+  if (grp) {
+    const RepArgs& a = grp[blockIdx.z];
+    spec = (const cplx<T>*)a.spec;
+    out = (T*)a.rwork;
+    if (ph != nullptr) ph = a.ph;
+    sc = a.sc;
+    part_k = a.part_k;
+  }
+  if (ph != nullptr && blockIdx.y == 0) {  // as k_xy_inv
+    if (blockIdx.x == 0) homo_strain_tail(ph, sc, part_k, nblk_k);
+    return;
+  }
+  FG_DYN_SMEM(smem_raw);
+  CV<T>* const buf = reinterpret_cast<CV<T>*>(smem_raw);
+  __shared__ cplx<T> tabx[kLaneMax], taby[kLaneMax], col0[kLaneMax];
+  const int nt = blockDim.x, tid = threadIdx.x;
+  const int Lx = g.Lx, Ly = g.Ly, m = g.m;
+  const int z = blockIdx.x, c = blockIdx.y - (ph != nullptr ? 1 : 0);
+  const cplx<T>* const src = spec + (long long)c * g.ncplx + (long long)z * g.plane_c;
+  T* const dst = out + (long long)c * g.nsite + (long long)z * g.plane_r;
+  const unsigned long long pol = l2_evict_first();
+  auto ldc = [&](const cplx<T>* a) {
+    if constexpr (sizeof(T) == 4 || FG_L2_HINT_FP64) return ld_first(a, pol);
+    else return *a;
+  };
+  const int *revy = posm + m, *posy = posm + m + Ly;
+  for (int sl = tid; sl < Ly; sl += nt) {
+    const int ky = __ldg(&revy[sl]), sp = __ldg(&posy[ky == 0 ? 0 : Ly - ky]);
+    const cplx<T>*r = src + (long long)sl * g.KXP, *rm = src + (long long)sp * g.KXP;
+    col0[sl] = y_join(ldc(r), ldc(rm), ldc(r + m), ldc(rm + m));
+  }
+  for (int k = tid; k < Lx; k += nt) tabx[k] = twx[k];
+  for (int k = tid; k < Ly; k += nt) taby[k] = twy[k];
+  __syncthreads();
+  second_radix(h.RY2, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+    for (int t = tid; t < h.NJ * h.RY1; t += nt) {
+      const int a = fdiv(t, h.dNJ), j = t - a * h.NJ;
+      const cplx<T>* r = src + (long long)(a * R) * g.KXP + W * j;
+      CV<T> v[R];
+#pragma unroll
+      for (int s = 0; s < R; ++s) {
+        if constexpr (sizeof(T) == 4) v[s] = cv_of(ld_first(reinterpret_cast<const float4*>(r + (long long)s * g.KXP), pol));
+        else v[s] = cv_of(ldc(r + (long long)s * g.KXP));
+      }
+      if (j == 0) {
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+          const cplx<T> x = col0[a * R + s];
+          v[s] = CV<T>{vpack(x.x, vget<W - 1>(v[s].re)), vpack(x.y, vget<W - 1>(v[s].im))};
+        }
+      }
+      DftV<T, R, true>::run(v);
+      CV<T>* d = buf + j * h.JS + a * R;
+#pragma unroll
+      for (int s = 0; s < R; ++s) cv_st(d + s, v[s]);
+    }
+  });
+  __syncthreads();
+  first_radix(h.RY1, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+    for (int t = tid; t < h.NJ * h.RY2; t += nt) {
+      const int b = fdiv(t, h.dNJ), j = t - b * h.NJ;
+      CV<T>* d = buf + j * h.JS + b;
+      CV<T> v[R];
+      v[0] = cv_ld(d);
+#pragma unroll
+      for (int s = 1; s < R; ++s) v[s] = cvtw<T, true>(cv_ld(d + s * h.RY2), taby[s * b]);
+      DftV<T, R, true>::run(v);
+#pragma unroll
+      for (int s = 0; s < R; ++s) cv_row(reinterpret_cast<rowvec<T>*>(d + s * h.RY2), v[s]);
+    }
+  });
+  __syncthreads();
+  second_radix(h.R2, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+    const int al = fdiv(tid, h.dNQ), q = tid - al * h.NQ;
+    const bool on = tid < (h.R1 / 2) * h.NQ;
+    const int a1 = al == 0 ? h.R1 / 2 : h.R1 - al;
+    CV<T> v0[R], v1[R];
+    if (on) {
+      const bool full = q + h.NQ * (2 * W - 1) < Ly, third = q + 2 * h.NQ < Ly;
+      class_columns<R>(v0, v1, al, a1, h.R1, [&](int k, CV<T>& A, CV<T>& B, bool dc) {
+        T p[2][2], n[2][2];
+#pragma unroll
+        for (int l = 0; l < W; ++l) {
+          const cplx<T> zero = mk<cplx<T>>((T)0, (T)0);
+          const cplx<T> x = l == 0 || third ? *column_at<T>(buf, h.JS, k, q + 2 * l * h.NQ) : zero;
+          const cplx<T> y = l < W - 1 || full ? *column_at<T>(buf, h.JS, k, q + (2 * l + 1) * h.NQ) : zero;
+          const T x0[2] = {x.x, x.y}, x1[2] = {y.x, y.y};
+          pack_rows(x0, x1, dc, p[l], n[l]);
+        }
+        A = CV<T>{vpack(p[0][0], p[W - 1][0]), vpack(p[0][1], p[W - 1][1])};
+        B = CV<T>{vpack(n[0][0], n[W - 1][0]), vpack(n[0][1], n[W - 1][1])};
+      });
+      DftV<T, R, true>::run(v0);
+      DftV<T, R, true>::run(v1);
+    }
+    __syncthreads();
+    if (on) {
+      CV<T>* r = buf + q * h.QS;
+#pragma unroll
+      for (int t = 0; t < R; ++t) cv_st(r + al * R + t, v0[t]);
+#pragma unroll
+      for (int t = 0; t < R; ++t) cv_st(r + a1 * R + t, v1[t]);
+    }
+  });
+  __syncthreads();
+  pdl_launch();
+  const int rows = h.NQ * Lx;
+  first_radix(h.R1, [&](auto radix) {
+    constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+    for (int t = tid; t < h.NQ * h.R2; t += nt) {
+      const int q = fdiv(t, h.dR2), b = t - q * h.R2;
+      const bool full = q + h.NQ * (2 * W - 1) < Ly, third = q + 2 * h.NQ < Ly;
+      const CV<T>* d = buf + q * h.QS + b;
+      CV<T> v[R];
+      v[0] = cv_ld(d);
+#pragma unroll
+      for (int s = 1; s < R; ++s) v[s] = cvtw<T, true>(cv_ld(d + s * h.R2), tabx[s * b]);
+      DftV<T, R, true>::run(v);
+      T* r = dst + q * Lx + b;
+#pragma unroll
+      for (int s = 0; s < R; ++s) {
+        T* o = r + s * h.R2;
+        o[0] = vget<0>(v[s].re);
+        if (W == 2 || full) o[rows] = vget<0>(v[s].im);
+        if constexpr (W == 2) {
+          if (third) o[2 * rows] = vget<W - 1>(v[s].re);
+          if (full) o[3 * rows] = vget<W - 1>(v[s].im);
+        }
+      }
+    }
+  });
+}
+
 // ------------------------------------------------- z tiles (shared helpers)
 // A z tile is CW pencils (kx slot, ky slot) with all z, nc components, held
 // in shared memory as buf[c][z][cw].  Blocks [0, nreg) take CW consecutive kx
@@ -1517,6 +1856,15 @@ __global__ void __launch_bounds__(256, 2) k_z_kspace(cplx<T>* __restrict__ spec,
 // neighbours the second stage's lanes (pw, a) fall on different banks.  The
 // stages have compile-time offsets; the k-space step works on W wavevectors
 // at a time.  Nyquist tiles (kx = Lx/2): the lanes of an element are ky slots.
+// LZ = PW = 0: a length of two stages known at run time (ZGeo, up to 160), any
+// tile of 1, 2 or 4 elements, and rows whose Lx/2 is no multiple of the tile
+// or odd (the last element of a row is then (Lx/2 - 1, Lx/2) and there are no
+// Nyquist tiles).
+struct ZGeo {
+  int R1, R2, lpw;  // stages, log2 of the elements per tile
+  int ncol;         // columns of the regular tiles: Lx/2, odd Lx/2: Lx/2 + 1
+  FastDiv d1, d2;   // by R1, R2
+};
 template <typename T, int LZ, int PW, bool ACOU>
 struct ZCT {
   static constexpr int W = kLanes<T>, NC = ACOU ? 12 : 9;
@@ -1533,15 +1881,28 @@ struct ZCT {
   static_assert(ct_nst(LZ) == 2 && R2 % 2 == 0 && NT % PW == 0, "");
 };
 
+template <typename T, bool ACOU>
+struct ZCT<T, 0, 0, ACOU> {
+  static constexpr int W = kLanes<T>, NC = ACOU ? 12 : 9, R1 = 0, R2 = 0, T1 = 0, T2 = 0, NT = 256, MINB = 2;
+};
+
 template <typename T, int LZ, int PW, bool ACOU = false>
 __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>::MINB)
     k_z_lane(cplx<T>* __restrict__ spec, const T* __restrict__ dtab, const cplx<T>* __restrict__ ckmod,
-             cplx<T>* __restrict__ acouK_out, Geom g, FftPlan, const cplx<T>* __restrict__ twz, KMaps km,
+             cplx<T>* __restrict__ acouK_out, Geom g, ZGeo h, const cplx<T>* __restrict__ twz, KMaps km,
              const Phys* __restrict__ ph, double* __restrict__ part, DevScalars* sc, ZTiles zt,
-             const T* __restrict__, const RepArgs* __restrict__ grp = nullptr) {
+             const RepArgs* __restrict__ grp = nullptr) {
   using Z = ZCT<T, LZ, PW, ACOU>;
   using V = lane_t<T>;
-  constexpr int W = Z::W, NC = Z::NC, R1 = Z::R1, R2 = Z::R2, NT = Z::NT, ZS = LZ * PW;
+  constexpr bool RT = LZ == 0;
+  constexpr int W = Z::W, NC = Z::NC, NT = Z::NT, PWM = RT ? 4 : PW;
+  const int Lz = RT ? g.Lz : LZ, pwn = RT ? 1 << h.lpw : PW, r1 = RT ? h.R1 : Z::R1, r2 = RT ? h.R2 : Z::R2;
+  const int ZS = Lz * pwn;  // (pwn: 1, 2 or 4)
+  const int swap = RT ? ~r2 & 1 : 1;  // odd R2: the lanes are apart without the swap
+  // quotients by the tile width, R1, R2 (compile-time: the compiler's)
+  auto by_pw = [&](int n) { return RT ? n >> h.lpw : n / (PW > 0 ? PW : 1); };
+  auto by_r1 = [&](int n) { return RT ? fdiv(n, h.d1) : n / (Z::R1 > 0 ? Z::R1 : 1); };
+  auto by_r2 = [&](int n) { return RT ? fdiv(n, h.d2) : n / (Z::R2 > 0 ? Z::R2 : 1); };
   if (grp) {
     const RepArgs& a = grp[blockIdx.y];
     spec = (cplx<T>*)a.spec;
@@ -1552,12 +1913,17 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
   }
   FG_DYN_SMEM(smem_raw);
   CV<T>* const buf = reinterpret_cast<CV<T>*>(smem_raw);
-  __shared__ cplx<T> tab[LZ];
-  __shared__ double sAB[PW][W][10];  // S(k) along a pencil: A_q + B_q cos kz (sin kz for yz, zx)
+  __shared__ cplx<T> tab[RT ? kLaneMax : LZ];
+  __shared__ double sAB[PWM][W][10];  // S(k) along a pencil: A_q + B_q cos kz (sin kz for yz, zx)
   __shared__ double reds[NT / 32][NQ_K];
   const int tid = threadIdx.x;
-  const int pw = tid % PW, tile = blockIdx.x;
-  stage_twiddles<T, LZ, R1, R2>(tab, twz, (T)1);
+  const int pw = tid & (pwn - 1), tile = blockIdx.x;
+  if constexpr (RT) {
+    for (int k = tid; k < Lz; k += NT) tab[k] = twz[k];
+  } else {
+    stage_twiddles<T, LZ, Z::R1, Z::R2>(tab, twz, (T)1);
+  }
+  auto twid = [&](int s, int b) { return RT ? tab[s * b] : tab[s * r2 + b]; };
   // this thread's element: slots (ys, col) and (ys, col + 1), of a Nyquist
   // tile (ys, m) and (ys + 1, m)
   const bool nyq = tile < zt.nnyq;
@@ -1567,8 +1933,11 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     ys = nyq ? tile * zt.CW + W * pw : r / zt.ntx;
     col = nyq ? g.m : (r - ys * zt.ntx) * zt.CW + W * pw;
   }
-  const bool ok = ys < g.Ly, okb = nyq && W == 2 ? ys + 1 < g.Ly : ok;
-  if (!ok) ys = 0;
+  const bool ok = ys < g.Ly && (!RT || nyq || col < h.ncol), okb = nyq && W == 2 ? ys + 1 < g.Ly : ok;
+  if (!ok) {  // an element that does not count takes zeros through a regular K(k)
+    ys = 1;
+    if (RT && !nyq) col = 0;
+  }
   const int colb = W == 2 && !nyq ? col + 1 : col, ysb = W == 2 && nyq && okb ? ys + 1 : ys;
   V k1, k2, w1;
   bool has_k0;
@@ -1576,10 +1945,10 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     k1 = vpack((T)__ldg(&km.kvx_s[col]), (T)__ldg(&km.kvx_s[colb]));
     k2 = vpack((T)__ldg(&km.kvy_s[ys]), (T)__ldg(&km.kvy_s[ysb]));
     // full-spectrum multiplicity: kx = 0 is slot 0, kx = Lx/2 slot m
-    w1 = vpack(!ok ? (T)0 : (col == 0 || nyq) ? (T)1 : (T)2, !okb ? (T)0 : nyq ? (T)1 : (T)2);
-    has_k0 = !nyq && col == 0 && ys == 0;  // lane 0 (ky = 0 is slot 0)
+    w1 = vpack(!ok ? (T)0 : (col == 0 || col == g.m) ? (T)1 : (T)2, !okb ? (T)0 : colb == g.m ? (T)1 : (T)2);
+    has_k0 = ok && !nyq && col == 0 && ys == 0;  // lane 0 (ky = 0 is slot 0)
     // S(k) of a pencil: one thread per pencil, each in a warp of its own
-    if (tid % 32 < PW && tid / 32 < W) {
+    if (tid % 32 < pwn && tid / 32 < W) {
       const double* j = ph->j;
       const double kap = ph->kap2x2;
       const double2 ty = __ldg(&km.try_s[tid / 32 == 0 ? ys : ysb]), tx = __ldg(&km.trx_s[tid / 32 == 0 ? col : colb]);
@@ -1607,44 +1976,69 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
   const unsigned zstep = (unsigned)g.plane_c * ES, cstep = (unsigned)g.ncplx * ES;
   const unsigned o0 = (unsigned)(ys * g.KXP + col) * ES, o1 = (unsigned)(ysb * g.KXP + colb) * ES;
   const unsigned long long pol = l2_evict_first();  // the input spectrum is consumed
+  // element at byte offset off of the spectrum's first z and component
+  auto gload = [&](unsigned off, auto nyqt) -> CV<T> {
+    const char* q = reinterpret_cast<const char*>(spec) + off;
+    if (!decltype(nyqt)::value && !(RT && nyq)) {
+      if (RT && !ok) return CV<T>{vall((T)0), vall((T)0)};
+      const rowvec<T>* r = reinterpret_cast<const rowvec<T>*>(q + o0);
+      if constexpr (sizeof(T) == 4) return cv_of(ld_first(r, pol));
+      else return cv_of(*r);
+    } else {
+      const cplx<T> zero = mk<cplx<T>>((T)0, (T)0);
+      const cplx<T> x = ok ? *reinterpret_cast<const cplx<T>*>(q + o0) : zero;
+      const cplx<T> y = okb ? *reinterpret_cast<const cplx<T>*>(q + o1) : zero;
+      return CV<T>{vpack(x.x, y.x), vpack(x.y, y.y)};
+    }
+  };
+  auto gstore = [&](unsigned off, const CV<T>& v, auto nyqt) {
+    char* q = reinterpret_cast<char*>(spec) + off;
+    if (!decltype(nyqt)::value && !(RT && nyq)) {
+      if (!RT || ok) cv_row(reinterpret_cast<rowvec<T>*>(q + o0), v);
+    } else {
+      if (ok) *reinterpret_cast<cplx<T>*>(q + o0) = mk<cplx<T>>(vget<0>(v.re), vget<0>(v.im));
+      if (W == 2 && okb) *reinterpret_cast<cplx<T>*>(q + o1) = mk<cplx<T>>(vget<W - 1>(v.re), vget<W - 1>(v.im));
+    }
+  };
+  // tasks 0 .. count-1 (compile-time COUNT, or rt at run time)
+  auto tasks = [&](auto count, int rt, auto&& f) {
+    if constexpr (RT) {
+#pragma unroll 1
+      for (int t = tid; t < rt; t += NT) f(t);
+    } else {
+      lane_tasks<decltype(count)::value, NT>(tid, f);
+    }
+  };
   // forward: first stage from the spectrum
-  auto first = [&](auto nyqt) {
-    lane_tasks<Z::T1, NT>(tid, [&](int t) {
-      const int b = t / PW % R2, c = t / (PW * R2);
+  auto first = [&](auto nyqt, auto radix) {
+    constexpr int R = decltype(radix)::value;
+    tasks(std::integral_constant<int, Z::T1>(), NC * pwn * r2, [&](int t) {
+      const int r = by_pw(t), c = by_r2(r), b = r - c * r2, bx = b ^ swap;
       unsigned off = c * cstep + b * zstep;
-      CV<T> v[R1];
+      CV<T> v[R];
 #pragma unroll
-      for (int s = 0; s < R1; ++s, off += R2 * zstep) {
-        const char* q = reinterpret_cast<const char*>(spec) + off;
-        if constexpr (!decltype(nyqt)::value) {
-          const rowvec<T>* r = reinterpret_cast<const rowvec<T>*>(q + o0);
-          if constexpr (sizeof(T) == 4) v[s] = cv_of(ld_first(r, pol));
-          else v[s] = cv_of(*r);
-        } else {
-          const cplx<T> zero = mk<cplx<T>>((T)0, (T)0);
-          const cplx<T> x = ok ? *reinterpret_cast<const cplx<T>*>(q + o0) : zero;
-          const cplx<T> y = okb ? *reinterpret_cast<const cplx<T>*>(q + o1) : zero;
-          v[s] = CV<T>{vpack(x.x, y.x), vpack(x.y, y.y)};
-        }
-      }
-      DftV<T, R1, false>::run(v);
+      for (int s = 0; s < R; ++s, off += r2 * zstep) v[s] = gload(off, nyqt);
+      DftV<T, R, false>::run(v);
       CV<T>* d = buf + c * ZS + pw;
-      cv_st(d + b * PW, v[0]);
+      cv_st(d + b * pwn, v[0]);
 #pragma unroll
-      for (int s = 1; s < R1; ++s)
-        cv_st(d + (((s & 1) ? b ^ 1 : b) + R2 * s) * PW, cvtw<T, false>(v[s], tab[s * R2 + b]));
+      for (int s = 1; s < R; ++s) cv_st(d + (((s & 1) ? bx : b) + r2 * s) * pwn, cvtw<T, false>(v[s], twid(s, b)));
     });
   };
-  if (nyq) first(std::true_type());
-  else first(std::false_type());
+  if constexpr (RT) {
+    first_radix(r1, [&](auto radix) { first(std::false_type(), radix); });
+  } else {
+    if (nyq) first(std::true_type(), std::integral_constant<int, Z::R1>());
+    else first(std::false_type(), std::integral_constant<int, Z::R1>());
+  }
   // The dipole table's 6 values of W neighbouring slots, [slot / W][6][W], of
   // this thread's k-space element e: the next one's are loaded while the
   // strain part of the present one is computed
   V D[6];
   auto load_D = [&](int e) {
-    const unsigned tz = (unsigned)(e / PW) * g.KXP;
+    const unsigned tz = (unsigned)by_pw(e) * g.KXP;
     if (!nyq) {
-      const CV<T>* Dp = reinterpret_cast<const CV<T>*>(dtab + ((size_t)(ys * LZ * g.KXP) + tz + col) * 6);
+      const CV<T>* Dp = reinterpret_cast<const CV<T>*>(dtab + ((size_t)ys * Lz * g.KXP + tz + col) * 6);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const CV<T> v = cv_stream(Dp + q);
@@ -1654,25 +2048,33 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     } else {
 #pragma unroll
       for (int q = 0; q < 6; ++q)
-        D[q] = vpack(dtab[tab_index<T>((long long)ys * LZ * g.KXP + tz + col, q)],
-                     dtab[tab_index<T>((long long)ysb * LZ * g.KXP + tz + colb, q)]);
+        D[q] = vpack(dtab[tab_index<T>((long long)ys * Lz * g.KXP + tz + col, q)],
+                     dtab[tab_index<T>((long long)ysb * Lz * g.KXP + tz + colb, q)]);
     }
   };
-  if (tid < LZ * PW) load_D(tid);
+  if (tid < ZS) load_D(tid);
   __syncthreads();
-  auto second = [&](auto inv) {
-    lane_tasks<Z::T2, NT>(tid, [&](int t) {
-      const int a = t / PW % R1, c = t / (PW * R1), x = a & 1;
-      CV<T>*d0 = buf + c * ZS + pw + (a * R2 + x) * PW, *d1 = d0 - 2 * x * PW;  // z even / odd of the block
-      CV<T> v[R2];
+  auto second = [&](auto inv, auto radix) {
+    constexpr int R = decltype(radix)::value;
+    tasks(std::integral_constant<int, Z::T2>(), NC * pwn * r1, [&](int t) {
+      const int r = by_pw(t), c = by_r1(r), a = r - c * r1, x = a & swap;
+      CV<T>*d0 = buf + c * ZS + pw + (a * r2 + x) * pwn, *d1 = d0 - 2 * x * pwn;  // z even / odd of the block
+      CV<T> v[R];
 #pragma unroll
-      for (int q = 0; q < R2; ++q) v[q] = cv_ld(((q & 1) ? d1 : d0) + q * PW);
-      DftV<T, R2, decltype(inv)::value>::run(v);
+      for (int q = 0; q < R; ++q) v[q] = cv_ld(((q & 1) ? d1 : d0) + q * pwn);
+      DftV<T, R, decltype(inv)::value>::run(v);
 #pragma unroll
-      for (int q = 0; q < R2; ++q) cv_st(((q & 1) ? d1 : d0) + q * PW, v[q]);
+      for (int q = 0; q < R; ++q) cv_st(((q & 1) ? d1 : d0) + q * pwn, v[q]);
     });
   };
-  second(std::false_type());
+  auto second_stage = [&](auto inv) {
+    if constexpr (RT) {
+      if (r2 > 1) second_radix(r2, [&](auto radix) { second(inv, radix); });
+    } else {
+      second(inv, std::integral_constant<int, Z::R2>());
+    }
+  };
+  second_stage(std::false_type());
   __syncthreads();
   // ---- k space
   const double Ninv = ph->Ninv;
@@ -1682,9 +2084,9 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
   const bool mod = ph->modulation_on != 0;
   double acc[NQ_K] = {0, 0, 0, 0, 0};
 #pragma unroll 1
-  for (int e = tid; e < LZ * PW; e += NT) {
-    const int zs = e / PW, zx = zs ^ (zs / R2 & 1);
-    CV<T>* el = buf + zx * PW + pw;
+  for (int e = tid; e < ZS; e += NT) {
+    const int zs = by_pw(e), zx = zs ^ (by_r2(zs) & swap);
+    CV<T>* el = buf + zx * pwn + pw;
     CV<T> u[3], d[6];
 #pragma unroll
     for (int a = 0; a < 3; ++a) u[a] = cv_ld(el + a * ZS);
@@ -1722,7 +2124,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
       cv_st(el + a * ZS, CV<T>{vfma(D[a], u[a].re, vfma(dab, u[b].re, vmul(dac, u[c].re))),
                                vfma(D[a], u[a].im, vfma(dab, u[b].im, vmul(dac, u[c].im)))});
     }
-    if (e + NT < LZ * PW) load_D(e + NT);
+    if (e + NT < ZS) load_D(e + NT);
     // ---- inhomogeneous strain
 #pragma unroll
     for (int i = 0; i < 6; ++i) d[i] = cv_ld(el + (3 + i) * ZS);
@@ -1760,7 +2162,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
       if (mod) {
 #pragma unroll
         for (int l = 0; l < W; ++l)
-          m[l] = ckmod[((long long)(l == 0 ? ys : ysb) * LZ * g.KXP + tz + (l == 0 ? col : colb)) * 3 + a];
+          m[l] = ckmod[((long long)(l == 0 ? ys : ysb) * Lz * g.KXP + tz + (l == 0 ? col : colb)) * 3 + a];
       }
       ck[a] = CV<T>{vpack(m[0].x, m[1].x), vpack(m[0].y, m[1].y)};
     }
@@ -1835,9 +2237,9 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     if (acouK_out) {
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        if (ok) acouK_out[((long long)ys * LZ * g.KXP + tz + col) * 3 + a] = mk<cplx<T>>(vget<0>(acou[a].re), vget<0>(acou[a].im));
+        if (ok) acouK_out[((long long)ys * Lz * g.KXP + tz + col) * 3 + a] = mk<cplx<T>>(vget<0>(acou[a].re), vget<0>(acou[a].im));
         if (W == 2 && okb)
-          acouK_out[((long long)ysb * LZ * g.KXP + tz + colb) * 3 + a] = mk<cplx<T>>(vget<W - 1>(acou[a].re), vget<W - 1>(acou[a].im));
+          acouK_out[((long long)ysb * Lz * g.KXP + tz + colb) * 3 + a] = mk<cplx<T>>(vget<W - 1>(acou[a].re), vget<W - 1>(acou[a].im));
       }
     }
     // inhoK = k (x) acou / N
@@ -1866,7 +2268,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
   }
   __syncthreads();
   // inverse: the last forward stage first, the first one to the spectrum
-  second(std::true_type());
+  second_stage(std::true_type());
   if (tid < NQ_K) {
     double s = 0.0;
     for (int w = 0; w < NT / 32; ++w) s += reds[w][tid];
@@ -1874,32 +2276,27 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
   }
   __syncthreads();
   pdl_launch();
-  auto last = [&](auto nyqt) {
-    lane_tasks<Z::T1, NT>(tid, [&](int t) {
-      const int b = t / PW % R2, c = t / (PW * R2);
+  auto last = [&](auto nyqt, auto radix) {
+    constexpr int R = decltype(radix)::value;
+    tasks(std::integral_constant<int, Z::T1>(), NC * pwn * r2, [&](int t) {
+      const int r = by_pw(t), c = by_r2(r), b = r - c * r2, bx = b ^ swap;
       const CV<T>* d = buf + c * ZS + pw;
-      CV<T> v[R1];
-      v[0] = cv_ld(d + b * PW);
+      CV<T> v[R];
+      v[0] = cv_ld(d + b * pwn);
 #pragma unroll
-      for (int s = 1; s < R1; ++s)
-        v[s] = cvtw<T, true>(cv_ld(d + (((s & 1) ? b ^ 1 : b) + R2 * s) * PW), tab[s * R2 + b]);
-      DftV<T, R1, true>::run(v);
+      for (int s = 1; s < R; ++s) v[s] = cvtw<T, true>(cv_ld(d + (((s & 1) ? bx : b) + r2 * s) * pwn), twid(s, b));
+      DftV<T, R, true>::run(v);
       unsigned off = c * cstep + b * zstep;
 #pragma unroll
-      for (int s = 0; s < R1; ++s, off += R2 * zstep) {
-        char* q = reinterpret_cast<char*>(spec) + off;
-        if constexpr (!decltype(nyqt)::value) {
-          cv_row(reinterpret_cast<rowvec<T>*>(q + o0), v[s]);
-        } else {
-          if (ok) *reinterpret_cast<cplx<T>*>(q + o0) = mk<cplx<T>>(vget<0>(v[s].re), vget<0>(v[s].im));
-          if (W == 2 && okb)
-            *reinterpret_cast<cplx<T>*>(q + o1) = mk<cplx<T>>(vget<W - 1>(v[s].re), vget<W - 1>(v[s].im));
-        }
-      }
+      for (int s = 0; s < R; ++s, off += r2 * zstep) gstore(off, v[s], nyqt);
     });
   };
-  if (nyq) last(std::true_type());
-  else last(std::false_type());
+  if constexpr (RT) {
+    first_radix(r1, [&](auto radix) { last(std::false_type(), radix); });
+  } else {
+    if (nyq) last(std::true_type(), std::integral_constant<int, Z::R1>());
+    else last(std::false_type(), std::integral_constant<int, Z::R1>());
+  }
 }
 
 // ------------------------------------------------------------------ k_assemble
