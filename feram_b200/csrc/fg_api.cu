@@ -201,6 +201,7 @@ struct fg_ctx {
   double* part_r = nullptr;
   double* part_ke = nullptr;
   double* part_avg = nullptr;
+  double* didi = nullptr;         // Geom::didi (mixed path)
   unsigned int* done = nullptr;   // last-block tickets: [0] kicks, [1] z k-space, [2] assemble
   double* avg6 = nullptr;
   double* staging = nullptr;      // padded Fortran-layout FP64 (3 components)
@@ -778,6 +779,7 @@ RepArgs rep_args(const fg_ctx* c) {
   a.done_as = c->done + 2;
   a.layer_minv = c->layer_minv;
   a.layer_sump = c->layer_sump;
+  a.didi = c->didi;
   return a;
 }
 
@@ -1237,6 +1239,14 @@ int create_impl(fg_ctx* ctx) {
   CK(cudaMalloc(&ctx->part_r, sizeof(double) * NQ_R * (size_t)ctx->grid_elem));
   CK(cudaMalloc(&ctx->part_ke, sizeof(double) * 3 * (size_t)ctx->grid_elem));
   CK(cudaMalloc(&ctx->part_avg, sizeof(double) * 6 * (size_t)ctx->grid_elem));
+  if (sizeof(T) == 4) {  // one row per warp of launch_xy_fwd's blocks
+    int nt = ctx->xyg.nt;
+    if (nt == 0) with_xy_fwd<T, SRC_U9>(g.m, g.Ly, [&](auto, int n) { nt = n; });
+    g.didi_rows = g.Lz * (nt / 32);
+    CK(cudaMalloc(&ctx->didi, sizeof(double) * 9 * (size_t)g.didi_rows));
+  }
+  g.didi = ctx->didi;
+  g.k0_exact = sizeof(T) == 4 ? 1 : 0;
   CK(cudaMalloc(&ctx->avg6, sizeof(double) * 6));
   CK(cudaMalloc(&ctx->done, sizeof(unsigned int) * 4));
   CK(cudaMemset(ctx->done, 0, sizeof(unsigned int) * 4));
@@ -1580,6 +1590,7 @@ int set_zsite(fg_ctx* ctx, bool on) {
   ctx->smem_z = smem_z;
   ctx->smem_z3 = (int)(3 * (size_t)g.Lz * zt.CW * sizeof(cplx<T>));
   ctx->zsite = on;
+  ctx->g.k0_exact = sizeof(T) == 4 && !on ? 1 : 0;  // Z* u has no plane sums
   ctx->ltab_ready = false;
   CK(cudaMalloc(&ctx->spec, (size_t)ncx * sizeof(cplx<T>) * (size_t)g.ncplx));
   CK(cudaMemsetAsync(ctx->spec, 0, (size_t)ncx * sizeof(cplx<T>) * (size_t)g.ncplx, ctx->stream));
@@ -1836,7 +1847,7 @@ void fg_destroy(fg_ctx* ctx) {
                   ctx->twm, ctx->twy, ctx->twz, ctx->twx64, ctx->twm64, ctx->twy64, ctx->twz64, ctx->L64, ctx->ltab, ctx->revx,
                   ctx->revy, ctx->revz, ctx->posm, ctx->kvx, ctx->kvy, ctx->kvz, ctx->trx, ctx->try_, ctx->trz, ctx->trz_s, ctx->kvz_s,
                   ctx->layer_minv, ctx->layer_sump, ctx->ph, ctx->sc, ctx->part_k, ctx->part_r, ctx->part_ke,
-                  ctx->part_avg, ctx->avg6, ctx->staging, ctx->dipoRavg, ctx->done, ctx->layer_macou, ctx->layer_all,
+                  ctx->part_avg, ctx->didi, ctx->avg6, ctx->staging, ctx->dipoRavg, ctx->done, ctx->layer_macou, ctx->layer_all,
                   ctx->site_minv, ctx->site_macou, ctx->site_sump, ctx->site_species, ctx->site_zstar, ctx->site_E,
                   ctx->layer_nsum, ctx->samples};
   for (void* b : bufs)

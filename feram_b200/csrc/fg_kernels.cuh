@@ -38,6 +38,15 @@ struct Geom {
   long long nsite;    // Lx*Ly*Lz
   long long ncplx;    // Lz*Ly*KXP
   long long nkpos;    // Ly*Lz*KXP
+  // Mixed path: FP64 sums of u and u u, [didi_rows][9], one row per warp of a
+  // plane's block, written by the forward x-y pass and summed by
+  // homo_strain_tail (null: FP64 path, whose spectra have them).  The homogeneous strain and the k = 0 part of the
+  // dipole energies follow these nine numbers; their FP32 rounding (4e-8 of
+  // the k = 0 spectrum) moved the energies by 1e-3 eV from step to step at 64^3,
+  // the largest part of the thermostat's error.  k0_exact: the k-space pass
+  // leaves k = 0 out of the dipole energies and the tail adds it.
+  int k0_exact, didi_rows;
+  double* didi;
 };
 
 // Constants of the Hamiltonian and integrators, resident on the device.
@@ -80,6 +89,7 @@ struct DevScalars {
   double strain[6];
   double w_hom[6];    // sum_i strain_i * HC2(i, j)
   double didiK0[6];   // Re didiK(k = 0)
+  double D0[6];       // the dipole table at k = 0 (Geom::k0_exact)
   double E[3];        // uniform external field
   double ke_sum;      // last masked sum p^2/m
   // Nose-Poincare half step (35a), (38), (35c) of the next step, prepared by
@@ -115,6 +125,7 @@ struct RepArgs {
   unsigned int* done_as;  // k_assemble's last-block ticket
   const double* layer_minv;
   const unsigned char* layer_sump;
+  double* didi;           // Geom::didi of the replica
 };
 
 // ---------------------------------------------------------------- reductions
@@ -124,7 +135,7 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Block-wide sum of NQ values; thread 0 writes part[blockid*NQ + q].
+// Block-wide sum of NQ values; thread q < NQ writes part[blockid*NQ + q].
 // Fixed reduction order, so results are reproducible run to run.
 template <int NQ>
 __device__ void block_partials(double* v, double* part, long long blockid) {
@@ -136,13 +147,11 @@ __device__ void block_partials(double* v, double* part, long long blockid) {
     if (lane == 0) red[wid][q] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int q = 0; q < NQ; ++q) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += red[w][q];
-      part[blockid * NQ + q] = s;
-    }
+  if (threadIdx.x < NQ) {
+    const int q = threadIdx.x, nw = (blockDim.x + 31) >> 5;
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += red[w][q];
+    part[blockid * NQ + q] = s;
   }
   __syncthreads();
 }
@@ -158,12 +167,11 @@ __device__ void block_partials2(const double* va, const double* vb, double* pa, 
     if (lane == 0) red[wid][q] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < NA + NB; ++q) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += red[w][q];
-      (q < NA ? pa[blockid * NA + q] : pb[blockid * NB + q - NA]) = s;
-    }
+  if (threadIdx.x < NA + NB) {
+    const int q = threadIdx.x;
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += red[w][q];
+    (q < NA ? pa[blockid * NA + q] : pb[blockid * NB + q - NA]) = s;
   }
   __syncthreads();
 }
@@ -191,46 +199,85 @@ __device__ double reduce_partials(const double* part, int nblk, int NQ, int q) {
 static_assert(sizeof(DevScalars) % 8 == 0, "DevScalars is copied as doubles");
 static_assert(sizeof(Phys) % 8 == 0, "Phys is copied as doubles");
 // The reduction of one or two sets of block partials (columns 0 .. NA-1 from
-// pa, then NB from pb) and the scalar work on the totals v[NA + NB]: the loads
-// of the constants and scalars are in flight with those of the partials, so a
-// tail costs one round trip to the L2, not two.
-template <int NA, int NB, class F>
+// the nblk rows of pa, then NB from the nblk_b rows of pb) and the scalar work
+// on the totals v[NA + NB]: the loads of the constants and scalars are in
+// flight with those of the partials, so a tail costs one round trip to the
+// L2, not two.  Lane l of a warp takes column l % PA (PB) of the rows its
+// thread index selects: 3 to 7 shuffles a warp, where every thread taking whole
+// rows needs 5 per column (14 columns: 140 instructions a warp, all in one
+// SM's shuffle unit).  The loads are batched by hand: left to the compiler
+// they went out one by one (28 us for 64^3's plane sums, 14 batched).  body
+// runs on the first LANES threads.
+// Step of 16^3, mixed: 22.5 -> 21.5 us with this and the nine plane sums that
+// cost 1.7 us before it.
+template <int N>
+struct PadCols {
+  static constexpr int value = N <= 1 ? 1 : N <= 2 ? 2 : N <= 4 ? 4 : N <= 8 ? 8 : 16;
+};
+// The thread's sums of both sets, 8 loads of each in flight.
+template <int NA, int NB>
+__device__ __forceinline__ void column_sums(const double* __restrict__ pa, int na, const double* __restrict__ pb, int nb,
+                                            double* sa, double* sb) {
+  constexpr int PA = PadCols<NA>::value, PB = PadCols<NB>::value, U = 8;
+  const int ca = threadIdx.x % PA, ra = blockDim.x / PA;
+  const int cb = threadIdx.x % PB, rb = blockDim.x / PB;
+  int ia = threadIdx.x / PA, ib = threadIdx.x / PB;
+  if (ca >= NA) ia = na;
+  if (NB == 0 || cb >= NB) ib = nb;
+  *sa = *sb = 0.0;
+  while (ia < na || ib < nb) {
+    double a[U], b[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int i = ia + k * ra, j = ib + k * rb;
+      a[k] = i < na ? __ldcg(&pa[(long long)i * NA + ca]) : 0.0;
+      b[k] = NB > 0 && j < nb ? __ldcg(&pb[(long long)j * NB + cb]) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      *sa += a[k];
+      *sb += b[k];
+    }
+    ia += U * ra;
+    ib += U * rb;
+  }
+}
+template <int N>
+__device__ __forceinline__ double column_warp_sum(double s) {
+#pragma unroll
+  for (int o = 16; o >= PadCols<N>::value; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  return s;
+}
+template <int NA, int NB, int LANES = 1, class F>
 __device__ __forceinline__ void reduced_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ pa,
-                                             const double* __restrict__ pb, int nblk, F&& body) {
+                                             const double* __restrict__ pb, int nblk, int nblk_b, F&& body) {
   constexpr int NQ = NA + NB;
   __shared__ Phys sph;
   __shared__ DevScalars ssc;
-  __shared__ double red[32][NQ];
+  __shared__ double red[NQ][32];
   __shared__ double tot[NQ];
   constexpr int NP = (int)(sizeof(Phys) / 8), NS = (int)(sizeof(DevScalars) / 8);
   for (int i = threadIdx.x; i < NP; i += blockDim.x)
     reinterpret_cast<double*>(&sph)[i] = __ldg(reinterpret_cast<const double*>(ph) + i);
   for (int i = threadIdx.x; i < NS; i += blockDim.x)
     reinterpret_cast<double*>(&ssc)[i] = __ldcg(reinterpret_cast<const double*>(sc) + i);
-  double s[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) s[q] = 0.0;
-#pragma unroll 4
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-#pragma unroll
-    for (int q = 0; q < NA; ++q) s[q] += __ldcg(&pa[(long long)b * NA + q]);
-#pragma unroll
-    for (int q = 0; q < NB; ++q) s[NA + q] += __ldcg(&pb[(long long)b * NB + q]);
-  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    const double t = warp_sum(s[q]);
-    if (lane == 0) red[wid][q] = t;
+  double sa, sb;
+  column_sums<NA, NB>(pa, nblk, pb, nblk_b, &sa, &sb);
+  const double ta = column_warp_sum<NA>(sa);
+  if (lane < NA) red[lane][wid] = ta;
+  if constexpr (NB > 0) {
+    const double tb = column_warp_sum<NB>(sb);
+    if (lane < NB) red[NA + lane][wid] = tb;
   }
   __syncthreads();
   if (threadIdx.x < NQ) {
     double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += red[w][threadIdx.x];
+    for (int w = 0; w < nw; ++w) t += red[threadIdx.x][w];
     tot[threadIdx.x] = t;
   }
   __syncthreads();
-  if (threadIdx.x == 0) body(static_cast<const Phys*>(&sph), &ssc, tot);
+  if (threadIdx.x < LANES) body(static_cast<const Phys*>(&sph), &ssc, tot);
   __syncthreads();
   for (int i = threadIdx.x; i < NS; i += blockDim.x)
     reinterpret_cast<double*>(sc)[i] = reinterpret_cast<const double*>(&ssc)[i];
@@ -240,9 +287,9 @@ __device__ __forceinline__ void reduced_tail(const Phys* __restrict__ ph, DevSca
 // takes a ticket; the block drawing the last ticket sees all of them and
 // finishes the grid-wide work (classic threadfence reduction, no waiting).
 // The counter is reset for the next launch by that block.  Only thread 0
-// fences: the tails read nothing but the partials thread 0 wrote (and values
-// whose writers fence themselves), so the other threads retire without
-// waiting for their bulk stores to drain.
+// fences, after the barrier that puts the partials' stores by the block's
+// first warp before it: the tails read nothing but those partials (and values
+// whose writers fence themselves).
 __device__ __forceinline__ bool is_last_block(unsigned int* counter) {
   __shared__ bool last;
   __syncthreads();
@@ -276,7 +323,8 @@ __host__ __device__ inline void short_range_k(const double* j, double kap2x2, co
 }
 
 __device__ __noinline__ void homo_strain_tail(const Phys* __restrict__ ph, DevScalars* sc,
-                                              const double* __restrict__ part_k, int nblk);
+                                              const double* __restrict__ part_k, int nblk,
+                                              const double* __restrict__ didi, const Geom g);
 
 // ------------------------------------------------------------------ k_xy_fwd
 enum { SRC_U9 = 0, SRC_FIELD = 1 };
@@ -487,6 +535,30 @@ __device__ __forceinline__ void columns_to_class(const CV<T>* buf, CV<T>* lo, CV
   }
 }
 
+// Sum of an element's values (of FP32 lanes: the mixed path's plane sums).
+__device__ __forceinline__ float cv_sum(const CV<float>* v, int n) {
+  F2 a = v[0].re, b = v[0].im;
+#pragma unroll
+  for (int s = 1; s < n; ++s) {
+    a = vadd(a, v[s].re);
+    b = vadd(b, v[s].im);
+  }
+  a = vadd(a, b);
+  return vget<0>(a) + vget<1>(a);
+}
+__device__ __forceinline__ double cv_sum(const CV<double>*, int) { return 0.0; }
+// Geom::didi entry of component c of plane z's first warp, null where there
+// is none; every warp writes its own row.
+template <typename T, int MODE>
+__device__ __forceinline__ double* plane_didi(const Geom& g, const RepArgs* grp, int c, int z) {
+  if (MODE != 0 || sizeof(T) != 4 || g.didi == nullptr || c > 8) return nullptr;
+  return (grp ? grp[blockIdx.z].didi : g.didi) + (long long)z * (blockDim.x / 32) * 9 + c;
+}
+__device__ __forceinline__ void plane_sum(double s, double* didi) {
+  s = warp_sum(s);
+  if (threadIdx.x % 32 == 0) didi[threadIdx.x / 32 * 9] = s;
+}
+
 // Forward transform of one plane: pa (and, for products, pb) the real rows,
 // dst the plane's spectrum rows.  128^2 FP32: 256 threads, 2 CTAs per SM.
 enum { PLANE_PLAIN = 0, PLANE_SQUARE = 1, PLANE_PRODUCT = 2 };
@@ -494,11 +566,12 @@ template <typename T, int MC, int LYC>
 __device__ __forceinline__ void xy_fwd_ct(const T* __restrict__ pa, const T* __restrict__ pb, int kind,
                                           cplx<T>* __restrict__ dst, int kxp, unsigned char* smem,
                                           const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twy,
-                                          const int* __restrict__ posm) {
+                                          const int* __restrict__ posm, double* __restrict__ didi) {
   using C = XyCT<T, MC, LYC>;
   constexpr int NT = C::NT, R1 = C::R1, R2 = C::R2, RY1 = C::RY1, RY2 = C::RY2, W = C::W;
   CV<T>* buf = reinterpret_cast<CV<T>*>(smem);
   __shared__ cplx<T> tabx[R1 * C::NB], taby[LYC], col0[LYC];
+  double sum = 0.0;
   stage_twiddles<T, C::LX, R1, C::NB>(tabx, twx, (T)0.5);  // halved: see unpack_rows
   stage_twiddles<T, LYC, RY1, RY2>(taby, twy, (T)1);
   __syncthreads();
@@ -521,6 +594,7 @@ __device__ __forceinline__ void xy_fwd_ct(const T* __restrict__ pa, const T* __r
 #pragma unroll
       for (int s = 0; s < R1; ++s) v[s] = CV<T>{vmul(v[s].re, v[s].re), vmul(v[s].im, v[s].im)};
     }
+    if (didi) sum += (double)cv_sum(v, R1);
     DftV<T, R1, false>::run(v);
     CV<T>* d = buf + q * C::QS + b;
     const lane_t<T> half = vall((T)0.5);
@@ -528,6 +602,7 @@ __device__ __forceinline__ void xy_fwd_ct(const T* __restrict__ pa, const T* __r
 #pragma unroll
     for (int s = 1; s < R1; ++s) cv_st(d + s * R2, cvtw<T, false>(v[s], tabx[s * C::NB + bg]));
   });
+  if (didi) plane_sum(sum, didi);
   __syncthreads();
   // second x stage with the separation of the rows
   {
@@ -729,13 +804,15 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
   cplx<T>* dst = spec + (long long)(out_comp0 + c) * g.ncplx + (long long)z * g.plane_c;
   if constexpr (MC > 0) {
     const int kind = plain ? PLANE_PLAIN : (!zu && c < 6) ? PLANE_SQUARE : PLANE_PRODUCT;
-    xy_fwd_ct<T, MC, LYC>(pa, pb, kind, dst, g.KXP, smem_raw, twx, twy, posm);
+    xy_fwd_ct<T, MC, LYC>(pa, pb, kind, dst, g.KXP, smem_raw, twx, twy, posm, plane_didi<T, MODE>(g, grp, c, z));
   } else {
     pdl_wait();
     cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
     const int m = g.m, Ly = g.Ly, RS = m + 1, Lx = 2 * m;
     const int buf_len = Ly * RS;
     const int total = Ly * m;
+    double* const didi = plane_didi<T, MODE>(g, grp, c, z);
+    double sum = 0.0;
     if (plain) {
       // asynchronous copies of packed (x even, x odd) pairs
       for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
@@ -743,6 +820,12 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
         cp_async<(int)sizeof(cplx<T>)>(&buf[y * RS + jx], pa + (long long)y * Lx + 2 * jx);
       }
       cp_async_wait();
+      if (didi)  // this thread's own copies
+        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+          const int y = idx / m;
+          const cplx<T> v = buf[y * RS + idx - y * m];
+          sum += (double)(v.x + v.y);
+        }
     } else {
       // products: kLB independent loads in flight per thread, then compute
       constexpr int kLB = 4;
@@ -763,11 +846,14 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
           const int idx = base + r * blockDim.x;
           if (idx < total) {
             const int y = idx / m, jx = idx - y * m;
-            buf[y * RS + jx] = mk<cplx<T>>(va[r].x * vb[r].x, va[r].y * vb[r].y);
+            const cplx<T> v = mk<cplx<T>>(va[r].x * vb[r].x, va[r].y * vb[r].y);
+            if (didi) sum += (double)(v.x + v.y);
+            buf[y * RS + jx] = v;
           }
         }
       }
     }
+    if (didi) plane_sum(sum, didi);
     // X pass; row stride RS = m+1 keeps the row-interleaved mapping bank-conflict free
     __syncthreads();
     Batch B{Ly, 1, 0, RS, 1, true};
@@ -834,7 +920,7 @@ __global__ void __launch_bounds__(xy_threads<T, MC, LYC>(), xy_min_blocks<T, MC,
   // from that pass's block partials (nothing in this kernel needs them;
   // k_assemble does), beside the transforms instead of ahead of a plane's.
   if (ph != nullptr && blockIdx.y == 0) {
-    if (blockIdx.x == 0) homo_strain_tail(ph, sc, part_k, nblk_k);
+    if (blockIdx.x == 0) homo_strain_tail(ph, sc, part_k, nblk_k, grp && g.didi ? grp[blockIdx.z].didi : g.didi, g);
     return;
   }
   FG_DYN_SMEM(smem_raw);
@@ -953,6 +1039,8 @@ __global__ void __launch_bounds__(512, 1)
   const int nt = blockDim.x, tid = threadIdx.x;
   const int Lx = g.Lx, Ly = g.Ly, m = g.m;
   const int z = blockIdx.x, c = blockIdx.y;
+  double* const didi = plane_didi<T, MODE>(g, grp, c, z);
+  double sum = 0.0;
   for (int k = tid; k < Lx; k += nt) tabx[k] = mk<cplx<T>>((T)0.5 * twx[k].x, (T)0.5 * twx[k].y);  // halved: unpack_rows
   for (int k = tid; k < Ly; k += nt) taby[k] = twy[k];
   __syncthreads();
@@ -991,6 +1079,7 @@ __global__ void __launch_bounds__(512, 1)
           v[s] = CV<T>{vmul(v[s].re, w.re), vmul(v[s].im, w.im)};
         }
       }
+      if (didi) sum += (double)cv_sum(v, R);
       DftV<T, R, false>::run(v);
       CV<T>* d = buf + q * h.QS + b;
       const lane_t<T> half = vall((T)0.5);
@@ -999,6 +1088,7 @@ __global__ void __launch_bounds__(512, 1)
       for (int s = 1; s < R; ++s) cv_st(d + s * h.R2, cvtw<T, false>(v[s], tabx[s * b]));
     }
   });
+  if (didi) plane_sum(sum, didi);
   __syncthreads();
   // second x stage with the separation of the rows
   second_radix(h.R2, [&](auto radix) {
@@ -1104,7 +1194,7 @@ __global__ void __launch_bounds__(512, 1)
     part_k = a.part_k;
   }
   if (ph != nullptr && blockIdx.y == 0) {  // as k_xy_inv
-    if (blockIdx.x == 0) homo_strain_tail(ph, sc, part_k, nblk_k);
+    if (blockIdx.x == 0) homo_strain_tail(ph, sc, part_k, nblk_k, grp && g.didi ? grp[blockIdx.z].didi : g.didi, g);
     return;
   }
   FG_DYN_SMEM(smem_raw);
@@ -1334,24 +1424,42 @@ __device__ __forceinline__ void check_finite(DevScalars* sc, const double* v, in
 // After the k-space pass: k-space energies, homogeneous strain
 // (optimize-homo-strain.F:27-186) and w_hom for k_assemble.
 __device__ __noinline__ void homo_strain_tail(const Phys* __restrict__ ph, DevScalars* sc,
-                                              const double* __restrict__ part_k, int nblk) {
-  reduced_tail<NQ_K, 0>(ph, sc, part_k, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
-    double* e = S->e;
-    const double es = v[0] * P->Ninv / 2;  // (1/2N) sum w' Re(uK* S uK)
-    const double edd = v[1] / 2;           // (1/2)  sum w' Re(uK* D uK), D = (S + Z*^2 L)/N
-    e[E_SHORT] = es;
-    e[E_LONG] = edd - es;
-    e[E_IS] = v[2] * P->Ninv;
-    e[E_IC] = v[3] * 2 * P->Ninv;
-    e[E_IM] = P->modulation_on ? v[4] * 2 * P->Ninv : 0.0;
-    double hc2uu[6];
-    for (int i = 0; i < 6; ++i) {
-      double t = 0.0;
-      for (int jj = 0; jj < 6; ++jj) t += P->HC2[i][jj] * S->didiK0[jj];
-      hc2uu[i] = t;
+                                              const double* __restrict__ part_k, int nblk,
+                                              const double* __restrict__ didi, const Geom g) {
+  // On one warp: lane i has row i of the products, every lane the energies and
+  // the triangular solves; stores at the end, so that all loads go ahead of
+  // the chain.
+  reduced_tail<NQ_K, 9, 32>(ph, sc, part_k, didi, nblk, didi ? g.didi_rows : 0,
+                            [&](const Phys* P, DevScalars* S, const double* v) {
+    double es = v[0], edd = v[1];
+    if (g.k0_exact) {  // S(0) has no off-diagonal entries
+      const double* U = v + NQ_K;
+      const double one[3] = {1.0, 1.0, 1.0}, zero[3] = {0.0, 0.0, 0.0};
+      double S0[6];
+      short_range_k(P->j, P->kap2x2, one, zero, S0);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const int b = (a + 1) % 3, c = (a + 2) % 3;  // off-diagonal slots: yz 3, zx 4, xy 5
+        es += S0[a] * (U[a] * U[a]);
+        edd += S->D0[a] * (U[a] * U[a]) + 2 * S->D0[3 + a] * (U[b] * U[c]);
+      }
     }
-    for (int i = 0; i < 3; ++i) hc2uu[i] = hc2uu[i] + P->pNa03[i];
-    double* st = S->strain;
+    es = es * P->Ninv / 2;  // (1/2N) sum w' Re(uK* S uK)
+    edd = edd / 2;          // (1/2)  sum w' Re(uK* D uK), D = (S + Z*^2 L)/N
+    const int i = threadIdx.x % 6;
+    const double* dd = didi ? v + NQ_K + 3 : S->didiK0;
+    double d[6], hcol[6], hrow[6], hc2uu[6], st[6];
+    double t = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      d[j] = dd[j];
+      hcol[j] = P->HC2[j][i];
+      hrow[j] = P->H[i][j];
+      t += P->HC2[i][j] * d[j];
+    }
+    if (i < 3) t += P->pNa03[i];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) hc2uu[j] = lane_value(t, j);
     const double(*H)[6] = P->H;
     if (P->bulk_or_film == 2) {  // epit
       st[0] = P->epi_strain;
@@ -1372,32 +1480,44 @@ __device__ __noinline__ void homo_strain_tail(const Phys* __restrict__ ph, DevSc
       st[1] = P->epi_strain + delta;
       st[5] = -2 * delta;
     } else {
-      for (int i = 0; i < 6; ++i) st[i] = -hc2uu[i];
-      for (int i = 0; i < 6; ++i) {
-        double t = 0.0;
-        for (int jj = 0; jj < i; ++jj) t = t + P->HG[i][jj] * st[jj];
-        st[i] = (st[i] - t) * P->HG_inv[i];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        double x = 0.0;
+#pragma unroll
+        for (int c = 0; c < r; ++c) x = x + P->HG[r][c] * st[c];
+        st[r] = (-hc2uu[r] - x) * P->HG_inv[r];
       }
-      for (int i = 5; i >= 0; --i) {
-        double t = 0.0;
-        for (int jj = i + 1; jj < 6; ++jj) t = t + st[jj] * P->HG[jj][i];
-        st[i] = (st[i] - t) * P->HG_inv[i];
+#pragma unroll
+      for (int r = 5; r >= 0; --r) {
+        double x = 0.0;
+#pragma unroll
+        for (int c = r + 1; c < 6; ++c) x = x + st[c] * P->HG[c][r];
+        st[r] = (st[r] - x) * P->HG_inv[r];
       }
     }
-    double hs = 0.0;
-    for (int i = 0; i < 6; ++i) {
-      double d = 0.0;
-      for (int jj = 0; jj < 6; ++jj) d += H[i][jj] * st[jj];
-      hs = hs + st[i] * d;
+    double hd = 0.0, w = 0.0, hs = 0.0, hc = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      hd += hrow[j] * st[j];
+      w = w + st[j] * hcol[j];
+      hc += st[j] * hc2uu[j];
     }
-    e[E_HS] = hs / 2;
-    double hc = 0.0;
-    for (int i = 0; i < 6; ++i) hc += st[i] * hc2uu[i];
-    e[E_HC] = hc;
-    for (int jj = 0; jj < 6; ++jj) {
-      double w = 0.0;
-      for (int i = 0; i < 6; ++i) w = w + st[i] * P->HC2[i][jj];
-      S->w_hom[jj] = w;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) hs = hs + st[j] * lane_value(hd, j);
+    if (threadIdx.x < 6) S->w_hom[threadIdx.x] = w;
+    if (threadIdx.x == 0) {
+      S->e[E_SHORT] = es;
+      S->e[E_LONG] = edd - es;
+      S->e[E_IS] = v[2] * P->Ninv;
+      S->e[E_IC] = v[3] * 2 * P->Ninv;
+      S->e[E_IM] = P->modulation_on ? v[4] * 2 * P->Ninv : 0.0;
+      S->e[E_HS] = hs / 2;
+      S->e[E_HC] = hc;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {
+        S->strain[j] = st[j];
+        S->didiK0[j] = d[j];
+      }
     }
   });
 }
@@ -1468,14 +1588,14 @@ __device__ __forceinline__ void np_close_body(const Phys* P, DevScalars* S, cons
 
 __device__ __noinline__ void force_energies_tail(const Phys* __restrict__ ph, DevScalars* sc,
                                                  const double* __restrict__ part_r, int nblk, bool np_close) {
-  reduced_tail<NQ_R, 0>(ph, sc, part_r, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+  reduced_tail<NQ_R, 0>(ph, sc, part_r, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     force_energies_body(P, S, v);
     if (np_close) np_post_body(P, S, 1.0 / S->pend_s, log(S->pend_s));
   });
 }
 __device__ __noinline__ void np_close_tail(const Phys* __restrict__ ph, DevScalars* sc,
                                            const double* __restrict__ part, int nblk, bool step_done) {
-  reduced_tail<3, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+  reduced_tail<3, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     np_close_body(P, S, v, 1.0 / S->s, log(S->s), step_done);
   });
 }
@@ -1483,7 +1603,7 @@ __device__ __noinline__ void np_close_tail(const Phys* __restrict__ ph, DevScala
 __device__ __noinline__ void np_step_tail(const Phys* __restrict__ ph, DevScalars* sc,
                                           const double* __restrict__ part_r, const double* __restrict__ part_ke,
                                           int nblk) {
-  reduced_tail<NQ_R, 3>(ph, sc, part_r, part_ke, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+  reduced_tail<NQ_R, 3>(ph, sc, part_r, part_ke, nblk, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
     const double inv_s = 1.0 / S->pend_s, log_s = log(S->pend_s);
     force_energies_body(P, S, v);
     np_post_body(P, S, inv_s, log_s);
@@ -1495,7 +1615,7 @@ __device__ __noinline__ void np_step_tail(const Phys* __restrict__ ph, DevScalar
 // momenta, the factor sqrt(target / KE) for k_scale, total.  The reported
 // dipo_kinetic is the value before rescaling, as in the reference.
 __device__ void vs_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk) {
-  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     S->ke_sum = v[0];
     S->e[E_DIPO] = ke_from(P, v[0]);
     S->vs_scale = sqrt(P->target_ke / S->e[E_DIPO]);
@@ -1509,7 +1629,7 @@ __device__ void vs_tail(const Phys* __restrict__ ph, DevScalars* sc, const doubl
 // with vs also the rescale factor (velocity_scaling.F:86-98) and the total.
 __device__ void acou_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk,
                           bool vs) {
-  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     S->e[E_ACOU] = v[0] / 2;
     if (vs) {
       S->vs_scale_acou = sqrt(P->target_ke / S->e[E_ACOU]);
@@ -1521,7 +1641,7 @@ __device__ void acou_tail(const Phys* __restrict__ ph, DevScalars* sc, const dou
 
 // Leapfrog closing reduction (leapfrog.F:151) and total.
 __device__ void lf_final_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk) {
-  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
+  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     S->ke_sum = v[0];
     S->e[E_DIPO] = ke_from(P, v[0]);
     S->e[E_TOT] = S->e[E_DIPO] / (S->s * S->s) + S->e[E_ACOU] + sum_potential(S->e);
@@ -1692,7 +1812,13 @@ __global__ void __launch_bounds__(256, 2) k_z_kspace(cplx<T>* __restrict__ spec,
       double qd[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) qd[q] = (double)qv[q];
-      const double es = (double)w1 * (S[0] * qd[0] + S[1] * qd[1] + S[2] * qd[2] + 2.0 * (S[3] * qd[3] + S[4] * qd[4] + S[5] * qd[5]));
+      const bool tail_k0 = !ZSC && k0 && g.k0_exact;
+      if (tail_k0) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sc->D0[q] = (double)D[q];
+      }
+      const double we = tail_k0 ? 0.0 : (double)w1;
+      const double es = we * (S[0] * qd[0] + S[1] * qd[1] + S[2] * qd[2] + 2.0 * (S[3] * qd[3] + S[4] * qd[4] + S[5] * qd[5]));
       acc[0] += es;
       if constexpr (ZSC) {
         // short range on uK, long range on FFT(Z* u): Fl = (L/N) ZuK,
@@ -1719,7 +1845,7 @@ __global__ void __launch_bounds__(256, 2) k_z_kspace(cplx<T>* __restrict__ spec,
 #pragma unroll
         for (int q = 0; q < 6; ++q) D[q] = (T)(S[q] * Ninv);
       } else {
-        acc[1] += (double)w1 * ((double)D[0] * qd[0] + (double)D[1] * qd[1] + (double)D[2] * qd[2] +
+        acc[1] += we * ((double)D[0] * qd[0] + (double)D[1] * qd[1] + (double)D[2] * qd[2] +
                                 2.0 * ((double)D[3] * qd[3] + (double)D[4] * qd[4] + (double)D[5] * qd[5]));
       }
     }
@@ -2091,6 +2217,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
 #pragma unroll
     for (int a = 0; a < 3; ++a) u[a] = cv_ld(el + a * ZS);
     const long long tz = (long long)zs * g.KXP;  // table positions of the element's lanes
+    const bool k0 = has_k0 && zs == 0;           // slot 0 holds kz = 0
     {
       // Re(conj(u_a) u_b): xx, yy, zz, yz, zx, xy
       const V qv[6] = {vfma(u[0].re, u[0].re, vmul(u[0].im, u[0].im)), vfma(u[1].re, u[1].re, vmul(u[1].im, u[1].im)),
@@ -2108,7 +2235,12 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
           qd[q] = (double)vget<L>(qv[q]);
           dd[q] = (double)vget<L>(D[q]);
         }
-        const double w = (double)vget<L>(w1);
+        double w = (double)vget<L>(w1);
+        if (L == 0 && k0 && g.k0_exact) {  // left to homo_strain_tail
+#pragma unroll
+          for (int q = 0; q < 6; ++q) sc->D0[q] = dd[q];
+          w = 0.0;
+        }
         acc[0] += w * ((a[0] + a[6] * tzc.x) * qd[0] + (a[1] + a[7] * tzc.x) * qd[1] + (a[2] + a[8] * tzc.x) * qd[2] +
                        2.0 * (a[3] * tzc.y * qd[3] + a[4] * tzc.y * qd[4] + (a[5] + a[9] * tzc.x) * qd[5]));
         acc[1] += w * (dd[0] * qd[0] + dd[1] * qd[1] + dd[2] * qd[2] + 2.0 * (dd[3] * qd[3] + dd[4] * qd[4] + dd[5] * qd[5]));
@@ -2128,7 +2260,6 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     // ---- inhomogeneous strain
 #pragma unroll
     for (int i = 0; i < 6; ++i) d[i] = cv_ld(el + (3 + i) * ZS);
-    const bool k0 = has_k0 && zs == 0;  // slot 0 holds kz = 0
     if (k0) {
 #pragma unroll
       for (int i = 0; i < 6; ++i) sc->didiK0[i] = (double)vget<0>(d[i].re);
@@ -2408,10 +2539,26 @@ __device__ __forceinline__ T force_hi(double o) { return (T)o; }
 template <typename T>
 __device__ __forceinline__ T force_lo(double o, T hi) { return sizeof(T) == 4 ? (T)(o - (double)hi) : (T)0; }
 
+// A kick or drift coefficient, FP64, times a field value in T.  FP32: the
+// coefficient's rounding would be the same error on every site (6e-8 of each
+// kick, which the energy sums up coherently), so its low part is kept; the
+// product is rounded once per site.
+template <typename T> struct StepCoef;
+template <> struct StepCoef<double> {
+  double c;
+  __device__ __forceinline__ explicit StepCoef(double v) : c(v) {}
+  __device__ __forceinline__ double operator*(double x) const { return c * x; }
+};
+template <> struct StepCoef<float> {
+  float hi, lo;
+  __device__ __forceinline__ explicit StepCoef(double v) : hi((float)v), lo((float)(v - (double)hi)) {}
+  __device__ __forceinline__ float operator*(float x) const { return fmaf(hi, x, lo * x); }
+};
+
 // Masked kinetic sums of the closing kick (35f) of one site: p <- p - c F
 // and p^2/m, p.F/m, F^2/m in T, added to ke (FP64) when the site counts.
 template <typename T>
-__device__ __forceinline__ void close_site(T* __restrict__ p, long long ns, long long i, T c, T o0, T o1, T o2,
+__device__ __forceinline__ void close_site(T* __restrict__ p, long long ns, long long i, const StepCoef<T>& c, T o0, T o1, T o2,
                                            bool counted, double mi, double* ke) {
   const T q0 = p[i] - c * o0, q1 = p[ns + i] - c * o1, q2 = p[2 * ns + i] - c * o2;
   p[i] = q0;
@@ -2463,7 +2610,7 @@ __global__ void __launch_bounds__(256, 2)
   const long long ns = g.nsite;
   // pend_kick_f: prepared by the previous step's tail, not changed by this
   // step's commit
-  const T cf = CLOSE ? (T)__ldcg(&sc->pend_kick_f) : (T)0;
+  const StepCoef<T> cf(CLOSE ? __ldcg(&sc->pend_kick_f) : 0.0);
   double ke[3] = {0.0, 0.0, 0.0};
   const unsigned long long pol_rw = l2_evict_first();
   // k: the static constants (kernel parameter, built by asm_const on the
@@ -2637,7 +2784,7 @@ __global__ void __launch_bounds__(256) k_kick(T* __restrict__ p, const T* __rest
   // site_minv / site_sump: per-site masses and masks (.relaxor, .defects)
   // instead of the per-layer tables; they take the scalar loop.
   const long long ns = g.nsite;
-  const T c = (T)(*coef);
+  const StepCoef<T> c(*coef);
   double acc[1] = {0.0};
   constexpr int NV = V16<T>::n;
   using AV = V16<T>;
@@ -2810,7 +2957,7 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
     layer_minv = a.layer_minv;
   }
   const long long ns = g.nsite;
-  const T ck = (T)sc->kick_coef;
+  const StepCoef<T> ck(sc->kick_coef);
   const double cd = sc->pend_drift;
   constexpr int NV = V16<T>::n;
   using AV = V16<T>;
@@ -2818,7 +2965,7 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
   if (g.plane_r % NV == 0 && site_minv == nullptr) {
     for (long long iv = (long long)blockIdx.x * blockDim.x + threadIdx.x; iv < ns / NV; iv += stride) {
       const long long i = iv * NV;
-      const T f = (T)(cd * layer_minv[(int)(i / g.plane_r)]);
+      const StepCoef<T> f(cd * layer_minv[(int)(i / g.plane_r)]);
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         V16<T> q = ldv(p + a * ns + i), x = ldv(u + a * ns + i);
@@ -2834,7 +2981,7 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
     }
   } else {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
-      const T f = (T)(cd * (site_minv ? (double)site_minv[i] : layer_minv[(int)(i / g.plane_r)]));
+      const StepCoef<T> f(cd * (site_minv ? (double)site_minv[i] : layer_minv[(int)(i / g.plane_r)]));
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const T q = p[a * ns + i] - ck * F[a * ns + i];
@@ -2866,7 +3013,7 @@ __global__ void __launch_bounds__(256) k_kick_close(T* __restrict__ p, const T* 
   if (!PREP && blockIdx.x == 0) force_energies_tail(ph, sc, part_r, nblk_r, true);
   const long long ns = g.nsite;
   // pend_kick_f is not changed by block 0's commit
-  const T c = PREP ? (T)0 : (T)__ldcg(&sc->pend_kick_f);
+  const StepCoef<T> c(PREP ? 0.0 : __ldcg(&sc->pend_kick_f));
   double acc[3] = {0.0, 0.0, 0.0};
   constexpr int NV = V16<T>::n;
   using AV = V16<T>;
@@ -2938,7 +3085,7 @@ __global__ void __launch_bounds__(256) k_drift(T* __restrict__ u, const T* __res
   if (g.plane_r % NV == 0 && site_minv == nullptr) {
     for (long long iv = (long long)blockIdx.x * blockDim.x + threadIdx.x; iv < ns / NV; iv += stride) {
       const long long i = iv * NV;
-      const T f = (T)(c * layer_minv[(int)(i / g.plane_r)]);
+      const StepCoef<T> f(c * layer_minv[(int)(i / g.plane_r)]);
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         V16<T> x = ldv(u + a * ns + i);
@@ -2951,7 +3098,7 @@ __global__ void __launch_bounds__(256) k_drift(T* __restrict__ u, const T* __res
   } else {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
       const int z = (int)(i / g.plane_r);
-      const T f = (T)(c * (site_minv ? (double)site_minv[i] : layer_minv[z]));
+      const StepCoef<T> f(c * (site_minv ? (double)site_minv[i] : layer_minv[z]));
       u[i] = u[i] + f * p[i];
       u[ns + i] = u[ns + i] + f * p[ns + i];
       u[2 * ns + i] = u[2 * ns + i] + f * p[2 * ns + i];
