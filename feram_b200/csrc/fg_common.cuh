@@ -61,10 +61,6 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-// v of lane `lane`, the whole warp converged
-__device__ __forceinline__ double lane_value(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
-#else
-inline double lane_value(double v, int) { return v; }  // the emulated launches run no scalar tails
 #endif  // FG_HOST_EMU
 
 // L2 eviction priority for data read once and not needed again before it is

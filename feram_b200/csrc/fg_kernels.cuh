@@ -135,6 +135,13 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// v of lane `lane`, the whole warp converged
+#ifndef FG_HOST_EMU
+__device__ __forceinline__ double lane_value(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+#else
+inline double lane_value(double v, int) { return v; }  // the emulated launches run no scalar tails
+#endif
+
 // Block-wide sum of NQ values; thread q < NQ writes part[blockid*NQ + q].
 // Fixed reduction order, so results are reproducible run to run.
 template <int NQ>
