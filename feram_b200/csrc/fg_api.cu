@@ -196,7 +196,6 @@ struct fg_ctx {
   Phys ph_host{};
   DevScalars* sc = nullptr;
   DevScalars* sc_host = nullptr;  // pinned
-  double* E_host = nullptr;       // pinned staging of fg_set_uniform_E
   double* part_k = nullptr;
   double* part_r = nullptr;
   double* part_ke = nullptr;
@@ -525,7 +524,7 @@ AsmConst asm_const(const fg_ctx* ctx) {
 
 // flo: also store the FP32 residual of the force (mixed path)
 template <typename T, bool CLOSE>
-void launch_assemble(fg_ctx* ctx, int tail, bool flo = false) {
+void launch_assemble(fg_ctx* ctx, int tail, bool flo = false, DevScalars* host = nullptr) {
   const bool sites = ctx->site_species || ctx->site_zstar || ctx->site_E ||
                      (CLOSE && (ctx->site_minv || ctx->site_sump));
   launch_dep(ctx, sites ? k_assemble<T, CLOSE, true> : k_assemble<T, CLOSE, false>,
@@ -533,7 +532,7 @@ void launch_assemble(fg_ctx* ctx, int tail, bool flo = false) {
              ctx->done + 2, ctx->site_species, (const T*)ctx->site_zstar, (const T*)ctx->site_E,
              ctx->zsite ? zu_comp(ctx) : 0, (T*)ctx->p, ctx->layer_minv, ctx->layer_sump, (const T*)ctx->site_minv,
              ctx->site_sump, ctx->part_ke, (flo && sizeof(T) == 4) ? (T*)ctx->Flo : (T*)nullptr, asm_const(ctx),
-             (const RepArgs*)nullptr);
+             (const RepArgs*)nullptr, host);
 }
 
 // Force modes: FORCE_PLAIN finishes the energies in k_assemble's tail;
@@ -542,9 +541,10 @@ void launch_assemble(fg_ctx* ctx, int tail, bool flo = false) {
 enum { FORCE_PLAIN = 0, FORCE_NP_POST = 1, FORCE_NP_CLOSE = 2 };
 
 // flo: the force-only evaluation of fg_mirror_force_mirror, which keeps the
-// FP32 residual of the mixed path's force for fg_get_state
+// FP32 residual of the mixed path's force for fg_get_state; host: the host's
+// copy of the scalars, if the last tail is to write it
 template <typename T>
-int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false) {
+int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false, DevScalars* host = nullptr) {
   const Geom& g = ctx->g;
   cudaStream_t st = ctx->stream;
   T* u = (T*)ctx->u;
@@ -559,8 +559,8 @@ int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false) {
     return rc;
   if ((rc = launch_z_kspace<T>(ctx, ctx->store_acouK ? (cplx<T>*)ctx->acouK : nullptr))) return rc;
   if ((rc = launch_xy_inv<T>(ctx, (const cplx<T>*)ctx->spec, (T*)ctx->rwork, ctx->ncx, true))) return rc;
-  if (mode == FORCE_NP_CLOSE) launch_assemble<T, true>(ctx, TAIL_NONE);
-  else launch_assemble<T, false>(ctx, mode == FORCE_NP_POST ? TAIL_NONE : TAIL_ENERGIES, flo);
+  if (mode == FORCE_NP_CLOSE) launch_assemble<T, true>(ctx, TAIL_NONE, false, host);
+  else launch_assemble<T, false>(ctx, mode == FORCE_NP_POST ? TAIL_NONE : TAIL_ENERGIES, flo, host);
   CKL();
   if (ctx->P.bulk_or_film == FG_FILM || ctx->P.bulk_or_film == FG_EPIT) {
     k_mirror<T><<<ctx->grid_elem, kThreadsElem, 0, st>>>((T*)ctx->F, g, ctx->P.gap_id);
@@ -643,10 +643,10 @@ int enqueue_kick_drift(fg_ctx* ctx) {
 
 // prep: sums of the current state only (np_prepare)
 template <typename T, bool PREP>
-int enqueue_kick_close(fg_ctx* ctx) {
+int enqueue_kick_close(fg_ctx* ctx, DevScalars* host = nullptr) {
   launch_dep(ctx, k_kick_close<T, PREP>, ctx->grid_kc, kThreadsElem, 0,
       (T*)ctx->p, (const T*)ctx->F, ctx->g, ctx->layer_minv, ctx->layer_sump, ctx->part_ke, ctx->done, ctx->ph,
-      ctx->sc, ctx->part_r, ctx->grid_as, (const T*)ctx->site_minv, ctx->site_sump);
+      ctx->sc, ctx->part_r, ctx->grid_as, (const T*)ctx->site_minv, ctx->site_sump, host);
   CKL();
   return FG_OK;
 }
@@ -665,7 +665,7 @@ int enqueue_kick_close(fg_ctx* ctx) {
 // of several steps, and its first kernel does the same after the previous
 // step's closing kick.
 template <typename T>
-int enqueue_np(fg_ctx* ctx, bool follows_step = false) {
+int enqueue_np(fg_ctx* ctx, bool follows_step = false, DevScalars* host = nullptr) {
   const bool pdl = !ctx->bulk_or_film_mirror();
   int rc = enqueue_wave(ctx);
   if (rc) return rc;
@@ -675,8 +675,8 @@ int enqueue_np(fg_ctx* ctx, bool follows_step = false) {
   // bulk: the closing kick runs inside k_assemble; films mirror the force
   // first, so the kick is a kernel of its own
   const bool fused = !ctx->bulk_or_film_mirror();
-  if (!rc) rc = enqueue_force<T>(ctx, fused ? FORCE_NP_CLOSE : FORCE_NP_POST);
-  if (!rc && !fused) rc = enqueue_kick_close<T, false>(ctx);
+  if (!rc) rc = enqueue_force<T>(ctx, fused ? FORCE_NP_CLOSE : FORCE_NP_POST, false, fused ? host : nullptr);
+  if (!rc && !fused) rc = enqueue_kick_close<T, false>(ctx, host);
   ctx->pdl = false;
   return rc;
 }
@@ -742,7 +742,7 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
              (const T*)nullptr, (T*)nullptr, g, (const Phys*)nullptr, (DevScalars*)nullptr, (double*)nullptr,
              (int)TAIL_NONE, (unsigned int*)nullptr, (const unsigned char*)nullptr, (const T*)nullptr,
              (const T*)nullptr, 0, (T*)nullptr, (const double*)nullptr, (const unsigned char*)nullptr,
-             (const T*)nullptr, (const unsigned char*)nullptr, (double*)nullptr, (T*)nullptr, asm_const(c0), grp);
+             (const T*)nullptr, (const unsigned char*)nullptr, (double*)nullptr, (T*)nullptr, asm_const(c0), grp, (DevScalars*)nullptr);
   CKL();
   c0->pdl = false;
   return FG_OK;
@@ -803,10 +803,14 @@ int run_graph(fg_ctx* ctx, cudaGraphExec_t* gx, int which) {
   int rc = FG_OK;
   if (which == 0) {
     rc = capture(ctx, gx, [&] {
-      return ctx->prec == FG_PREC_MIXED ? enqueue_force<float>(ctx, FORCE_PLAIN, true) : enqueue_force<double>(ctx);
+      return ctx->prec == FG_PREC_MIXED ? enqueue_force<float>(ctx, FORCE_PLAIN, true, ctx->sc_host)
+                                        : enqueue_force<double>(ctx, FORCE_PLAIN, false, ctx->sc_host);
     });
   } else if (which == 1) {
-    rc = capture(ctx, gx, [&] { return ctx->prec == FG_PREC_MIXED ? enqueue_np<float>(ctx) : enqueue_np<double>(ctx); });
+    rc = capture(ctx, gx, [&] {
+      return ctx->prec == FG_PREC_MIXED ? enqueue_np<float>(ctx, false, ctx->sc_host)
+                                        : enqueue_np<double>(ctx, false, ctx->sc_host);
+    });
   } else if (which == 4) {
     rc = capture(ctx, gx, [&] {
       int r = FG_OK;
@@ -824,8 +828,10 @@ int run_graph(fg_ctx* ctx, cudaGraphExec_t* gx, int which) {
   return FG_OK;
 }
 
-int pull_scalars(fg_ctx* ctx) {
-  CK(cudaMemcpyAsync(ctx->sc_host, ctx->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
+// Waits for the stream, whose work has left the scalars in sc_host (a graph
+// whose last tail writes them there, a copy enqueued before), and looks at
+// their status.
+int wait_scalars(fg_ctx* ctx) {
   CK(cudaStreamSynchronize(ctx->stream));
   int rc = check_device_error(ctx);
   if (rc) return rc;
@@ -833,6 +839,11 @@ int pull_scalars(fg_ctx* ctx) {
     return fail(ctx, FG_ERR_NAN, "Nose-Poincare update (38): 1 - CB dt/Q < 0, Q_Nose is too small for this supercell");
   if (ctx->sc_host->status == FG_ERR_NAN) return fail(ctx, FG_ERR_NAN, "non-finite energy in a device reduction");
   return FG_OK;
+}
+
+int pull_scalars(fg_ctx* ctx) {
+  CK(cudaMemcpyAsync(ctx->sc_host, ctx->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
+  return wait_scalars(ctx);
 }
 
 int push_scalars(fg_ctx* ctx) {
@@ -1201,7 +1212,6 @@ int create_impl(fg_ctx* ctx) {
   // scalars
   CK(cudaMalloc(&ctx->sc, sizeof(DevScalars)));
   CK(cudaMallocHost(&ctx->sc_host, sizeof(DevScalars)));
-  CK(cudaMallocHost(&ctx->E_host, 3 * sizeof(double)));
   std::memset(ctx->sc_host, 0, sizeof(DevScalars));
   ctx->sc_host->s = 1.0;
   ctx->sc_host->pi = 0.0;
@@ -1388,37 +1398,53 @@ int set_modulation_flag(fg_ctx* ctx, int on) {
   return FG_OK;
 }
 
+// The copy through the staging buffer is enqueued only: src stays in use until
+// the caller has waited for the stream.
 template <typename T>
-int set_field(fg_ctx* ctx, void* dst, const double* src) {
+int enqueue_set_field(fg_ctx* ctx, void* dst, const double* src) {
   const size_t nin = (size_t)3 * ctx->NXP * ctx->NYP * ctx->P.Lz;
   CK(cudaMemcpyAsync(ctx->staging, src, sizeof(double) * nin, cudaMemcpyHostToDevice, ctx->stream));
   k_fortran_to_soa<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>((T*)dst, ctx->staging, ctx->g, 3, ctx->NXP,
                                                                          ctx->NYP);
   CKL();
-  CK(cudaStreamSynchronize(ctx->stream));
   return FG_OK;
 }
 
 template <typename T>
-int get_field(fg_ctx* ctx, double* dst, const void* src) {
+int set_field(fg_ctx* ctx, void* dst, const double* src) {
+  const int rc = enqueue_set_field<T>(ctx, dst, src);
+  if (rc) return rc;
+  CK(cudaStreamSynchronize(ctx->stream));
+  return FG_OK;
+}
+
+// dst holds the field once the caller has waited for the stream.
+template <typename T>
+int enqueue_get_field(fg_ctx* ctx, double* dst, const void* src) {
   const size_t nin = (size_t)3 * ctx->NXP * ctx->NYP * ctx->P.Lz;
   k_soa_to_fortran<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>(ctx->staging, (const T*)src, ctx->g, 3,
                                                                          ctx->NXP, ctx->NYP);
   CKL();
   CK(cudaMemcpyAsync(dst, ctx->staging, sizeof(double) * nin, cudaMemcpyDeviceToHost, ctx->stream));
+  return FG_OK;
+}
+
+template <typename T>
+int get_field(fg_ctx* ctx, double* dst, const void* src) {
+  const int rc = enqueue_get_field<T>(ctx, dst, src);
+  if (rc) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   return FG_OK;
 }
 
 // A field held as hi + lo (the mixed path's force after fg_mirror_force_mirror)
 template <typename T>
-int get_field2(fg_ctx* ctx, double* dst, const void* hi, const void* lo) {
+int enqueue_get_field2(fg_ctx* ctx, double* dst, const void* hi, const void* lo) {
   const size_t nin = (size_t)3 * ctx->NXP * ctx->NYP * ctx->P.Lz;
   k_soa2_to_fortran<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>(ctx->staging, (const T*)hi, (const T*)lo,
                                                                           ctx->g, 3, ctx->NXP, ctx->NYP);
   CKL();
   CK(cudaMemcpyAsync(dst, ctx->staging, sizeof(double) * nin, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
   return FG_OK;
 }
 
@@ -1853,7 +1879,6 @@ void fg_destroy(fg_ctx* ctx) {
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (ctx->sc_host) cudaFreeHost(ctx->sc_host);
-  if (ctx->E_host) cudaFreeHost(ctx->E_host);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -1938,25 +1963,29 @@ int fg_time_fft(fg_ctx* ctx, int reps, double* ms) {
   return ctx->prec == FG_PREC_MIXED ? time_fft_impl<float>(ctx, reps, ms) : time_fft_impl<double>(ctx, reps, ms);
 }
 
-int fg_set_state(fg_ctx* ctx, const double* dipoR, const double* dipoP, double s, double pi, double H0) {
-  if (!ctx || !ctx->stream) return FG_ERR_ARG;
-  int rc;
-  if (dipoR) {
-    rc = ctx->prec == FG_PREC_MIXED ? set_field<float>(ctx, ctx->u, dipoR) : set_field<double>(ctx, ctx->u, dipoR);
-    if (rc) return rc;
-  }
-  if (dipoP) {
-    rc = ctx->prec == FG_PREC_MIXED ? set_field<float>(ctx, ctx->p, dipoP) : set_field<double>(ctx, ctx->p, dipoP);
-    if (rc) return rc;
-  }
-  if ((rc = pull_scalars(ctx))) return rc;
+// s, pi and H0 on the device and in sc_host, and the momentum kick they imply
+static int set_thermostat(fg_ctx* ctx, double s, double pi, double H0) {
   ctx->sc_host->s = s;
   ctx->sc_host->pi = pi;
   ctx->sc_host->H0 = H0;
   ctx->sc_host->kick_coef = ctx->P.dt_2 * s;
-  if ((rc = push_scalars(ctx))) return rc;
-  ctx->force_fresh = false;
+  k_set_thermostat<<<1, 32, 0, ctx->stream>>>(ctx->sc, s, pi, H0, ctx->P.dt_2 * s);
+  CKL();
   ctx->np_ready = false;
+  return FG_OK;
+}
+
+int fg_set_state(fg_ctx* ctx, const double* dipoR, const double* dipoP, double s, double pi, double H0) {
+  if (!ctx || !ctx->stream) return FG_ERR_ARG;
+  // one wait for both fields and the scalars
+  const bool f32 = ctx->prec == FG_PREC_MIXED;
+  int rc = FG_OK;
+  if (dipoR) rc = f32 ? enqueue_set_field<float>(ctx, ctx->u, dipoR) : enqueue_set_field<double>(ctx, ctx->u, dipoR);
+  if (!rc && dipoP) rc = f32 ? enqueue_set_field<float>(ctx, ctx->p, dipoP) : enqueue_set_field<double>(ctx, ctx->p, dipoP);
+  if (rc) cudaStreamSynchronize(ctx->stream);  // no copy of the caller's arrays outlives the call
+  if (rc || (rc = pull_scalars(ctx))) return rc;
+  if ((rc = set_thermostat(ctx, s, pi, H0))) return rc;
+  ctx->force_fresh = false;
   return FG_OK;
 }
 
@@ -1964,12 +1993,7 @@ int fg_set_thermostat(fg_ctx* ctx, double s, double pi, double H0) {
   if (!ctx || !ctx->stream) return FG_ERR_ARG;
   int rc;
   if ((rc = pull_scalars(ctx))) return rc;
-  ctx->sc_host->s = s;
-  ctx->sc_host->pi = pi;
-  ctx->sc_host->H0 = H0;
-  ctx->sc_host->kick_coef = ctx->P.dt_2 * s;
-  ctx->np_ready = false;
-  return push_scalars(ctx);
+  return set_thermostat(ctx, s, pi, H0);
 }
 
 int fg_get_params(const fg_ctx* ctx, fg_params* p) {
@@ -2054,15 +2078,16 @@ int fg_get_state(fg_ctx* ctx, double* dipoR, double* dipoP, double* dVddi, doubl
                  double* H0) {
   if (!ctx || !ctx->stream) return FG_ERR_ARG;
   int rc;
+  // one wait for all fields and the scalars
   const bool f32 = ctx->prec == FG_PREC_MIXED;
-  if (dipoR && (rc = f32 ? get_field<float>(ctx, dipoR, ctx->u) : get_field<double>(ctx, dipoR, ctx->u))) return rc;
-  if (dipoP && (rc = f32 ? get_field<float>(ctx, dipoP, ctx->p) : get_field<double>(ctx, dipoP, ctx->p))) return rc;
-  if (dVddi) {
-    if (f32 && ctx->flo_valid) rc = get_field2<float>(ctx, dVddi, ctx->F, ctx->Flo);
-    else rc = f32 ? get_field<float>(ctx, dVddi, ctx->F) : get_field<double>(ctx, dVddi, ctx->F);
-    if (rc) return rc;
-  }
-  if ((rc = pull_scalars(ctx))) return rc;
+  auto get = [&](double* dst, const void* src) {
+    return f32 ? enqueue_get_field<float>(ctx, dst, src) : enqueue_get_field<double>(ctx, dst, src);
+  };
+  rc = dipoR ? get(dipoR, ctx->u) : FG_OK;
+  if (!rc && dipoP) rc = get(dipoP, ctx->p);
+  if (!rc && dVddi) rc = f32 && ctx->flo_valid ? enqueue_get_field2<float>(ctx, dVddi, ctx->F, ctx->Flo) : get(dVddi, ctx->F);
+  if (rc) cudaStreamSynchronize(ctx->stream);
+  if (rc || (rc = pull_scalars(ctx))) return rc;
   if (strain)
     for (int i = 0; i < 6; ++i) strain[i] = ctx->sc_host->strain[i];
   if (s) *s = ctx->sc_host->s;
@@ -2128,12 +2153,10 @@ int fg_get_acouK(fg_ctx* ctx, double* acouK) {
 }
 
 int fg_set_uniform_E(fg_ctx* ctx, const double E[3]) {
-  if (!ctx || !ctx->stream || !ctx->E_host || !E) return FG_ERR_ARG;
-  // Staged in pinned memory and copied in stream order, without waiting:
-  // every call that reads results synchronises the stream, and a second
-  // fg_set_uniform_E before the copy ran only makes the later field win.
-  for (int a = 0; a < 3; ++a) ctx->E_host[a] = ctx->sc_host->E[a] = E[a];  // sc_host: for push_scalars
-  CK(cudaMemcpyAsync(ctx->sc->E, ctx->E_host, 3 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  if (!ctx || !ctx->stream || !ctx->sc_host || !E) return FG_ERR_ARG;
+  for (int a = 0; a < 3; ++a) ctx->sc_host->E[a] = E[a];  // for push_scalars
+  k_set_field<<<1, 32, 0, ctx->stream>>>(ctx->sc, E[0], E[1], E[2]);
+  CKL();
   // The stored dVddi and energies stay those of the last evaluation, as
   // c%dVddi does when molecular-dynamics.F:66-76 changes c%E_field between
   // steps: the next force evaluation sees the new field.
@@ -2176,7 +2199,7 @@ int fg_mirror_force_mirror(fg_ctx* ctx, fg_energy* e) {
   int rc = ensure_ready(ctx);
   if (rc) return rc;
   if ((rc = force_now(ctx))) return rc;
-  if ((rc = pull_scalars(ctx))) return rc;
+  if ((rc = wait_scalars(ctx))) return rc;  // written by the graph's last tail
   if (e) energy_out(ctx->sc_host, e, true);
   return FG_OK;
 }
@@ -2188,7 +2211,7 @@ int fg_nose_poincare(fg_ctx* ctx, fg_energy* e) {
   if ((rc = run_graph(ctx, &ctx->g_np, 1))) return rc;
   ctx->np_ready = true;
   ctx->flo_valid = false;
-  if ((rc = pull_scalars(ctx))) return rc;
+  if ((rc = wait_scalars(ctx))) return rc;  // written by the graph's last tail
   if (e) energy_out(ctx->sc_host, e, false);
   return FG_OK;
 }

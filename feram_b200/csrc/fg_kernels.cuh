@@ -214,7 +214,9 @@ static_assert(sizeof(Phys) % 8 == 0, "Phys is copied as doubles");
 // rows needs 5 per column (14 columns: 140 instructions a warp, all in one
 // SM's shuffle unit).  The loads are batched by hand: left to the compiler
 // they went out one by one (28 us for 64^3's plane sums, 14 batched).  body
-// runs on the first LANES threads.
+// runs on the first LANES threads.  host (may be null): the host's copy of the
+// scalars, in pinned memory, for the calls that return a step's energies: 0.6
+// kB of posted writes instead of a copy of its own after the last kernel.
 // Step of 16^3, mixed: 22.5 -> 21.5 us with this and the nine plane sums that
 // cost 1.7 us before it.
 template <int N>
@@ -257,7 +259,8 @@ __device__ __forceinline__ double column_warp_sum(double s) {
 }
 template <int NA, int NB, int LANES = 1, class F>
 __device__ __forceinline__ void reduced_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ pa,
-                                             const double* __restrict__ pb, int nblk, int nblk_b, F&& body) {
+                                             const double* __restrict__ pb, int nblk, int nblk_b, F&& body,
+                                             DevScalars* host = nullptr) {
   constexpr int NQ = NA + NB;
   __shared__ Phys sph;
   __shared__ DevScalars ssc;
@@ -286,8 +289,11 @@ __device__ __forceinline__ void reduced_tail(const Phys* __restrict__ ph, DevSca
   __syncthreads();
   if (threadIdx.x < LANES) body(static_cast<const Phys*>(&sph), &ssc, tot);
   __syncthreads();
-  for (int i = threadIdx.x; i < NS; i += blockDim.x)
-    reinterpret_cast<double*>(sc)[i] = reinterpret_cast<const double*>(&ssc)[i];
+  for (int i = threadIdx.x; i < NS; i += blockDim.x) {
+    const double v = reinterpret_cast<const double*>(&ssc)[i];
+    reinterpret_cast<double*>(sc)[i] = v;
+    if (host) reinterpret_cast<double*>(host)[i] = v;
+  }
 }
 
 // Last-block-done: thread 0 of every block fences the block's partials and
@@ -1594,28 +1600,30 @@ __device__ __forceinline__ void np_close_body(const Phys* P, DevScalars* S, cons
 }
 
 __device__ __noinline__ void force_energies_tail(const Phys* __restrict__ ph, DevScalars* sc,
-                                                 const double* __restrict__ part_r, int nblk, bool np_close) {
+                                                 const double* __restrict__ part_r, int nblk, bool np_close,
+                                                 DevScalars* host = nullptr) {
   reduced_tail<NQ_R, 0>(ph, sc, part_r, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     force_energies_body(P, S, v);
     if (np_close) np_post_body(P, S, 1.0 / S->pend_s, log(S->pend_s));
-  });
+  }, host);
 }
 __device__ __noinline__ void np_close_tail(const Phys* __restrict__ ph, DevScalars* sc,
-                                           const double* __restrict__ part, int nblk, bool step_done) {
+                                           const double* __restrict__ part, int nblk, bool step_done,
+                                           DevScalars* host) {
   reduced_tail<3, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     np_close_body(P, S, v, 1.0 / S->s, log(S->s), step_done);
-  });
+  }, host);
 }
 // Both for k_assemble with the fused closing kick, in one tail.
 __device__ __noinline__ void np_step_tail(const Phys* __restrict__ ph, DevScalars* sc,
                                           const double* __restrict__ part_r, const double* __restrict__ part_ke,
-                                          int nblk) {
+                                          int nblk, DevScalars* host) {
   reduced_tail<NQ_R, 3>(ph, sc, part_r, part_ke, nblk, nblk, [&](const Phys* P, DevScalars* S, const double* v) {
     const double inv_s = 1.0 / S->pend_s, log_s = log(S->pend_s);
     force_energies_body(P, S, v);
     np_post_body(P, S, inv_s, log_s);
     np_close_body(P, S, v + NQ_R, inv_s, log_s, true);
-  });
+  }, host);
 }
 
 // Velocity scaling (velocity_scaling.F:74-83): kinetic energy of the kicked
@@ -2593,7 +2601,7 @@ __global__ void __launch_bounds__(256, 2)
                const T* __restrict__ site_E, int zl0, T* __restrict__ p, const double* __restrict__ layer_minv,
                const unsigned char* __restrict__ layer_sump, const T* __restrict__ site_minv,
                const unsigned char* __restrict__ site_sump, double* __restrict__ part_ke, T* __restrict__ Flo,
-               const AsmConst k, const RepArgs* __restrict__ grp = nullptr) {
+               const AsmConst k, const RepArgs* __restrict__ grp, DevScalars* host) {
   pdl_launch();  // one resident wave: nothing of this grid is left to schedule
   pdl_wait();
   if (grp) {
@@ -2769,10 +2777,10 @@ __global__ void __launch_bounds__(256, 2)
   }
   if constexpr (CLOSE) {
     block_partials2<NQ_R, 3>(acc, ke, part, part_ke, blockIdx.x);
-    if (is_last_block(done)) np_step_tail(ph, sc, part, part_ke, gridDim.x);
+    if (is_last_block(done)) np_step_tail(ph, sc, part, part_ke, gridDim.x, host);
   } else {
     block_partials<NQ_R>(acc, part, blockIdx.x);
-    if (tail == TAIL_ENERGIES && is_last_block(done)) force_energies_tail(ph, sc, part, gridDim.x, false);
+    if (tail == TAIL_ENERGIES && is_last_block(done)) force_energies_tail(ph, sc, part, gridDim.x, false, host);
   }
 }
 
@@ -2935,6 +2943,25 @@ __host__ __device__ inline void wave_field(int type, long long i_step, int n_the
   }
 }
 
+// fg_set_uniform_E and the thermostat of fg_set_state: the values travel as
+// arguments of the launch (a copy from pinned memory took 2 us longer, and
+// its source had to stay untouched until it had run).
+__global__ void k_set_field(DevScalars* sc, double e0, double e1, double e2) {
+  if (threadIdx.x == 0) {
+    sc->E[0] = e0;
+    sc->E[1] = e1;
+    sc->E[2] = e2;
+  }
+}
+__global__ void k_set_thermostat(DevScalars* sc, double s, double pi, double H0, double kick_coef) {
+  if (threadIdx.x == 0) {
+    sc->s = s;
+    sc->pi = pi;
+    sc->H0 = H0;
+    sc->kick_coef = kick_coef;
+  }
+}
+
 // Start of a step under the device-side field schedule: the step counter
 // advances and the uniform field becomes that step's wave value
 // (molecular-dynamics.F:66-76, before the step's force evaluation).
@@ -3014,7 +3041,8 @@ __global__ void __launch_bounds__(256) k_kick_close(T* __restrict__ p, const T* 
                                                     const Phys* __restrict__ ph, DevScalars* sc,
                                                     const double* __restrict__ part_r, int nblk_r,
                                                     const T* __restrict__ site_minv = nullptr,
-                                                    const unsigned char* __restrict__ site_sump = nullptr) {
+                                                    const unsigned char* __restrict__ site_sump = nullptr,
+                                                    DevScalars* host = nullptr) {
   pdl_launch();  // one resident wave: nothing of this grid is left to schedule
   pdl_wait();
   if (!PREP && blockIdx.x == 0) force_energies_tail(ph, sc, part_r, nblk_r, true);
@@ -3076,7 +3104,7 @@ __global__ void __launch_bounds__(256) k_kick_close(T* __restrict__ p, const T* 
     }
   }
   block_partials<3>(acc, part, blockIdx.x);
-  if (is_last_block(done)) np_close_tail(ph, sc, part, gridDim.x, !PREP);
+  if (is_last_block(done)) np_close_tail(ph, sc, part, gridDim.x, !PREP, host);
 }
 
 // u <- u + coef * p * m^-1 (nose-poincare.F:41-53, leapfrog.F:104-114)
