@@ -523,12 +523,30 @@ AsmConst asm_const(const fg_ctx* ctx) {
 }
 
 // flo: also store the FP32 residual of the force (mixed path)
+// Threads' worth of work: vectors of sites where the layers are multiples of
+// one, else (and with per-site arrays) sites.
+template <typename T>
+long long asm_work(const fg_ctx* ctx, bool sites) {
+  constexpr int NV = V16<T>::n;
+  return !sites && ctx->g.plane_r % NV == 0 ? ctx->g.nsite / NV : ctx->g.nsite;
+}
+// Blocks of k_assemble: those that have work, at most the plan's.  Every block
+// costs a ticket and a row of partials: 48^3 has work for 108 blocks (FP32),
+// and its step took 37.9 us with the 296 of the plan, 36.7 with 108.  Smaller
+// blocks on more SMs were slower (16^3 FP64, 64 threads: 22.3 against 21.0):
+// the last block's tail has fewer threads for its loads.
+template <typename T, bool CLOSE>
+int asm_grid(const fg_ctx* ctx) {
+  const bool sites = ctx->site_species || ctx->site_zstar || ctx->site_E ||
+                     (CLOSE && (ctx->site_minv || ctx->site_sump));
+  return std::min(CLOSE ? ctx->grid_asc : ctx->grid_as, div_up(asm_work<T>(ctx, sites), kThreadsElem));
+}
+
 template <typename T, bool CLOSE>
 void launch_assemble(fg_ctx* ctx, int tail, bool flo = false, DevScalars* host = nullptr) {
   const bool sites = ctx->site_species || ctx->site_zstar || ctx->site_E ||
                      (CLOSE && (ctx->site_minv || ctx->site_sump));
-  launch_dep(ctx, sites ? k_assemble<T, CLOSE, true> : k_assemble<T, CLOSE, false>,
-             CLOSE ? ctx->grid_asc : ctx->grid_as, kThreadsElem, 0, (const T*)ctx->rwork, (const T*)ctx->u, (T*)ctx->F, ctx->g, ctx->ph, ctx->sc, ctx->part_r, tail,
+  launch_dep(ctx, sites ? k_assemble<T, CLOSE, true> : k_assemble<T, CLOSE, false>, asm_grid<T, CLOSE>(ctx), kThreadsElem, 0, (const T*)ctx->rwork, (const T*)ctx->u, (T*)ctx->F, ctx->g, ctx->ph, ctx->sc, ctx->part_r, tail,
              ctx->done + 2, ctx->site_species, (const T*)ctx->site_zstar, (const T*)ctx->site_E,
              ctx->zsite ? zu_comp(ctx) : 0, (T*)ctx->p, ctx->layer_minv, ctx->layer_sump, (const T*)ctx->site_minv,
              ctx->site_sump, ctx->part_ke, (flo && sizeof(T) == 4) ? (T*)ctx->Flo : (T*)nullptr, asm_const(ctx),
@@ -646,7 +664,7 @@ template <typename T, bool PREP>
 int enqueue_kick_close(fg_ctx* ctx, DevScalars* host = nullptr) {
   launch_dep(ctx, k_kick_close<T, PREP>, ctx->grid_kc, kThreadsElem, 0,
       (T*)ctx->p, (const T*)ctx->F, ctx->g, ctx->layer_minv, ctx->layer_sump, ctx->part_ke, ctx->done, ctx->ph,
-      ctx->sc, ctx->part_r, ctx->grid_as, (const T*)ctx->site_minv, ctx->site_sump, host);
+      ctx->sc, ctx->part_r, asm_grid<T, false>(ctx), (const T*)ctx->site_minv, ctx->site_sump, host);
   CKL();
   return FG_OK;
 }
@@ -738,7 +756,7 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
   if (!rc) rc = launch_z_kspace<T>(c0, nullptr, nrep, grp);
   if (!rc) rc = launch_xy_inv<T>(c0, nullptr, nullptr, c0->ncx, true, nrep, grp);
   if (rc) return rc;
-  launch_dep(c0, k_assemble<T, true>, dim3(c0->grid_asc, nrep), kThreadsElem, 0, (const T*)nullptr,
+  launch_dep(c0, k_assemble<T, true>, dim3(asm_grid<T, true>(c0), nrep), kThreadsElem, 0, (const T*)nullptr,
              (const T*)nullptr, (T*)nullptr, g, (const Phys*)nullptr, (DevScalars*)nullptr, (double*)nullptr,
              (int)TAIL_NONE, (unsigned int*)nullptr, (const unsigned char*)nullptr, (const T*)nullptr,
              (const T*)nullptr, 0, (T*)nullptr, (const double*)nullptr, (const unsigned char*)nullptr,
