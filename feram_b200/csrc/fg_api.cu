@@ -216,7 +216,7 @@ struct fg_ctx {
   unsigned gen = 0;       // bumped when buffers that graphs hold are replaced
   bool broken = false;    // a reallocation failed half way: refuse further work
   bool store_acouK = false;
-  bool wave_dev = false;  // the step graphs start with k_wave_step (fg_set_wave)
+  bool wave_dev = false;  // the steps evaluate the field wave on the device (fg_set_wave)
   double n_sum_p = 0;
   int NXP = 0, NYP = 0;
   bool bulk_or_film_mirror() const { return P.bulk_or_film == FG_FILM || P.bulk_or_film == FG_EPIT; }
@@ -519,10 +519,16 @@ AsmConst asm_const(const fg_ctx* ctx) {
   k.hx = h.HC2[0][0]; k.hy = h.HC2[0][1]; k.h4 = h.HC2[3][3];
   k.Zs = h.Zstar;
   k.E_on = h.E_on;
+  k.gap_id = ctx->bulk_or_film_mirror() ? (int)ctx->P.gap_id : 0;
   return k;
 }
 
-// flo: also store the FP32 residual of the force (mixed path)
+// A film whose step mirrors inside its kernels (enqueue_np).
+bool film_fused(const fg_ctx* ctx) {
+  return ctx->bulk_or_film_mirror() && !ctx->site_species && !ctx->site_zstar && !ctx->site_E && !ctx->site_minv &&
+         !ctx->site_sump;
+}
+
 // Threads' worth of work: vectors of sites where the layers are multiples of
 // one, else (and with per-site arrays) sites.
 template <typename T>
@@ -539,14 +545,20 @@ template <typename T, bool CLOSE>
 int asm_grid(const fg_ctx* ctx) {
   const bool sites = ctx->site_species || ctx->site_zstar || ctx->site_E ||
                      (CLOSE && (ctx->site_minv || ctx->site_sump));
-  return std::min(CLOSE ? ctx->grid_asc : ctx->grid_as, div_up(asm_work<T>(ctx, sites), kThreadsElem));
+  long long work = asm_work<T>(ctx, sites);
+  if (CLOSE && film_fused(ctx)) work = work / ctx->g.Lz * film_layers(ctx->g.Lz, ctx->P.gap_id);
+  return std::min(CLOSE ? ctx->grid_asc : ctx->grid_as, div_up(work, kThreadsElem));
 }
 
+// flo: also store the FP32 residual of the force (mixed path)
 template <typename T, bool CLOSE>
 void launch_assemble(fg_ctx* ctx, int tail, bool flo = false, DevScalars* host = nullptr) {
   const bool sites = ctx->site_species || ctx->site_zstar || ctx->site_E ||
                      (CLOSE && (ctx->site_minv || ctx->site_sump));
-  launch_dep(ctx, sites ? k_assemble<T, CLOSE, true> : k_assemble<T, CLOSE, false>, asm_grid<T, CLOSE>(ctx), kThreadsElem, 0, (const T*)ctx->rwork, (const T*)ctx->u, (T*)ctx->F, ctx->g, ctx->ph, ctx->sc, ctx->part_r, tail,
+  auto kern = sites ? k_assemble<T, CLOSE, true> : k_assemble<T, CLOSE, false>;
+  if constexpr (CLOSE)
+    if (film_fused(ctx)) kern = k_assemble<T, true, false, true>;
+  launch_dep(ctx, kern, asm_grid<T, CLOSE>(ctx), kThreadsElem, 0, (const T*)ctx->rwork, (const T*)ctx->u, (T*)ctx->F, ctx->g, ctx->ph, ctx->sc, ctx->part_r, tail,
              ctx->done + 2, ctx->site_species, (const T*)ctx->site_zstar, (const T*)ctx->site_E,
              ctx->zsite ? zu_comp(ctx) : 0, (T*)ctx->p, ctx->layer_minv, ctx->layer_sump, (const T*)ctx->site_minv,
              ctx->site_sump, ctx->part_ke, (flo && sizeof(T) == 4) ? (T*)ctx->Flo : (T*)nullptr, asm_const(ctx),
@@ -566,7 +578,8 @@ int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false, DevScal
   const Geom& g = ctx->g;
   cudaStream_t st = ctx->stream;
   T* u = (T*)ctx->u;
-  if (ctx->P.bulk_or_film == FG_FILM || ctx->P.bulk_or_film == FG_EPIT) {
+  const bool mirror = ctx->bulk_or_film_mirror() && mode != FORCE_NP_CLOSE;  // else inside the step's kernels
+  if (mirror) {
     k_mirror<T><<<ctx->grid_elem, kThreadsElem, 0, st>>>(u, g, ctx->P.gap_id);
     CKL();
   }
@@ -580,7 +593,7 @@ int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false, DevScal
   if (mode == FORCE_NP_CLOSE) launch_assemble<T, true>(ctx, TAIL_NONE, false, host);
   else launch_assemble<T, false>(ctx, mode == FORCE_NP_POST ? TAIL_NONE : TAIL_ENERGIES, flo, host);
   CKL();
-  if (ctx->P.bulk_or_film == FG_FILM || ctx->P.bulk_or_film == FG_EPIT) {
+  if (mirror) {
     k_mirror<T><<<ctx->grid_elem, kThreadsElem, 0, st>>>((T*)ctx->F, g, ctx->P.gap_id);
     CKL();
     if (flo && sizeof(T) == 4) {
@@ -651,10 +664,12 @@ int enqueue_wave(fg_ctx* ctx) {
   return FG_OK;
 }
 
+// film: u is mirrored in the same pass; wave: the step's field is set in it
 template <typename T>
-int enqueue_kick_drift(fg_ctx* ctx) {
+int enqueue_kick_drift(fg_ctx* ctx, bool film = false, bool wave = false) {
   launch_dep(ctx, k_kick_drift<T>, ctx->grid_kd, kThreadsElem, 0, (T*)ctx->p, (T*)ctx->u, (const T*)ctx->F,
-             ctx->sc, ctx->g, ctx->layer_minv, (const T*)ctx->site_minv, (const RepArgs*)nullptr);
+             ctx->sc, ctx->g, ctx->layer_minv, (const T*)ctx->site_minv,
+             (const Phys*)(wave ? ctx->ph : nullptr), film ? (int)ctx->P.gap_id : -1, (const RepArgs*)nullptr);
   CKL();
   return FG_OK;
 }
@@ -684,15 +699,16 @@ int enqueue_kick_close(fg_ctx* ctx, DevScalars* host = nullptr) {
 // step's closing kick.
 template <typename T>
 int enqueue_np(fg_ctx* ctx, bool follows_step = false, DevScalars* host = nullptr) {
-  const bool pdl = !ctx->bulk_or_film_mirror();
-  int rc = enqueue_wave(ctx);
-  if (rc) return rc;
-  ctx->pdl = pdl && follows_step && !ctx->wave_dev;
-  rc = enqueue_kick_drift<T>(ctx);
+  // The closing kick runs inside k_assemble, which also mirrors a film's
+  // force (and k_kick_drift its u).  Films with per-site arrays, whose sites'
+  // masses and species need not be mirror images, mirror by k_mirror, so that
+  // their closing kick is a kernel of its own.
+  const bool mirror = ctx->bulk_or_film_mirror(), film = mirror && film_fused(ctx);
+  const bool fused = !mirror || film;
+  const bool pdl = fused;
+  ctx->pdl = pdl && follows_step;
+  int rc = enqueue_kick_drift<T>(ctx, film, ctx->wave_dev);
   ctx->pdl = pdl;
-  // bulk: the closing kick runs inside k_assemble; films mirror the force
-  // first, so the kick is a kernel of its own
-  const bool fused = !ctx->bulk_or_film_mirror();
   if (!rc) rc = enqueue_force<T>(ctx, fused ? FORCE_NP_CLOSE : FORCE_NP_POST, false, fused ? host : nullptr);
   if (!rc && !fused) rc = enqueue_kick_close<T, false>(ctx, host);
   ctx->pdl = false;
@@ -748,7 +764,8 @@ int enqueue_np_group(fg_ctx* c0, const RepArgs* grp, int nrep) {
   const Geom& g = c0->g;
   c0->pdl = false;
   launch_dep(c0, k_kick_drift<T>, dim3(c0->grid_kd, nrep), kThreadsElem, 0, (T*)nullptr, (T*)nullptr,
-             (const T*)nullptr, (const DevScalars*)nullptr, g, (const double*)nullptr, (const T*)nullptr, grp);
+             (const T*)nullptr, (DevScalars*)nullptr, g, (const double*)nullptr, (const T*)nullptr, (const Phys*)nullptr,
+             -1, grp);
   CKL();
   c0->pdl = true;
   int rc = launch_xy_fwd<T, SRC_U9>(c0, nullptr, nullptr, c0->ncx, (const cplx<T>*)c0->twx, (const cplx<T>*)c0->twm,

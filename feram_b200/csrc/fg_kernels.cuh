@@ -2497,7 +2497,7 @@ struct AsmConst {
   double hx, hy, h4;                   // homogeneous_coupling_2: B1xx/2, B1yy/2, B4yz
   double Zs;
   int E_on;
-  int pad;
+  int gap_id;                          // of a film (k_assemble's FILM instance)
 };
 // Per-step values of the site force, read from DevScalars: strain . B2 and
 // the uniform field.
@@ -2544,6 +2544,16 @@ __device__ __forceinline__ void assemble_site(const Poly& pl, const AsmConst& k,
   o1 = f1 + 2 * w1 * uy + w3 * uz + w5 * ux;
   o2 = f2 + 2 * w2 * uz + w3 * uy + w4 * ux;
 }
+
+// Film mirror (mirror.F:9-36): layers z and partner(z) hold (f_x, f_y, f_z) and
+// (-f_x, -f_y, f_z); the lower one is the source.  z itself: a layer without
+// a partner.
+__device__ __forceinline__ int film_partner(int z, int Lz, int gap_id) {
+  if (gap_id == 0) return Lz - 1 - z;
+  return z > 0 ? Lz - z : 0;
+}
+// Layers that are nobody's image; they are the first ones.
+__host__ __device__ __forceinline__ int film_layers(int Lz, int gap_id) { return gap_id == 0 ? (Lz + 1) / 2 : Lz / 2 + 1; }
 
 // The force of one site in the field type T.  The mixed path (T = float)
 // rounds the FP64 sum once; with lo != null it also stores the rounding
@@ -2593,7 +2603,14 @@ __device__ __forceinline__ void close_site(T* __restrict__ p, long long ns, long
 // (np_close_tail: KE, H_NP and (38) of the next step).
 // Flo (mixed path, may be null): the FP32 residual of each force component,
 // F + Flo = the FP64 site sum.
-template <typename T, bool CLOSE = false, bool SITES = false>
+// FILM (with CLOSE, without per-site arrays): only the source layers' forces
+// are computed; each is written to its partner too, with the mirror's signs,
+// and both sites' momenta are kicked and counted.  The partner's u is the
+// mirrored one, so its on-site energy is the source's.  Half of the field
+// sums and of the site polynomials, and no k_mirror between this kernel and a
+// closing kick of its own: film step 64x64x32, mixed, 53 -> 44 us with the
+// mirrored drift (k_kick_drift).
+template <typename T, bool CLOSE = false, bool SITES = false, bool FILM = false>
 __global__ void __launch_bounds__(256, 2)
     k_assemble(const T* __restrict__ rw, const T* __restrict__ u, T* __restrict__ F, Geom g,
                const Phys* __restrict__ ph, DevScalars* sc, double* __restrict__ part, int tail, unsigned int* done,
@@ -2639,6 +2656,8 @@ __global__ void __launch_bounds__(256, 2)
   if (threadIdx.x == 8) dy.E2 = sc->E[2];
   __syncthreads();
   double acc[NQ_R] = {0.0, 0.0};
+  // FILM: sources and layers without a partner come first (film_partner)
+  const long long nown = FILM ? (long long)film_layers(g.Lz, k.gap_id) * g.plane_r : ns;
   constexpr int NV = V16<T>::n;
   using AV = V16<T>;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -2698,7 +2717,31 @@ __global__ void __launch_bounds__(256, 2)
       }
     }
   } else if (g.plane_r % NV == 0) {
-    for (long long iv = (long long)blockIdx.x * blockDim.x + threadIdx.x; iv < ns / NV; iv += stride) {
+    // closing kick of NV sites of layer z and their masked sums
+    auto close = [&](long long i, int z, const AV& o0, const AV& o1, const AV& o2) {
+      AV q[3] = {ldv(p + i), ldv(p + ns + i), ldv(p + 2 * ns + i)};
+      T pp = 0, pf = 0, ff = 0;
+#pragma unroll
+      for (int l = 0; l < NV; ++l) {
+        const T f3[3] = {o0.v[l], o1.v[l], o2.v[l]};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          q[a].v[l] = q[a].v[l] - cf * f3[a];
+          pp += q[a].v[l] * q[a].v[l];
+          pf += q[a].v[l] * f3[a];
+          ff += f3[a] * f3[a];
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) stv(p + a * ns + i, q[a]);
+      if (layer_sump[z]) {
+        const double mi = layer_minv[z];
+        ke[0] += (double)pp * mi;
+        ke[1] += (double)pf * mi;
+        ke[2] += (double)ff * mi;
+      }
+    };
+    for (long long iv = (long long)blockIdx.x * blockDim.x + threadIdx.x; iv < nown / NV; iv += stride) {
       const long long i = iv * NV;
       const AV ux = ldv(u + i), uy = ldv(u + ns + i), uz = ldv(u + 2 * ns + i);
       // rw is consumed here: evict_first keeps u, p and F in L2
@@ -2708,11 +2751,13 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
       for (int q = 0; q < 6; ++q) e[q] = ldv_first(rw + (3 + q) * ns + i, pol_rw);
       AV o0, o1, o2, l0, l1, l2;
+      double as[NQ_R] = {0.0, 0.0};
 #pragma unroll
       for (int l = 0; l < NV; ++l) {
         const double eta[6] = {e[0].v[l], e[1].v[l], e[2].v[l], e[3].v[l], e[4].v[l], e[5].v[l]};
         double d0, d1, d2;
-        assemble_site(k.pl, k, k.Zs, dy, ux.v[l], uy.v[l], uz.v[l], a0.v[l], a1.v[l], a2.v[l], eta, d0, d1, d2, acc);
+        assemble_site(k.pl, k, k.Zs, dy, ux.v[l], uy.v[l], uz.v[l], a0.v[l], a1.v[l], a2.v[l], eta, d0, d1, d2,
+                      FILM ? as : acc);
         o0.v[l] = force_hi<T>(d0);
         o1.v[l] = force_hi<T>(d1);
         o2.v[l] = force_hi<T>(d2);
@@ -2730,36 +2775,38 @@ __global__ void __launch_bounds__(256, 2)
       }
       if constexpr (CLOSE) {
         const int z = (int)(i / g.plane_r);
-        AV q[3] = {ldv(p + i), ldv(p + ns + i), ldv(p + 2 * ns + i)};
-        T pp = 0, pf = 0, ff = 0;
+        close(i, z, o0, o1, o2);
+        if constexpr (FILM) {
+          const int zd = film_partner(z, g.Lz, k.gap_id);
+          acc[0] += as[0];
+          acc[1] += as[1];
+          if (zd != z) {
+            const long long d = i + (long long)(zd - z) * g.plane_r;
+            AV m0, m1;
 #pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const T f3[3] = {o0.v[l], o1.v[l], o2.v[l]};
-#pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            q[a].v[l] = q[a].v[l] - cf * f3[a];
-            pp += q[a].v[l] * q[a].v[l];
-            pf += q[a].v[l] * f3[a];
-            ff += f3[a] * f3[a];
+            for (int l = 0; l < NV; ++l) {
+              m0.v[l] = -o0.v[l];
+              m1.v[l] = -o1.v[l];
+              if (k.E_on)
+                acc[1] += k.Zs * ((double)uz.v[l] * dy.E2 - ((double)ux.v[l] * dy.E0 + (double)uy.v[l] * dy.E1));
+            }
+            acc[0] += as[0];
+            stv(F + d, m0);
+            stv(F + ns + d, m1);
+            stv(F + 2 * ns + d, o2);
+            close(d, zd, m0, m1, o2);
           }
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) stv(p + a * ns + i, q[a]);
-        if (layer_sump[z]) {
-          const double mi = layer_minv[z];
-          ke[0] += (double)pp * mi;
-          ke[1] += (double)pf * mi;
-          ke[2] += (double)ff * mi;
         }
       }
     }
   } else {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nown; i += stride) {
       double eta[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) eta[q] = (double)rw[(3 + q) * ns + i];
-      double o0, o1, o2;
-      assemble_site(k.pl, k, k.Zs, dy, u[i], u[ns + i], u[2 * ns + i], rw[i], rw[ns + i], rw[2 * ns + i], eta, o0, o1, o2, acc);
+      double o0, o1, o2, as[NQ_R] = {0.0, 0.0};
+      const double ux = u[i], uy = u[ns + i], uz = u[2 * ns + i];
+      assemble_site(k.pl, k, k.Zs, dy, ux, uy, uz, rw[i], rw[ns + i], rw[2 * ns + i], eta, o0, o1, o2, FILM ? as : acc);
       const T h0 = force_hi<T>(o0), h1 = force_hi<T>(o1), h2 = force_hi<T>(o2);
       F[i] = h0;
       F[ns + i] = h1;
@@ -2772,6 +2819,20 @@ __global__ void __launch_bounds__(256, 2)
       if constexpr (CLOSE) {
         const int z = (int)(i / g.plane_r);
         close_site(p, ns, i, cf, h0, h1, h2, layer_sump[z] != 0, layer_minv[z], ke);
+        if constexpr (FILM) {
+          const int zd = film_partner(z, g.Lz, k.gap_id);
+          acc[0] += as[0];
+          acc[1] += as[1];
+          if (zd != z) {
+            const long long d = i + (long long)(zd - z) * g.plane_r;
+            acc[0] += as[0];
+            if (k.E_on) acc[1] += k.Zs * (uz * dy.E2 - (ux * dy.E0 + uy * dy.E1));
+            F[d] = -h0;
+            F[ns + d] = -h1;
+            F[2 * ns + d] = h2;
+            close_site(p, ns, d, cf, -h0, -h1, h2, layer_sump[zd] != 0, layer_minv[zd], ke);
+          }
+        }
       }
     }
   }
@@ -2965,21 +3026,24 @@ __global__ void k_set_thermostat(DevScalars* sc, double s, double pi, double H0,
 // Start of a step under the device-side field schedule: the step counter
 // advances and the uniform field becomes that step's wave value
 // (molecular-dynamics.F:66-76, before the step's force evaluation).
-__global__ void k_wave_step(const Phys* __restrict__ ph, DevScalars* sc) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+__device__ inline void wave_step(const Phys* __restrict__ ph, DevScalars* sc) {
   const long long i = sc->i_step + 1;
   sc->i_step = i;
   double E[3];
   wave_field(ph->wave_type, i, ph->wave_n_thermalize, ph->wave_period, ph->wave_amp, E);
   for (int k = 0; k < 3; ++k) sc->E[k] = E[k];
 }
+// in front of the steps whose first kernel is not k_kick_drift
+__global__ void k_wave_step(const Phys* __restrict__ ph, DevScalars* sc) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) wave_step(ph, sc);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __restrict__ u, const T* __restrict__ F,
-                                                    const DevScalars* __restrict__ sc, Geom g,
+                                                    DevScalars* sc, Geom g,
                                                     const double* __restrict__ layer_minv,
-                                                    const T* __restrict__ site_minv = nullptr,
-                                                    const RepArgs* __restrict__ grp = nullptr) {
+                                                    const T* __restrict__ site_minv, const Phys* __restrict__ wave,
+                                                    int gap_id, const RepArgs* __restrict__ grp) {
   pdl_launch();  // one resident wave: nothing of this grid is left to schedule
   pdl_wait();
   if (grp) {
@@ -2990,6 +3054,10 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
     sc = a.sc;
     layer_minv = a.layer_minv;
   }
+  if (wave != nullptr && blockIdx.x == 0 && threadIdx.x == 0) wave_step(wave, sc);
+  // Film (gap_id >= 0): every layer's momenta are kicked, the source layers'
+  // dipoles drift and are written to their partners' layer as well
+  auto partner = [&](int z) { return gap_id < 0 ? z : film_partner(z, g.Lz, gap_id); };
   const long long ns = g.nsite;
   const StepCoef<T> ck(sc->kick_coef);
   const double cd = sc->pend_drift;
@@ -2999,28 +3067,46 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
   if (g.plane_r % NV == 0 && site_minv == nullptr) {
     for (long long iv = (long long)blockIdx.x * blockDim.x + threadIdx.x; iv < ns / NV; iv += stride) {
       const long long i = iv * NV;
-      const StepCoef<T> f(cd * layer_minv[(int)(i / g.plane_r)]);
+      const int z = (int)(i / g.plane_r), zd = partner(z);
+      const StepCoef<T> f(cd * layer_minv[z]);
+      V16<T> x[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        V16<T> q = ldv(p + a * ns + i), x = ldv(u + a * ns + i);
+        V16<T> q = ldv(p + a * ns + i);
+        x[a] = zd >= z ? ldv(u + a * ns + i) : q;  // not an image's u: its source is writing it
         const V16<T> y = ldv(F + a * ns + i);
 #pragma unroll
         for (int l = 0; l < NV; ++l) {
           q.v[l] = q.v[l] - ck * y.v[l];
-          x.v[l] = x.v[l] + f * q.v[l];
+          x[a].v[l] = x[a].v[l] + f * q.v[l];
         }
         stv(p + a * ns + i, q);
-        stv(u + a * ns + i, x);
+        if (zd >= z) stv(u + a * ns + i, x[a]);
+      }
+      if (zd > z) {
+        const long long d = i + (long long)(zd - z) * g.plane_r;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+#pragma unroll
+          for (int l = 0; l < NV; ++l) x[a].v[l] = a < 2 ? -x[a].v[l] : x[a].v[l];
+          stv(u + a * ns + d, x[a]);
+        }
       }
     }
   } else {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
-      const StepCoef<T> f(cd * (site_minv ? (double)site_minv[i] : layer_minv[(int)(i / g.plane_r)]));
+      const int z = (int)(i / g.plane_r), zd = partner(z);
+      const StepCoef<T> f(cd * (site_minv ? (double)site_minv[i] : layer_minv[z]));
+      const long long d = i + (long long)(zd - z) * g.plane_r;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const T q = p[a * ns + i] - ck * F[a * ns + i];
         p[a * ns + i] = q;
-        u[a * ns + i] = u[a * ns + i] + f * q;
+        if (zd >= z) {
+          const T x = u[a * ns + i] + f * q;
+          u[a * ns + i] = x;
+          if (zd > z) u[a * ns + d] = a < 2 ? -x : x;
+        }
       }
     }
   }
