@@ -605,39 +605,44 @@ int enqueue_force(fg_ctx* ctx, int mode = FORCE_PLAIN, bool flo = false, DevScal
 }
 
 template <typename T>
-int enqueue_kick(fg_ctx* ctx, const double* coef, int tail = TAIL_NONE, int zero_unmasked = 0) {
-  k_kick<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>(
+SecondField<T> acou_field(const fg_ctx* ctx) {
+  const long long off = 3 * ctx->g.nsite;
+  return {(T*)ctx->u + off, (T*)ctx->p + off, (const T*)ctx->rwork + 3 * off, ctx->layer_macou, ctx->layer_all,
+          (const T*)ctx->site_macou};
+}
+// Blocks of k_kick and k_drift: those that have work (asm_grid's reason).
+template <typename T>
+dim3 kick_grid(const fg_ctx* ctx, bool both) {
+  const bool sites = ctx->site_minv || ctx->site_sump || ctx->site_macou;
+  return dim3(std::min(ctx->grid_elem, div_up(asm_work<T>(ctx, sites), kThreadsElem)), both ? 2 : 1);
+}
+
+// both: the acoustic field's kick and kinetic sum in the same launch
+template <typename T>
+int enqueue_kick(fg_ctx* ctx, const double* coef, int tail = TAIL_NONE, int zero_unmasked = 0, bool both = false) {
+  k_kick<T><<<kick_grid<T>(ctx, both), kThreadsElem, 0, ctx->stream>>>(
       (T*)ctx->p, (const T*)ctx->F, coef, ctx->g, ctx->layer_minv, ctx->layer_sump, ctx->part_ke, tail, ctx->done,
-      ctx->ph, ctx->sc, zero_unmasked, (const T*)ctx->site_minv, ctx->site_sump);
+      ctx->ph, ctx->sc, zero_unmasked, (const T*)ctx->site_minv, ctx->site_sump, acou_field<T>(ctx));
   CKL();
   return FG_OK;
 }
 
+// The drift of u and, where it is dynamic, of the acoustic field.
 template <typename T>
 int enqueue_drift(fg_ctx* ctx, const double* coef) {
-  k_drift<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>((T*)ctx->u, (const T*)ctx->p, coef, ctx->g,
-                                                                ctx->layer_minv, (const T*)ctx->site_minv);
+  k_drift<T><<<kick_grid<T>(ctx, ctx->acou), kThreadsElem, 0, ctx->stream>>>(
+      (T*)ctx->u, (const T*)ctx->p, coef, ctx->g, ctx->layer_minv, (const T*)ctx->site_minv, acou_field<T>(ctx));
   CKL();
   return FG_OK;
 }
 
-// Acoustic momenta and displacements (acouP, acouR: components 3..5 of p and
-// u): kick by dVdacR (rwork components 9..11), no sum_p mask, uniform mass.
+// The acoustic field alone.
 template <typename T>
 int enqueue_kick_acou(fg_ctx* ctx, const double* coef, int tail) {
-  const long long ns = ctx->g.nsite;
-  k_kick<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>(
-      (T*)ctx->p + 3 * ns, (const T*)ctx->rwork + 9 * ns, coef, ctx->g, ctx->layer_macou, ctx->layer_all,
-      ctx->part_ke, tail, ctx->done, ctx->ph, ctx->sc, 0, (const T*)ctx->site_macou, nullptr);
-  CKL();
-  return FG_OK;
-}
-
-template <typename T>
-int enqueue_drift_acou(fg_ctx* ctx, const double* coef) {
-  const long long ns = ctx->g.nsite;
-  k_drift<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>((T*)ctx->u + 3 * ns, (const T*)ctx->p + 3 * ns, coef,
-                                                                ctx->g, ctx->layer_macou, (const T*)ctx->site_macou);
+  const SecondField<T> a = acou_field<T>(ctx);
+  k_kick<T><<<kick_grid<T>(ctx, false), kThreadsElem, 0, ctx->stream>>>(a.p, a.F, coef, ctx->g, a.layer_minv, a.layer_mask,
+                                                                         ctx->part_ke, tail, ctx->done, ctx->ph, ctx->sc,
+                                                                         0, a.site_minv, nullptr, a);
   CKL();
   return FG_OK;
 }
@@ -725,10 +730,8 @@ int enqueue_lf(fg_ctx* ctx) {
   if ((rc = enqueue_wave(ctx))) return rc;
   if ((rc = enqueue_pump<T>(ctx))) return rc;
   if ((rc = enqueue_drift<T>(ctx, &ctx->sc->lf_dt))) return rc;
-  if (ctx->acou && (rc = enqueue_drift_acou<T>(ctx, &ctx->sc->lf_dt))) return rc;
   if ((rc = enqueue_force<T>(ctx))) return rc;
-  if (ctx->acou && (rc = enqueue_kick_acou<T>(ctx, &ctx->sc->lf_dt, TAIL_ACOU))) return rc;
-  if ((rc = enqueue_kick<T>(ctx, &ctx->sc->lf_dt, TAIL_LF_FINAL))) return rc;
+  if ((rc = enqueue_kick<T>(ctx, &ctx->sc->lf_dt, TAIL_LF_FINAL, 0, ctx->acou))) return rc;
   return FG_OK;
 }
 
@@ -740,7 +743,6 @@ int enqueue_vs(fg_ctx* ctx) {
   int rc;
   if ((rc = enqueue_wave(ctx))) return rc;
   if ((rc = enqueue_drift<T>(ctx, &ctx->sc->lf_dt))) return rc;
-  if (ctx->acou && (rc = enqueue_drift_acou<T>(ctx, &ctx->sc->lf_dt))) return rc;
   if ((rc = enqueue_force<T>(ctx))) return rc;
   if ((rc = enqueue_kick<T>(ctx, &ctx->sc->lf_dt, TAIL_VS, 1))) return rc;
   k_scale<T><<<ctx->grid_elem, kThreadsElem, 0, ctx->stream>>>((T*)ctx->p, &ctx->sc->vs_scale, 3 * ctx->g.nsite);
@@ -2258,11 +2260,8 @@ int fg_leapfrog(fg_ctx* ctx, fg_energy* e, int i_step) {
     const bool f32 = ctx->prec == FG_PREC_MIXED;
     if ((rc = f32 ? enqueue_pump<float>(ctx) : enqueue_pump<double>(ctx))) return rc;
     if ((rc = force_now(ctx))) return rc;
-    if (ctx->acou && (rc = f32 ? enqueue_kick_acou<float>(ctx, &ctx->sc->lf_dt_2, TAIL_ACOU)
-                               : enqueue_kick_acou<double>(ctx, &ctx->sc->lf_dt_2, TAIL_ACOU)))
-      return rc;
-    if ((rc = f32 ? enqueue_kick<float>(ctx, &ctx->sc->lf_dt_2, TAIL_LF_FINAL)
-                  : enqueue_kick<double>(ctx, &ctx->sc->lf_dt_2, TAIL_LF_FINAL)))
+    if ((rc = f32 ? enqueue_kick<float>(ctx, &ctx->sc->lf_dt_2, TAIL_LF_FINAL, 0, ctx->acou)
+                  : enqueue_kick<double>(ctx, &ctx->sc->lf_dt_2, TAIL_LF_FINAL, 0, ctx->acou)))
       return rc;
   } else {
     if ((rc = run_graph(ctx, &ctx->g_lf, 2))) return rc;

@@ -303,19 +303,21 @@ __device__ __forceinline__ void reduced_tail(const Phys* __restrict__ ph, DevSca
 // fences, after the barrier that puts the partials' stores by the block's
 // first warp before it: the tails read nothing but those partials (and values
 // whose writers fence themselves).
-__device__ __forceinline__ bool is_last_block(unsigned int* counter) {
+__device__ __forceinline__ bool is_last_block(unsigned int* counter, unsigned nblocks) {
   __shared__ bool last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     const unsigned t = atomicAdd(counter, 1u);
-    last = (t == gridDim.x - 1);
+    last = (t == nblocks - 1);
     if (last) *counter = 0u;
   }
   __syncthreads();
   if (last) __threadfence();
   return last;
 }
+
+__device__ __forceinline__ bool is_last_block(unsigned int* counter) { return is_last_block(counter, gridDim.x); }
 
 // ------------------------------------------------------- analytic short range
 // S(k) of the 27-point stencil of dipole-dipole-short-range.F:35-83 (2 kappa2
@@ -1412,7 +1414,7 @@ __host__ __device__ __forceinline__ long long tab_index(long long pos, int q) {
 // ------------------------------------------------------------ scalar kernels
 // Grid-wide scalar steps; each runs either as a single-block kernel or in the
 // last block of the kernel whose partial sums it reduces (tail).
-enum { TAIL_NONE = 0, TAIL_ENERGIES = 1, TAIL_LF_FINAL = 3, TAIL_VS = 4, TAIL_ACOU = 5, TAIL_VS_ACOU = 6 };
+enum { TAIL_NONE = 0, TAIL_ENERGIES = 1, TAIL_LF_FINAL = 3, TAIL_VS = 4, TAIL_VS_ACOU = 6 };
 
 __device__ __forceinline__ double sum_potential(const double* e) {
   return e[E_SHORT] + e[E_LONG] + e[E_DIPE] + e[E_UNH] + e[E_HS] + e[E_HC] + e[E_IS] + e[E_IC] + e[E_IM];
@@ -1641,27 +1643,31 @@ __device__ void vs_tail(const Phys* __restrict__ ph, DevScalars* sc, const doubl
 }
 
 // Acoustic kinetic energy sum acouP^2 / m / 2 (kinetic_energy_acou.F:15-27);
-// with vs also the rescale factor (velocity_scaling.F:86-98) and the total.
-__device__ void acou_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk,
-                          bool vs) {
+// the rescale factor (velocity_scaling.F:86-98) and the total.
+__device__ void acou_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk) {
   reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
     S->e[E_ACOU] = v[0] / 2;
-    if (vs) {
-      S->vs_scale_acou = sqrt(P->target_ke / S->e[E_ACOU]);
-      if (!isfinite(S->vs_scale_acou)) S->status = 3;
-      S->e[E_TOT] = S->e[E_DIPO] / (S->s * S->s) + S->e[E_ACOU] + sum_potential(S->e);
-    }
+    S->vs_scale_acou = sqrt(P->target_ke / S->e[E_ACOU]);
+    if (!isfinite(S->vs_scale_acou)) S->status = 3;
+    S->e[E_TOT] = S->e[E_DIPO] / (S->s * S->s) + S->e[E_ACOU] + sum_potential(S->e);
   });
 }
 
-// Leapfrog closing reduction (leapfrog.F:151) and total.
-__device__ void lf_final_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part, int nblk) {
-  reduced_tail<1, 0>(ph, sc, part, nullptr, nblk, 0, [&](const Phys* P, DevScalars* S, const double* v) {
-    S->ke_sum = v[0];
-    S->e[E_DIPO] = ke_from(P, v[0]);
-    S->e[E_TOT] = S->e[E_DIPO] / (S->s * S->s) + S->e[E_ACOU] + sum_potential(S->e);
-    check_finite(S, S->e, E_COUNT);
-  });
+// Leapfrog closing reduction (leapfrog.F:151) and total; part_acou: the
+// acoustic field's sums as well (null without one).
+__device__ __forceinline__ void lf_final_body(const Phys* P, DevScalars* S, double sum) {
+  S->ke_sum = sum;
+  S->e[E_DIPO] = ke_from(P, sum);
+  S->e[E_TOT] = S->e[E_DIPO] / (S->s * S->s) + S->e[E_ACOU] + sum_potential(S->e);
+  check_finite(S, S->e, E_COUNT);
+}
+__device__ void lf_final_tail(const Phys* __restrict__ ph, DevScalars* sc, const double* __restrict__ part,
+                              const double* __restrict__ part_acou, int nblk) {
+  reduced_tail<1, 1>(ph, sc, part, part_acou, nblk, part_acou ? nblk : 0,
+                     [&](const Phys* P, DevScalars* S, const double* v) {
+                       if (part_acou) S->e[E_ACOU] = v[1] / 2;
+                       lf_final_body(P, S, v[0]);
+                     });
 }
 
 // Wavevectors, trig tables and slot maps shared by the k-space kernels.
@@ -2846,6 +2852,19 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // --------------------------------------------------------------- integrators
+// The acoustic field's arrays, for the launches that treat it beside the
+// dipoles' as a second row of blocks: one launch and one tail instead of two,
+// and twice the blocks in flight (48^3 FP64 has work for 216 of the 1184 that
+// fit).  Leapfrog step of 48^3 FP64: 55.7 -> 49.2 us.
+template <typename T>
+struct SecondField {
+  T *u, *p;
+  const T* F;
+  const double* layer_minv;
+  const unsigned char* layer_mask;
+  const T* site_minv;
+};
+
 // p <- p - coef * F on every site (leapfrog.F:134-138) and the masked sum
 // p^2 m^-1 of kinetic_energy_dipo.F:92-105.  Per-layer masses and sum_p
 // masks (film halves, dead layers).
@@ -2854,11 +2873,21 @@ __global__ void __launch_bounds__(256) k_kick(T* __restrict__ p, const T* __rest
                                               const double* __restrict__ layer_minv,
                                               const unsigned char* __restrict__ layer_sump, double* __restrict__ part,
                                               int tail, unsigned int* done, const Phys* __restrict__ ph,
-                                              DevScalars* sc, int zero_unmasked, const T* __restrict__ site_minv = nullptr,
-                                              const unsigned char* __restrict__ site_sump = nullptr) {
+                                              DevScalars* sc, int zero_unmasked, const T* __restrict__ site_minv,
+                                              const unsigned char* __restrict__ site_sump, const SecondField<T> acou) {
   // zero_unmasked: p = 0 outside sum_p (velocity_scaling.F:61-71).
   // site_minv / site_sump: per-site masses and masks (.relaxor, .defects)
   // instead of the per-layer tables; they take the scalar loop.
+  const double* const part0 = part;
+  if (blockIdx.y == 1) {
+    p = acou.p;
+    F = acou.F;
+    layer_minv = acou.layer_minv;
+    layer_sump = acou.layer_mask;
+    site_minv = acou.site_minv;
+    site_sump = nullptr;
+    part += gridDim.x;
+  }
   const long long ns = g.nsite;
   const StepCoef<T> c(*coef);
   double acc[1] = {0.0};
@@ -2903,10 +2932,10 @@ __global__ void __launch_bounds__(256) k_kick(T* __restrict__ p, const T* __rest
     }
   }
   block_partials<1>(acc, part, blockIdx.x);
-  if (tail != TAIL_NONE && is_last_block(done)) {
-    if (tail == TAIL_LF_FINAL) lf_final_tail(ph, sc, part, gridDim.x);
-    else if (tail == TAIL_VS) vs_tail(ph, sc, part, gridDim.x);
-    else if (tail == TAIL_ACOU || tail == TAIL_VS_ACOU) acou_tail(ph, sc, part, gridDim.x, tail == TAIL_VS_ACOU);
+  if (tail != TAIL_NONE && is_last_block(done, gridDim.x * gridDim.y)) {
+    if (tail == TAIL_LF_FINAL) lf_final_tail(ph, sc, part0, gridDim.y == 2 ? part0 + gridDim.x : nullptr, gridDim.x);
+    else if (tail == TAIL_VS) vs_tail(ph, sc, part0, gridDim.x);
+    else if (tail == TAIL_VS_ACOU) acou_tail(ph, sc, part0, gridDim.x);
   }
 }
 
@@ -3197,7 +3226,13 @@ __global__ void __launch_bounds__(256) k_kick_close(T* __restrict__ p, const T* 
 template <typename T>
 __global__ void __launch_bounds__(256) k_drift(T* __restrict__ u, const T* __restrict__ p, const double* coef, Geom g,
                                                const double* __restrict__ layer_minv,
-                                               const T* __restrict__ site_minv = nullptr) {
+                                               const T* __restrict__ site_minv, const SecondField<T> acou) {
+  if (blockIdx.y == 1) {
+    u = acou.u;
+    p = acou.p;
+    layer_minv = acou.layer_minv;
+    site_minv = acou.site_minv;
+  }
   const long long ns = g.nsite;
   const double c = *coef;
   constexpr int NV = V16<T>::n;
