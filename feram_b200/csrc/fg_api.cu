@@ -689,14 +689,16 @@ int enqueue_kick_close(fg_ctx* ctx, DevScalars* host = nullptr) {
   return FG_OK;
 }
 
-// nose_poincare (nose-poincare.F:24-75) as one graph of six kernels:
+// nose_poincare (nose-poincare.F:24-75) as one graph of five kernels:
 //   k_kick_drift       (35a) + (35c) with the coefficients prepared by the
-//                      previous closing tail ((38) solved there)
+//                      previous closing tail ((38) solved there); a film's u
+//                      mirrored, the field wave's value set
 //   force              xy_fwd, z_kspace, xy_inv (+ homogeneous strain),
-//                      k_assemble (partials only)
-//   k_kick_close       block 0: energies, commit of the half step, (35e);
-//                      all: (35f) and the three kinetic sums; last block:
+//   k_assemble         force, a film's mirrored, (35f) and the kinetic sums;
+//                      last block: energies, commit of the half step, (35e),
 //                      KE, H_NP of this step and the scalars of the next.
+// Films with per-site arrays: k_mirror before and after the force, and the
+// closing kick as a kernel of its own (k_kick_close).
 //
 // Each kernel after the first starts while its predecessor drains
 // (programmatic dependent launch); follows_step: the step continues a graph

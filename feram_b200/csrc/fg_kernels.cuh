@@ -10,7 +10,8 @@
 // One force evaluation (mirror_force_mirror.F:6-89) is four passes:
 //   k_xy_fwd     per (z-plane, component): r2c along x + DIF along y of
 //                u and u (x) u (dipoFFT.F:19-44) -> spec
-//   k_z_kspace   per (kx tile, ky): DIF along z, every k-space operation
+//   k_z_lane (k_z_kspace for the lengths and options it does not take)
+//                per (kx tile, ky): DIF along z, every k-space operation
 //                (dipole-dipole multiply, inhomogeneous strain solve,
 //                energies), DIT along z
 //   k_xy_inv     per (z-plane, component): DIT along y + c2r along x
