@@ -482,12 +482,13 @@ int plan_z(fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_
   if (with_z_lane<T>(g.Lz, zt.CW, ctx->acou, zsite,
                      [&](auto kern, auto shape) { setattr(kern, decltype(shape)::SMEM); })) {
   } else if (!zsite && g.Lz <= kLaneMax && pz.nst <= 2 && (pz.nst == 1 || pz.r[1] <= 10)) {
-    int pw = std::max(1, cw / W);
-    while (pw > 1 && (size_t)ncx * g.Lz * pw * 16 > (size_t)(smem_optin - 8192) / 2) pw /= 2;  // two tiles per SM
-    zk->CW = pw * W;
+    int lpw = 0;
+    while (lpw < 2 && (2 << lpw) * W <= cw) ++lpw;
+    while (lpw > 0 && ((size_t)ncx * g.Lz * 16 << lpw) > (size_t)(smem_optin - 8192) / 2) --lpw;  // two tiles per SM
+    zk->CW = W << lpw;
+    zg->lpw = lpw;
     zg->R1 = pz.r[0];
     zg->R2 = pz.nst == 2 ? pz.r[1] : 1;
-    zg->lpw = pw == 4 ? 2 : pw == 2 ? 1 : 0;
     zg->d1 = fast_div(zg->R1);
     zg->d2 = fast_div(zg->R2);
     // FP32 elements are pairs of slots: with an odd Lx/2 the last pair of a row
@@ -497,7 +498,7 @@ int plan_z(fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_
     zk->ntx = div_up(zg->ncol, zk->CW);
     zk->nreg = zk->ntx * g.Ly;
     zk->nnyq = with_nyq ? 0 : div_up(g.Ly, zk->CW);
-    const int smem = (int)((size_t)ncx * g.Lz * pw * 16);
+    const int smem = (int)((size_t)ncx * g.Lz * 16 << lpw);
     if (ctx->acou) setattr(k_z_lane<T, 0, 0, true>, smem);
     else setattr(k_z_lane<T, 0, 0, false>, smem);
   } else {
@@ -945,14 +946,18 @@ int validate(const fg_params* p, std::string* why) {
   return FG_OK;
 }
 
-// The widest z tile the context's plan allows.  By default 4 elements of 16
-// bytes (64-byte rows), or 2 where that leaves SMs without a tile (32^3 mixed:
-// z pass 14.6 us with 68 tiles, 12.6 with 136) and for acoustic 128-layer
-// supercells, whose wider tiles do not fit the ring (with_z_lane).
+// The widest z tile the context's plan allows, a power of two (a plan's width
+// may be any number: fg_set_plan, fg_wisdom_import).  By default 4 elements of
+// 16 bytes (64-byte rows), or 2 where that leaves SMs without a tile (32^3
+// mixed: z pass 14.6 us with 68 tiles, 12.6 with 136).
 template <typename T>
 int plan_cw(const fg_ctx* ctx, int nsm) {
   constexpr int cap = z_cw_cap<T>();
-  if (ctx->plan_zcw > 0) return std::min(ctx->plan_zcw, cap);
+  if (ctx->plan_zcw > 0) {
+    int cw = cap;
+    while (cw > ctx->plan_zcw) cw /= 2;
+    return cw;
+  }
   const Geom& g = ctx->g;
   if (g.m % cap == 0 && g.m / cap * g.Ly < nsm) return cap / 2;
   return cap;
