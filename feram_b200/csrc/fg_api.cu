@@ -126,7 +126,8 @@ struct fg_ctx {
   ZTiles zk{};  // tiles of the k-space pass (zt, or the runtime k_z_lane's)
   ZGeo zg{};    // runtime k_z_lane; R1 = 0: not in use
   XyGeo xyg{}, xyg64{};  // runtime two-stage x-y kernels (nt = 0: not in use) in the context's precision and in FP64
-  ZTiles zt{}, zt6{}, zt1{};  // z tiles: MD k-space (9 comps, T), table build (6, FP64), modulation (1, FP64)
+  // z tiles: MD k-space (9 comps, T), FFT entry points (3, T), table build (6, FP64), modulation (1, FP64)
+  ZTiles zt{}, zt3{}, zt6{}, zt1{};
   int smem_xy = 0, smem_xy64 = 0, smem_z = 0, smem_z3 = 0, smem_z6 = 0, smem_z1 = 0;
   int grid_elem = 1;
   // one resident wave of the step's streaming kernels (grid-stride loops):
@@ -946,21 +947,26 @@ int validate(const fg_params* p, std::string* why) {
   return FG_OK;
 }
 
-// The widest z tile the context's plan allows, a power of two (a plan's width
-// may be any number: fg_set_plan, fg_wisdom_import).  By default 4 elements of
-// 16 bytes (64-byte rows), or 2 where that leaves SMs without a tile (32^3
-// mixed: z pass 14.6 us with 68 tiles, 12.6 with 136).
+// The z tile width of the context's plan, a power of two (a plan's width may
+// be any number: fg_set_plan, fg_wisdom_import), the cap by default.  The z
+// pass of the FFT entry points takes it as it is: its compile-time kernels are
+// for the cap (32^3: forward transforms 13.2 us, 15.2 at half the cap).
+template <typename T>
+int plan_cw_max(const fg_ctx* ctx) {
+  int cw = z_cw_cap<T>();
+  while (ctx->plan_zcw > 0 && cw > ctx->plan_zcw) cw /= 2;
+  return cw;
+}
+
+// The widest tile of the k-space pass.  By default 4 elements of 16 bytes
+// (64-byte rows), or 2 where that leaves SMs without a tile (32^3 mixed:
+// z pass 14.6 us with 68 tiles, 12.6 with 136).
 template <typename T>
 int plan_cw(const fg_ctx* ctx, int nsm) {
-  constexpr int cap = z_cw_cap<T>();
-  if (ctx->plan_zcw > 0) {
-    int cw = cap;
-    while (cw > ctx->plan_zcw) cw /= 2;
-    return cw;
-  }
+  const int cw = plan_cw_max<T>(ctx);
   const Geom& g = ctx->g;
-  if (g.m % cap == 0 && g.m / cap * g.Ly < nsm) return cap / 2;
-  return cap;
+  if (ctx->plan_zcw == 0 && g.m % cw == 0 && g.m / cw * g.Ly < nsm) return cw / 2;
+  return cw;
 }
 
 // z tiles: CW is the largest power of two <= cwmax dividing Lx/2 whose
@@ -1028,12 +1034,13 @@ int create_impl(fg_ctx* ctx) {
   ctx->acou = P.mass_acou[0] > 0.0;
   ctx->ncx = ctx->acou ? 12 : 9;
   ctx->zt = tiles(ctx->ncx, sizeof(cplx<T>), plan_cw<T>(ctx, nsm));
+  ctx->zt3 = tiles(ctx->ncx, sizeof(cplx<T>), plan_cw_max<T>(ctx));
   ctx->zt6 = tiles(6, sizeof(cplx<double>), 8);
   ctx->zt1 = tiles(1, sizeof(cplx<double>), 8);
   if ((size_t)ctx->ncx * g.Lz * ctx->zt.CW * sizeof(cplx<T>) > (size_t)smem_max)
     return fail(ctx, FG_ERR_UNSUPPORTED, "a z pencil of the supercell does not fit in shared memory");
   ctx->smem_z = (int)(ctx->ncx * ((size_t)g.Lz * ctx->zt.CW) * sizeof(cplx<T>));
-  ctx->smem_z3 = (int)(3 * (size_t)g.Lz * ctx->zt.CW * sizeof(cplx<T>));
+  ctx->smem_z3 = (int)(3 * (size_t)g.Lz * ctx->zt3.CW * sizeof(cplx<T>));
   ctx->smem_z6 = (int)(6 * (size_t)g.Lz * ctx->zt6.CW * sizeof(cplx<double>));
   ctx->smem_z1 = (int)(1 * (size_t)g.Lz * ctx->zt1.CW * sizeof(cplx<double>));
   // FP64 too (the table build), so that both precisions leave the same slots
@@ -1067,8 +1074,8 @@ int create_impl(fg_ctx* ctx) {
       with_xy_fwd<double, SRC_FIELD>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy64); });
       with_xy_inv<T>(g.m, g.Ly, [&](auto k, int) { setattr(k, ctx->smem_xy); });
     }
-    with_z_pass<T, false>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
-    with_z_pass<T, true>(g.Lz, ctx->zt.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
+    with_z_pass<T, false>(g.Lz, ctx->zt3.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
+    with_z_pass<T, true>(g.Lz, ctx->zt3.CW, [&](auto k) { setattr(k, ctx->smem_z3); });
     setattr(k_z_ewald_pack<T>, ctx->smem_z6);
     setattr(k_z_modulation_pack<T>, ctx->smem_z1);
     if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
@@ -1516,9 +1523,9 @@ int get_acouK_impl(fg_ctx* ctx, double* out) {
 // z pass of the 3-component spectrum in ctx->spec
 template <typename T, bool INV>
 int launch_z_pass(fg_ctx* ctx) {
-  with_z_pass<T, INV>(ctx->g.Lz, ctx->zt.CW, [&](auto kern) {
-    kern<<<ctx->zt.nreg + ctx->zt.nnyq, kThreadsZ, ctx->smem_z3, ctx->stream>>>(
-        (cplx<T>*)ctx->spec, ctx->g, ctx->pz, (const cplx<T>*)ctx->twz, 3, ctx->zt);
+  with_z_pass<T, INV>(ctx->g.Lz, ctx->zt3.CW, [&](auto kern) {
+    kern<<<ctx->zt3.nreg + ctx->zt3.nnyq, kThreadsZ, ctx->smem_z3, ctx->stream>>>(
+        (cplx<T>*)ctx->spec, ctx->g, ctx->pz, (const cplx<T>*)ctx->twz, 3, ctx->zt3);
   });
   CKL();
   return FG_OK;
@@ -1658,7 +1665,6 @@ int set_zsite(fg_ctx* ctx, bool on) {
   ctx->zk = zk;
   ctx->zg = zg;
   ctx->smem_z = smem_z;
-  ctx->smem_z3 = (int)(3 * (size_t)g.Lz * zt.CW * sizeof(cplx<T>));
   ctx->zsite = on;
   ctx->g.k0_exact = sizeof(T) == 4 && !on ? 1 : 0;  // Z* u has no plane sums
   ctx->ltab_ready = false;
@@ -2906,13 +2912,14 @@ int apply_plan_t(fg_ctx* ctx, int zcw, int waves) {
   const int smem_max = smem_optin - 8192;
   const int old_zcw = ctx->plan_zcw;
   ctx->plan_zcw = zcw;
-  const int cwmax = plan_cw<T>(ctx, nsm);
+  const int cwmax = plan_cw<T>(ctx, nsm), cw3 = plan_cw_max<T>(ctx);
   ctx->plan_zcw = old_zcw;
+  const ZTiles zt3 = z_tiles(g, ctx->ncx, sizeof(cplx<T>), cw3, smem_max);
   const ZTiles zt = z_tiles(g, ctx->ncx, sizeof(cplx<T>), cwmax, smem_max);
   if ((size_t)ctx->ncx * g.Lz * zt.CW * sizeof(cplx<T>) > (size_t)smem_max)
     return fail(ctx, FG_ERR_UNSUPPORTED, "a z pencil of the supercell does not fit in shared memory");
   const int smem_z = (int)(ctx->ncx * ((size_t)g.Lz * zt.CW) * sizeof(cplx<T>));
-  const int smem_z3 = (int)(3 * (size_t)g.Lz * zt.CW * sizeof(cplx<T>));
+  const int smem_z3 = (int)(3 * (size_t)g.Lz * zt3.CW * sizeof(cplx<T>));
   cudaError_t ea = cudaSuccess;
   auto setattr = [&](auto kern, int bytes) {
     cudaFuncAttributes fa;
@@ -2925,8 +2932,8 @@ int apply_plan_t(fg_ctx* ctx, int zcw, int waves) {
   ZTiles zk;
   ZGeo zg;
   if (const int rc = plan_z<T>(ctx, zt, cwmax, ctx->ncx, ctx->zsite, smem_z, smem_optin, &zk, &zg)) return rc;
-  with_z_pass<T, false>(g.Lz, zt.CW, [&](auto k) { setattr(k, smem_z3); });
-  with_z_pass<T, true>(g.Lz, zt.CW, [&](auto k) { setattr(k, smem_z3); });
+  with_z_pass<T, false>(g.Lz, zt3.CW, [&](auto k) { setattr(k, smem_z3); });
+  with_z_pass<T, true>(g.Lz, zt3.CW, [&](auto k) { setattr(k, smem_z3); });
   if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
   CK(cudaStreamSynchronize(ctx->stream));
   if (zk.nreg + zk.nnyq > ctx->zk.nreg + ctx->zk.nnyq) {
@@ -2937,6 +2944,7 @@ int apply_plan_t(fg_ctx* ctx, int zcw, int waves) {
     ctx->broken = false;
   }
   ctx->zt = zt;
+  ctx->zt3 = zt3;
   ctx->zk = zk;
   ctx->zg = zg;
   ctx->smem_z = smem_z;

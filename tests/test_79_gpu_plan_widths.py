@@ -68,3 +68,24 @@ def test_any_width_with_a_zstar_per_site(fg, prec):
         for z in WIDTHS:
             ctx.set_plan(z)
             _check(_force(ctx, u), want)
+
+
+@pytest.mark.parametrize("prec", [A.FG_PREC_FP64, A.FG_PREC_MIXED])
+@pytest.mark.parametrize("L", ["16 16 16", "32 32 32", "24 24 24", "20 18 20", "18 5 9"])
+def test_fft_entry_points_at_any_width(fg, prec, L):
+    """The 3-component transforms, whose z tiles follow the plan but not the
+    k-space pass's default, against numpy: relative to the largest bin, 5
+    roundings per radix-2 level of the forward transform and as many again
+    for the way back."""
+    p = helpers.params(L=L)
+    f = helpers.fp32_config(helpers.seeded_u(p, 8, sigma=1.0))
+    x = A.physical(f, p)
+    want = np.fft.rfftn(x, axes=(0, 1, 2))
+    tol = 5 * np.log2(p.N) * (2.0**-53 if prec == A.FG_PREC_FP64 else 2.0**-24)
+    with fb.Context(p, prec) as ctx:
+        for z in (0,) + WIDTHS:
+            ctx.set_plan(z)
+            X = ctx.fft_r2c3(f)[:p.Lz, :p.Ly, :p.Lx // 2 + 1]
+            assert np.abs(X - want).max() <= tol * np.abs(want).max(), z
+            back = A.physical(ctx.fft_c2r3(ctx.fft_r2c3(f)), p) / p.N
+            assert np.abs(back - x).max() <= 2 * tol * np.abs(x).max(), z
