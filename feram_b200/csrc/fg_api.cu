@@ -671,12 +671,13 @@ int enqueue_wave(fg_ctx* ctx) {
   return FG_OK;
 }
 
-// film: u is mirrored in the same pass; wave: the step's field is set in it
+// film: u is mirrored in the same pass, to Lz - 1 - z for gap_id 0 and to
+// Lz - z for any other (negative ones too); wave: the step's field is set in it
 template <typename T>
 int enqueue_kick_drift(fg_ctx* ctx, bool film = false, bool wave = false) {
   launch_dep(ctx, k_kick_drift<T>, ctx->grid_kd, kThreadsElem, 0, (T*)ctx->p, (T*)ctx->u, (const T*)ctx->F,
              ctx->sc, ctx->g, ctx->layer_minv, (const T*)ctx->site_minv,
-             (const Phys*)(wave ? ctx->ph : nullptr), film ? (int)ctx->P.gap_id : -1, (const RepArgs*)nullptr);
+             (const Phys*)(wave ? ctx->ph : nullptr), film ? (int)(ctx->P.gap_id != 0) : -1, (const RepArgs*)nullptr);
   CKL();
   return FG_OK;
 }

@@ -3085,7 +3085,7 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
     layer_minv = a.layer_minv;
   }
   if (wave != nullptr && blockIdx.x == 0 && threadIdx.x == 0) wave_step(wave, sc);
-  // Film (gap_id >= 0): every layer's momenta are kicked, the source layers'
+  // gap_id: -1 for no film.  Film: every layer's momenta are kicked, the source layers'
   // dipoles drift and are written to their partners' layer as well
   auto partner = [&](int z) { return gap_id < 0 ? z : film_partner(z, g.Lz, gap_id); };
   const long long ns = g.nsite;

@@ -1,0 +1,41 @@
+"""Films whose mirror runs inside the step's kernels, where the inputs are out
+of the ordinary: a negative gap_id (every gap_id but 0 mirrors layer z to
+Lz - z, mirror.F:9-36; only positive ones freeze layers), against the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import helpers
+import oracle_lib
+from feram_b200 import _capi as A
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec", [A.FG_PREC_FP64, A.FG_PREC_MIXED])
+@pytest.mark.parametrize("L", ["8 12 10", "10 9 6"])
+def test_negative_gap_id_steps_match_oracle(fg, prec, L):
+    p = helpers.params(L=L, kelvin="250", bulk_or_film="'film'", gap_id="-2", external_E_field="0.001 -0.0005 0.002")
+    u, q = helpers.seeded_u(p, 21, sigma=0.08), helpers.seeded_p(p, 21, sigma=0.01)
+    o = oracle_lib.Oracle(p)
+    o.set_state(u, q)
+    eo = o.force()
+    eo.dipo_kinetic = o.kinetic_energy_dipo()
+    with fg.Context(p, prec) as ctx:
+        ctx.build_tables()
+        ctx.set_state(u, q)
+        eg = ctx.mirror_force_mirror()
+        o.set_state(None, None, 1.0, 0.0, 0.0)
+        h = o.L.oracle_nose_poincare_hamiltonian(o.h, C.byref(eo))
+        o.set_state(None, None, 1.0, 0.0, h)
+        ctx.set_thermostat(1.0, 0.0, h)
+        for _ in range(10):
+            o.nose_poincare(eo)
+            ctx.nose_poincare(eg)
+        so, sg = o.get_state(), ctx.get_state()
+    tol = 1e-9 if prec == A.FG_PREC_FP64 else 2e-5  # as the films of the other gap_ids
+    for k in ("dipoR", "dipoP", "dVddi"):
+        a, b = A.physical(sg[k], p), A.physical(so[k], p)
+        assert np.abs(a - b).max() <= tol * np.abs(b).max(), k
+    assert abs(sg["s"] - so["s"]) <= tol
