@@ -2588,8 +2588,9 @@ template <> struct StepCoef<float> {
 };
 
 // Masked kinetic sums of the closing kick (35f) of one site: p <- p - c F
-// and p^2/m, p.F/m, F^2/m in T, added to ke (FP64) when the site counts.
-template <typename T>
+// and p^2/m, p.F/m, F^2/m, formed in S and added to ke (FP64) when the site
+// counts.  S: T; FP64 for films, as k_kick_close's loop over sites.
+template <typename S, typename T>
 __device__ __forceinline__ void close_site(T* __restrict__ p, long long ns, long long i, const StepCoef<T>& c, T o0, T o1, T o2,
                                            bool counted, double mi, double* ke) {
   const T q0 = p[i] - c * o0, q1 = p[ns + i] - c * o1, q2 = p[2 * ns + i] - c * o2;
@@ -2597,9 +2598,9 @@ __device__ __forceinline__ void close_site(T* __restrict__ p, long long ns, long
   p[ns + i] = q1;
   p[2 * ns + i] = q2;
   if (counted) {
-    ke[0] += (double)(q0 * q0 + q1 * q1 + q2 * q2) * mi;
-    ke[1] += (double)(q0 * o0 + q1 * o1 + q2 * o2) * mi;
-    ke[2] += (double)(o0 * o0 + o1 * o1 + o2 * o2) * mi;
+    ke[0] += (double)((S)q0 * q0 + (S)q1 * q1 + (S)q2 * q2) * mi;
+    ke[1] += (double)((S)q0 * o0 + (S)q1 * o1 + (S)q2 * o2) * mi;
+    ke[2] += (double)((S)o0 * o0 + (S)o1 * o1 + (S)o2 * o2) * mi;
   }
 }
 
@@ -2719,7 +2720,7 @@ __global__ void __launch_bounds__(256, 2)
       }
       if constexpr (CLOSE) {
         const int z = (int)(i / g.plane_r);
-        close_site(p, ns, i, cf, h0, h1, h2, site_sump ? site_sump[i] != 0 : layer_sump[z] != 0,
+        close_site<T>(p, ns, i, cf, h0, h1, h2, site_sump ? site_sump[i] != 0 : layer_sump[z] != 0,
                    site_minv ? (double)site_minv[i] : layer_minv[z], ke);
       }
     }
@@ -2825,7 +2826,8 @@ __global__ void __launch_bounds__(256, 2)
       }
       if constexpr (CLOSE) {
         const int z = (int)(i / g.plane_r);
-        close_site(p, ns, i, cf, h0, h1, h2, layer_sump[z] != 0, layer_minv[z], ke);
+        using S = std::conditional_t<FILM, double, T>;
+        close_site<S>(p, ns, i, cf, h0, h1, h2, layer_sump[z] != 0, layer_minv[z], ke);
         if constexpr (FILM) {
           const int zd = film_partner(z, g.Lz, k.gap_id);
           acc[0] += as[0];
@@ -2837,7 +2839,7 @@ __global__ void __launch_bounds__(256, 2)
             F[d] = -h0;
             F[ns + d] = -h1;
             F[2 * ns + d] = h2;
-            close_site(p, ns, d, cf, -h0, -h1, h2, layer_sump[zd] != 0, layer_minv[zd], ke);
+            close_site<S>(p, ns, d, cf, -h0, -h1, h2, layer_sump[zd] != 0, layer_minv[zd], ke);
           }
         }
       }
