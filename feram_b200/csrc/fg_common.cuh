@@ -3,11 +3,23 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-// Bounds-checked builds (-DFG_BOUNDS_CHECK=1) test every shared-memory and
-// global index of the FFT and field kernels; an out-of-range access is
-// skipped and recorded in fg_dev_error (first offending index wins).
+// Bounds-checked builds (-DFG_BOUNDS_CHECK=1) test the index ranges of the
+// transforms whose shape is known at run time: the stages of fft_smem.cuh and
+// every stage and k-space step of k_xy_fwd_gen, k_xy_inv_gen and k_z_lane, in
+// shared memory and in the field, spectrum and table arrays.  A task that would
+// leave its range is skipped and its index recorded in g_fg_err (the first
+// one wins), which the next waiting call reports.  The x-y kernels of the
+// compile-time planes have constant offsets and are not tested.
 #ifndef FG_BOUNDS_CHECK
 #define FG_BOUNDS_CHECK 0
+#endif
+#if FG_BOUNDS_CHECK
+#define FG_SKIP_UNLESS(skip, ...) \
+  if (!(__VA_ARGS__)) skip
+#define FG_AND_CHECKED(...) &&(__VA_ARGS__)
+#else  // no code
+#define FG_SKIP_UNLESS(skip, ...)
+#define FG_AND_CHECKED(...)
 #endif
 
 namespace fg {
@@ -133,5 +145,14 @@ __device__ DevError g_fg_err;
 __device__ __forceinline__ void fg_record_error(int code, long long idx) {
   if (atomicCAS(&g_fg_err.code, 0, code) == 0) g_fg_err.idx = idx;
 }
+
+#if FG_BOUNDS_CHECK
+// lo .. hi inside 0 .. n - 1?  Records the first index outside.
+__device__ __forceinline__ bool fg_in_range(long long lo, long long hi, long long n) {
+  if (lo >= 0 && hi < n) return true;
+  fg_record_error(1, lo < 0 ? lo : hi);
+  return false;
+}
+#endif
 
 }  // namespace fg

@@ -1039,6 +1039,34 @@ __device__ __forceinline__ cplx<T>* column_at(CV<T>* buf, int JS, int k, int y) 
   return reinterpret_cast<cplx<T>*>(buf + k / W * JS + y) + k % W;
 }
 
+#if FG_BOUNDS_CHECK
+// What the tasks of these kernels touch (fg_in_range):
+// the first x stage's butterfly b of group q (elements of buf, rows of the
+// plane, twiddles), class al of group q and its partner a1 (elements; columns and
+// rows of the column layout) and block a of column element j (elements,
+// spectrum rows).
+template <int R, int W>
+__device__ __forceinline__ bool group_in_range(const Geom& g, const XyGeo& h, int q, int b) {
+  const int last = b + (R - 1) * h.R2;
+  const int row = q + h.NQ * (2 * W - 1) < g.Ly ? q + h.NQ * (2 * W - 1) : q + 2 * h.NQ < g.Ly && W == 2 ? q + 2 * h.NQ
+                  : W == 2 ? q + h.NQ : q;
+  return fg_in_range(q * h.QS + b, q * h.QS + last, h.smem / 16) && fg_in_range(b, last, g.Lx) && fg_in_range(q, row, g.Ly) &&
+         fg_in_range(0, (R - 1) * b, g.Lx);
+}
+template <int R, int W>
+__device__ __forceinline__ bool classes_in_range(const Geom& g, const XyGeo& h, int q, int al) {
+  const int a1 = al == 0 ? h.R1 / 2 : h.R1 - al;
+  const int k0 = al + h.R1 * ((R - 1) / 2), k1 = a1 + h.R1 * (R / 2 - 1), k = k0 > k1 ? k0 : k1;
+  return fg_in_range(q * h.QS + al * R, q * h.QS + a1 * R + R - 1, h.smem / 16) && fg_in_range(al, a1, h.R1) &&
+         fg_in_range(al, k, g.m) && fg_in_range(q, k / W * h.JS + g.Ly - 1, h.smem / 16);
+}
+template <int R, int W>
+__device__ __forceinline__ bool column_in_range(const Geom& g, const XyGeo& h, int j, int a) {
+  return fg_in_range(j * h.JS + a * R, j * h.JS + a * R + R - 1, h.smem / 16) && fg_in_range(a * R, a * R + R - 1, g.Ly) &&
+         fg_in_range(W * j, W * j + W - 1, g.KXP);
+}
+#endif
+
 template <typename T, int MODE>
 __global__ void __launch_bounds__(512, 1)
     k_xy_fwd_gen(const T* __restrict__ src, cplx<T>* __restrict__ spec, Geom g, XyGeo h, const cplx<T>* __restrict__ twx,
@@ -1079,6 +1107,7 @@ __global__ void __launch_bounds__(512, 1)
     for (int t = tid; t < h.NQ * h.R2; t += nt) {
       const int q = fdiv(t, h.dR2), b = t - q * h.R2;
       const bool full = q + h.NQ * (2 * W - 1) < Ly, third = q + 2 * h.NQ < Ly;
+      FG_SKIP_UNLESS(continue, group_in_range<R, W>(g, h, q, b));
       auto ld = [&](const T* r) {
         return CV<T>{vpack(r[0], W == 2 && third ? r[2 * rows] : (T)0),
                      vpack(W == 2 || full ? r[rows] : (T)0, W == 2 && full ? r[3 * rows] : (T)0)};
@@ -1110,7 +1139,7 @@ __global__ void __launch_bounds__(512, 1)
   second_radix(h.R2, [&](auto radix) {
     constexpr int R = decltype(radix)::value;
     const int al = fdiv(tid, h.dNQ), q = tid - al * h.NQ;
-    const bool on = tid < (h.R1 / 2) * h.NQ;
+    const bool on = tid < (h.R1 / 2) * h.NQ FG_AND_CHECKED(classes_in_range<R, W>(g, h, q, al));
     const int a1 = al == 0 ? h.R1 / 2 : h.R1 - al;
     CV<T> v0[R], v1[R];
     if (on) {
@@ -1146,6 +1175,7 @@ __global__ void __launch_bounds__(512, 1)
     for (int t = tid; t < h.NJ * h.RY2; t += nt) {
       const int b = fdiv(t, h.dNJ), j = t - b * h.NJ;
       CV<T>* d = buf + j * h.JS + b;
+      FG_SKIP_UNLESS(continue, fg_in_range(j * h.JS + b, j * h.JS + b + (R - 1) * h.RY2, h.smem / 16));
       CV<T> v[R];
 #pragma unroll
       for (int s = 0; s < R; ++s) v[s] = cv_of(*reinterpret_cast<const rowvec<T>*>(d + s * h.RY2));
@@ -1164,6 +1194,7 @@ __global__ void __launch_bounds__(512, 1)
     for (int t = tid; t < h.NJ * h.RY1; t += nt) {
       const int a = fdiv(t, h.dNJ), j = t - a * h.NJ;
       const CV<T>* d = buf + j * h.JS + a * R;
+      FG_SKIP_UNLESS(continue, column_in_range<R, W>(g, h, j, a));
       CV<T> v[R];
 #pragma unroll
       for (int s = 0; s < R; ++s) v[s] = cv_ld(d + s);
@@ -1241,6 +1272,7 @@ __global__ void __launch_bounds__(512, 1)
     for (int t = tid; t < h.NJ * h.RY1; t += nt) {
       const int a = fdiv(t, h.dNJ), j = t - a * h.NJ;
       const cplx<T>* r = src + (long long)(a * R) * g.KXP + W * j;
+      FG_SKIP_UNLESS(continue, column_in_range<R, W>(g, h, j, a));
       CV<T> v[R];
 #pragma unroll
       for (int s = 0; s < R; ++s) {
@@ -1267,6 +1299,7 @@ __global__ void __launch_bounds__(512, 1)
     for (int t = tid; t < h.NJ * h.RY2; t += nt) {
       const int b = fdiv(t, h.dNJ), j = t - b * h.NJ;
       CV<T>* d = buf + j * h.JS + b;
+      FG_SKIP_UNLESS(continue, fg_in_range(j * h.JS + b, j * h.JS + b + (R - 1) * h.RY2, h.smem / 16));
       CV<T> v[R];
       v[0] = cv_ld(d);
 #pragma unroll
@@ -1280,7 +1313,7 @@ __global__ void __launch_bounds__(512, 1)
   second_radix(h.R2, [&](auto radix) {
     constexpr int R = decltype(radix)::value;
     const int al = fdiv(tid, h.dNQ), q = tid - al * h.NQ;
-    const bool on = tid < (h.R1 / 2) * h.NQ;
+    const bool on = tid < (h.R1 / 2) * h.NQ FG_AND_CHECKED(classes_in_range<R, W>(g, h, q, al));
     const int a1 = al == 0 ? h.R1 / 2 : h.R1 - al;
     CV<T> v0[R], v1[R];
     if (on) {
@@ -1320,6 +1353,7 @@ __global__ void __launch_bounds__(512, 1)
       const int q = fdiv(t, h.dR2), b = t - q * h.R2;
       const bool full = q + h.NQ * (2 * W - 1) < Ly, third = q + 2 * h.NQ < Ly;
       const CV<T>* d = buf + q * h.QS + b;
+      FG_SKIP_UNLESS(continue, group_in_range<R, W>(g, h, q, b));
       CV<T> v[R];
       v[0] = cv_ld(d);
 #pragma unroll
@@ -2157,11 +2191,26 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
       lane_tasks<decltype(count)::value, NT>(tid, f);
     }
   };
+#if FG_BOUNDS_CHECK
+  // what a task touches (fg_in_range): butterfly b of the first stage (R
+  // elements r2 apart, as many z of the spectrum, twiddles) and block a of the
+  // second, in component c
+  const int blen = RT ? NC * Lz * (zt.CW / W) : NC * LZ * PW;  // elements of buf
+  auto first_in_range = [&](int c, int b, int R) {
+    const int lastz = b + (R - 1) * r2, y = ysb > ys ? ysb : ys;
+    return fg_in_range(c * ZS + b * pwn, c * ZS + (lastz | swap) * pwn + pw, blen) && fg_in_range(b, lastz, Lz) &&
+           fg_in_range(0, (R - 1) * b, Lz) && fg_in_range(ys, y, g.Ly) && fg_in_range(col, nyq ? col : col + W - 1, g.KXP);
+  };
+  auto second_in_range = [&](int c, int a, int R) {
+    return fg_in_range((c * Lz + a * r2) * pwn, (c * Lz + a * r2 + R - 1) * pwn + pw, blen) && fg_in_range(a, a, r1);
+  };
+#endif
   // forward: first stage from the spectrum
   auto first = [&](auto nyqt, auto radix) {
     constexpr int R = decltype(radix)::value;
     tasks(std::integral_constant<int, Z::T1>(), NC * pwn * r2, [&](int t) {
       const int r = by_pw(t), c = by_r2(r), b = r - c * r2, bx = b ^ swap;
+      FG_SKIP_UNLESS(return, first_in_range(c, b, R));
       unsigned off = c * cstep + b * zstep;
       CV<T> v[R];
 #pragma unroll
@@ -2206,6 +2255,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     constexpr int R = decltype(radix)::value;
     tasks(std::integral_constant<int, Z::T2>(), NC * pwn * r1, [&](int t) {
       const int r = by_pw(t), c = by_r1(r), a = r - c * r1, x = a & swap;
+      FG_SKIP_UNLESS(return, second_in_range(c, a, R));
       CV<T>*d0 = buf + c * ZS + pw + (a * r2 + x) * pwn, *d1 = d0 - 2 * x * pwn;  // z even / odd of the block
       CV<T> v[R];
 #pragma unroll
@@ -2234,6 +2284,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
 #pragma unroll 1
   for (int e = tid; e < ZS; e += NT) {
     const int zs = by_pw(e), zx = zs ^ (by_r2(zs) & swap);
+    FG_SKIP_UNLESS(continue, fg_in_range(zx * pwn + pw, (NC - 1) * ZS + zx * pwn + pw, blen) && fg_in_range(zs, zs, Lz));
     CV<T>* el = buf + zx * pwn + pw;
     CV<T> u[3], d[6];
 #pragma unroll
@@ -2433,6 +2484,7 @@ __global__ void __launch_bounds__(ZCT<T, LZ, PW, ACOU>::NT, ZCT<T, LZ, PW, ACOU>
     constexpr int R = decltype(radix)::value;
     tasks(std::integral_constant<int, Z::T1>(), NC * pwn * r2, [&](int t) {
       const int r = by_pw(t), c = by_r2(r), b = r - c * r2, bx = b ^ swap;
+      FG_SKIP_UNLESS(return, first_in_range(c, b, R));
       const CV<T>* d = buf + c * ZS + pw;
       CV<T> v[R];
       v[0] = cv_ld(d + b * pwn);
