@@ -133,6 +133,7 @@ struct fg_ctx {
   // one resident wave of the step's streaming kernels (grid-stride loops):
   // k_kick_drift, k_kick_close, k_assemble; <= grid_elem
   int grid_kd = 1, grid_kc = 1, grid_as = 1, grid_asc = 1;  // grid_asc: k_assemble<T, true>
+  int device = 0;  // current at fg_create
   cudaStream_t stream = nullptr;
   // fields (T = float or double)
   void* u = nullptr;
@@ -1022,6 +1023,7 @@ int create_impl(fg_ctx* ctx) {
     return fail(ctx, FG_ERR_UNSUPPORTED, "L/2 (x), Ly and Lz must factor into 2, 3 and 5");
   int dev = 0;
   CK(cudaGetDevice(&dev));
+  ctx->device = dev;
   int smem_max = 0, nsm = 0;
   CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const int smem_optin = smem_max;
@@ -2014,12 +2016,28 @@ int fg_time_fft(fg_ctx* ctx, int reps, double* ms) {
   return ctx->prec == FG_PREC_MIXED ? time_fft_impl<float>(ctx, reps, ms) : time_fft_impl<double>(ctx, reps, ms);
 }
 
+// The context's device made current while a scalar kernel is launched: the
+// calls of the stepping loop (fg_set_uniform_E, fg_set_thermostat, the steps'
+// graphs) may come from a thread whose current device is another one, where an
+// ordinary launch into the context's stream is refused.
+struct OnDevice {
+  int before = -1;
+  explicit OnDevice(int device) {
+    int cur = device;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != device && cudaSetDevice(device) == cudaSuccess) before = cur;
+  }
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 // s, pi and H0 on the device and in sc_host, and the momentum kick they imply
 static int set_thermostat(fg_ctx* ctx, double s, double pi, double H0) {
   ctx->sc_host->s = s;
   ctx->sc_host->pi = pi;
   ctx->sc_host->H0 = H0;
   ctx->sc_host->kick_coef = ctx->P.dt_2 * s;
+  const OnDevice on(ctx->device);
   k_set_thermostat<<<1, 32, 0, ctx->stream>>>(ctx->sc, s, pi, H0, ctx->P.dt_2 * s);
   CKL();
   ctx->np_ready = false;
@@ -2206,6 +2224,7 @@ int fg_get_acouK(fg_ctx* ctx, double* acouK) {
 int fg_set_uniform_E(fg_ctx* ctx, const double E[3]) {
   if (!ctx || !ctx->stream || !ctx->sc_host || !E) return FG_ERR_ARG;
   for (int a = 0; a < 3; ++a) ctx->sc_host->E[a] = E[a];  // for push_scalars
+  const OnDevice on(ctx->device);
   k_set_field<<<1, 32, 0, ctx->stream>>>(ctx->sc, E[0], E[1], E[2]);
   CKL();
   // The stored dVddi and energies stay those of the last evaluation, as
