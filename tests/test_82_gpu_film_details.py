@@ -60,3 +60,45 @@ def test_mixed_kinetic_energy_of_planes_cut_off_a_vector(fg, kind, L, gap):
             step = e.dipo_kinetic
             ke = ctx.kinetic_energy_dipo()
             assert abs(step - ke) <= 3 * p.N * 2.0**-53 * ke, (step, ke)
+
+
+@pytest.mark.parametrize("prec", [A.FG_PREC_FP64, A.FG_PREC_MIXED])
+@pytest.mark.parametrize("kind,L,gap", [("film", "12 10 8", 0), ("epit", "8 12 10", 2)])
+def test_device_field_wave_through_run_steps(fg, prec, kind, L, gap):
+    """The field wave set in the mirrored drift's launch, over two graphs of
+    eight steps and three single ones (molecular-dynamics.F:66-76), against
+    the oracle's molecular_dynamics.  Tolerances as for the films' steps."""
+    extra = {"epi_strain": "-0.01"} if kind == "epit" else {}
+    p = helpers.params(L=L, kelvin="280", bulk_or_film=f"'{kind}'", gap_id=str(gap), E_wave_type="'triangular_sin'",
+                       external_E_field="0.001 -0.0005 0.002", n_E_wave_period="12", n_thermalize="2", n_average="17",
+                       **extra)
+    u, q = helpers.seeded_u(p, 31, sigma=0.05), helpers.seeded_p(p, 31, sigma=0.01)
+    n = 19
+    w0 = (C.c_double * 3)()
+    amp = (C.c_double * 3)(*p.external_E_field)
+    assert A.lib().fg_wave(p.E_wave_type, 0, p.n_thermalize, p.n_E_wave_period, amp, w0) == 0
+    o = oracle_lib.Oracle(p)
+    o.set_state(u, q)
+    o.set_uniform_E(list(w0))
+    eo = o.force()
+    eo.dipo_kinetic = o.kinetic_energy_dipo()
+    o.md(1, n, 1, eo)
+    so = o.get_state()
+    with fg.Context(p, prec) as ctx:
+        ctx.build_tables()
+        ctx.set_state(u, q)
+        ctx.set_uniform_E(list(w0))
+        e = ctx.mirror_force_mirror()
+        e.dipo_kinetic = ctx.kinetic_energy_dipo()
+        ctx.nose_poincare_hamiltonian(e)
+        ctx.set_thermostat(1.0, 0.0, e.H_Nose_Poincare)
+        ctx.set_wave(True, 0)
+        eg = ctx.run_steps(n)
+        sg = ctx.get_state()
+    tol = 1e-9 if prec == A.FG_PREC_FP64 else 2e-5
+    for k in ("dipoR", "dipoP"):
+        a, b = A.physical(sg[k], p), A.physical(so[k], p)
+        assert np.abs(a - b).max() <= tol * np.abs(b).max(), k
+    assert abs(sg["s"] - so["s"]) <= tol
+    ee = helpers.energy_errors(eg, eo, A.POTENTIAL_FIELDS + ["dipo_kinetic"])
+    assert max(ee.values()) <= tol, ee
