@@ -462,13 +462,39 @@ int launch_z_kspace(fg_ctx* ctx, cplx<T>* acouK_out, int nrep = 1, const RepArgs
 
 // How the k-space pass runs on tiles zt of ncx components: the compile-time
 // k_z_lane where with_z_lane has it, else its runtime form for lengths of two
-// stages, whose rows need not divide into tiles (as wide as zt's cap `cw`
-// allows: 1, 2 or 4 elements), else k_z_kspace (smem_z bytes).  Raises the
-// kernel's shared-memory limit; the caller stores the result.
+// stages (zg->R1 > 0), whose rows need not divide into tiles (as wide as zt's
+// cap `cw` allows: 1, 2 or 4 elements), else k_z_kspace on zt.
 template <typename T>
-int plan_z(fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_z, int smem_optin, ZTiles* zk, ZGeo* zg) {
+void z_shape(const fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_optin, ZTiles* zk, ZGeo* zg) {
   constexpr int W = kLanes<T>;
   const Geom& g = ctx->g;
+  const FftPlan& pz = ctx->pz;
+  *zk = zt;
+  *zg = ZGeo{};
+  if (with_z_lane<T>(g.Lz, zt.CW, ctx->acou, zsite, [](auto, auto) {})) return;
+  if (zsite || g.Lz > kLaneMax || pz.nst > 2 || (pz.nst == 2 && pz.r[1] > 10)) return;
+  int lpw = 0;
+  while (lpw < 2 && (2 << lpw) * W <= cw) ++lpw;
+  while (lpw > 0 && ((size_t)ncx * g.Lz * 16 << lpw) > (size_t)(smem_optin - 8192) / 2) --lpw;  // two tiles per SM
+  zk->CW = W << lpw;
+  zg->lpw = lpw;
+  zg->R1 = pz.r[0];
+  zg->R2 = pz.nst == 2 ? pz.r[1] : 1;
+  zg->d1 = fast_div(zg->R1);
+  zg->d2 = fast_div(zg->R2);
+  // FP32 elements are pairs of slots: with an odd Lx/2 the last pair of a row
+  // ends with the Nyquist slot
+  const bool with_nyq = W == 2 && g.m % 2 != 0;
+  zg->ncol = g.m + (with_nyq ? 1 : 0);
+  zk->ntx = div_up(zg->ncol, zk->CW);
+  zk->nreg = zk->ntx * g.Ly;
+  zk->nnyq = with_nyq ? 0 : div_up(g.Ly, zk->CW);
+}
+
+// z_shape and its kernel's shared-memory limit (smem_z: bytes of k_z_kspace);
+// the caller stores the result.
+template <typename T>
+int plan_z(fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_z, int smem_optin, ZTiles* zk, ZGeo* zg) {
   cudaError_t ea = cudaSuccess;
   auto setattr = [&](auto kern, int bytes) {
     cudaFuncAttributes fa;
@@ -478,32 +504,13 @@ int plan_z(fg_ctx* ctx, const ZTiles& zt, int cw, int ncx, bool zsite, int smem_
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     if (e != cudaSuccess) ea = e;
   };
-  *zk = zt;
-  *zg = ZGeo{};
-  const FftPlan& pz = ctx->pz;
-  if (with_z_lane<T>(g.Lz, zt.CW, ctx->acou, zsite,
-                     [&](auto kern, auto shape) { setattr(kern, decltype(shape)::SMEM); })) {
-  } else if (!zsite && g.Lz <= kLaneMax && pz.nst <= 2 && (pz.nst == 1 || pz.r[1] <= 10)) {
-    int lpw = 0;
-    while (lpw < 2 && (2 << lpw) * W <= cw) ++lpw;
-    while (lpw > 0 && ((size_t)ncx * g.Lz * 16 << lpw) > (size_t)(smem_optin - 8192) / 2) --lpw;  // two tiles per SM
-    zk->CW = W << lpw;
-    zg->lpw = lpw;
-    zg->R1 = pz.r[0];
-    zg->R2 = pz.nst == 2 ? pz.r[1] : 1;
-    zg->d1 = fast_div(zg->R1);
-    zg->d2 = fast_div(zg->R2);
-    // FP32 elements are pairs of slots: with an odd Lx/2 the last pair of a row
-    // ends with the Nyquist slot
-    const bool with_nyq = W == 2 && g.m % 2 != 0;
-    zg->ncol = g.m + (with_nyq ? 1 : 0);
-    zk->ntx = div_up(zg->ncol, zk->CW);
-    zk->nreg = zk->ntx * g.Ly;
-    zk->nnyq = with_nyq ? 0 : div_up(g.Ly, zk->CW);
-    const int smem = (int)((size_t)ncx * g.Lz * 16 << lpw);
+  z_shape<T>(ctx, zt, cw, ncx, zsite, smem_optin, zk, zg);
+  if (zg->R1 > 0) {
+    const int smem = (int)((size_t)ncx * ctx->g.Lz * 16 << zg->lpw);
     if (ctx->acou) setattr(k_z_lane<T, 0, 0, true>, smem);
     else setattr(k_z_lane<T, 0, 0, false>, smem);
-  } else {
+  } else if (!with_z_lane<T>(ctx->g.Lz, zt.CW, ctx->acou, zsite,
+                             [&](auto kern, auto shape) { setattr(kern, decltype(shape)::SMEM); })) {
     with_z_kspace<T>(ctx->acou, zsite, [&](auto kern) { setattr(kern, smem_z); });
   }
   if (ea != cudaSuccess) return fail(ctx, FG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
@@ -2997,19 +3004,29 @@ void remember_plan(const fg_ctx* ctx, int mode) {
   g_wisdom[plan_key(ctx, mode)] = PlanVal{ctx->plan_zcw, ctx->plan_waves};
 }
 
-// The candidates: z-tile widths that give distinct tiles (widest first) and
-// the streaming grids (one and two resident waves, every block).
-std::vector<int> zcw_candidates(const fg_ctx* ctx) {
-  const int cap = ctx->prec == FG_PREC_MIXED ? z_cw_cap<float>() : z_cw_cap<double>();
-  std::vector<int> out;
-  int last = -1;
-  for (int w = cap; w >= 1 && (int)out.size() < 3; w /= 2) {
-    int cw = w;
-    while (cw > 1 && ctx->g.m % cw != 0) cw /= 2;
-    if (cw != last) out.push_back(w);
-    last = cw;
+// The candidates: plan widths that give distinct k-space tiles (widest first,
+// at most three; by z_shape, since the runtime k_z_lane's tiles need not divide
+// Lx/2) and the streaming grids (one and two resident waves, every block).
+template <typename T>
+int zcw_candidates(fg_ctx* ctx, std::vector<int>* out) {
+  int dev = 0, smem_optin = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  std::vector<std::pair<int, bool>> seen;
+  for (int w = z_cw_cap<T>(); w >= 1 && (int)out->size() < 3; w /= 2) {
+    ZTiles zk;
+    ZGeo zg;
+    z_shape<T>(ctx, z_tiles(ctx->g, ctx->ncx, sizeof(cplx<T>), w, smem_optin - 8192), w, ctx->ncx, ctx->zsite,
+               smem_optin, &zk, &zg);
+    const std::pair<int, bool> tile(zk.CW, zg.R1 > 0);
+    if (std::find(seen.begin(), seen.end(), tile) != seen.end()) continue;
+    seen.push_back(tile);
+    out->push_back(w);
   }
-  return out;
+  return FG_OK;
+}
+int zcw_candidates(fg_ctx* ctx, std::vector<int>* out) {
+  return ctx->prec == FG_PREC_MIXED ? zcw_candidates<float>(ctx, out) : zcw_candidates<double>(ctx, out);
 }
 const int kWaveCandidates[3] = {1, 2, 0};
 
@@ -3079,7 +3096,9 @@ int fg_tune(fg_ctx* ctx, int steps, int* zcw, int* waves, double* ms_per_step) {
   }
   double best = 1e300, t = 0.0;
   int bz = ctx->plan_zcw, bw = ctx->plan_waves;
-  for (int z : zcw_candidates(ctx)) {
+  std::vector<int> widths;
+  rc = zcw_candidates(ctx, &widths);
+  for (int z : widths) {
     if ((rc = apply_plan(ctx, z, bw)) || (rc = time_solo(ctx, steps, 3, &t))) break;
     if (t < best) best = t, bz = z;
   }
@@ -3398,7 +3417,9 @@ int fg_batch_tune(fg_batch* b, int steps, double* ms_before, double* ms_after) {
       return r;
     };
     bool better = false;
-    for (int z : zcw_candidates(b->ctx[i])) {
+    std::vector<int> widths;
+    if ((rc = zcw_candidates(b->ctx[i], &widths))) rc = batch_fail(b, rc, b->ctx[i]->err);
+    for (int z : widths) {
       if (z == bz) continue;
       if ((rc = try_plan(z, bw, &better))) break;
       if (better) bz = z;

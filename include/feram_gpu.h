@@ -401,9 +401,11 @@ int  fg_batch_run_point(fg_batch* b, const double* kelvin, const double* E, int 
    The reference plans its transforms with FFTW_MEASURE (coord_module.F:155-377)
    and imports saved FFTW wisdom at start-up (feram_common.F:56-69,
    feram_fftw_wisdom.F).  Here a plan is the z-pencil tile width (kx columns
-   per CTA of the z kernel; the widest that divides Lx/2 and fits shared
-   memory, up to 8 (mixed) / 4 (fp64)) and the grid of the streaming kernels
-   (waves: 1 or 2 resident waves of blocks, 0 = one block per 256 sites).
+   per CTA of the z kernels, up to 8 (mixed) / 4 (fp64), rounded down to a power
+   of two and to what fits shared memory; lengths with compile-time transforms,
+   those above 160 and per-site Z* take the widest that divides Lx/2, the others
+   cut a row's last tile short) and the grid of the streaming kernels (waves: 1
+   or 2 resident waves of blocks, 0 = one block per 256 sites).
    fg_tune times the candidates on the context's own Nose-Poincare steps and
    keeps the fastest; the state (u, p, strain, s, pi, H0) is restored after
    it.  The result goes to the process's wisdom, which fg_create (solo) and
@@ -415,9 +417,11 @@ int  fg_tune(fg_ctx* ctx, int steps, int* zcw, int* waves, double* ms_per_step);
    (replicas of one supercell share a plan) and keeps the fastest; states
    restored.  ms_before / ms_after: ms per batch step (may be NULL). */
 int  fg_batch_tune(fg_batch* b, int steps, double* ms_before, double* ms_after);
-/* A plan set by hand (zcw 0: the widest that fits). */
+/* A plan set by hand.  zcw 0: the widest tile, or half of it for the k-space
+   pass where whole tiles would be fewer than the GPU has SMs. */
 int  fg_set_plan(fg_ctx* ctx, int zcw, int waves);
-/* The tile width in use, the waves setting and the two main grids. */
+/* The widest tile that divides Lx/2 under the plan, the waves setting and the
+   two main grids. */
 int  fg_get_plan(const fg_ctx* ctx, int* zcw, int* waves, int* grid_kd, int* grid_asc);
 /* Wisdom as text: "feram_b200 wisdom 1", then one line per plan
    "<solo|batch> <fp64|mixed> Lx Ly Lz components zcw waves".  Export sets
