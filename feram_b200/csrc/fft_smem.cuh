@@ -417,31 +417,13 @@ __device__ __forceinline__ void ct_inverse_from(cplx<T>* buf, const cplx<T>* tws
     ct_inverse_from<T, N, ST - 1, NT, B>(buf, tws);
   }
 }
-// Stages ST .. END-1 (forward) or ST down to END+1 (inverse), each followed
-// by __syncthreads().
-template <typename T, int N, int ST, int END, int NT, class B>
-__device__ __forceinline__ void ct_forward_range(cplx<T>* buf, const cplx<T>* tws) {
-  if constexpr (ST < END) {
-    ct_stage<T, N, ct_ls(N, ST), ct_radix(N, ST), false, NT, B>(buf, tws);
-    __syncthreads();
-    ct_forward_range<T, N, ST + 1, END, NT, B>(buf, tws);
-  }
-}
-template <typename T, int N, int ST, int END, int NT, class B>
-__device__ __forceinline__ void ct_inverse_range(cplx<T>* buf, const cplx<T>* tws) {
-  if constexpr (ST > END) {
-    ct_stage<T, N, ct_ls(N, ST), ct_radix(N, ST), true, NT, B>(buf, tws);
-    __syncthreads();
-    ct_inverse_range<T, N, ST - 1, END, NT, B>(buf, tws);
-  }
-}
-
 // One compile-time stage of a batch of COUNT transforms whose elements are
 // read through ld(t, e) and written through st(t, e, v) (t = transform,
 // e = element): the first or last stage of a pass fused with its global load
 // or store.  JFAST: consecutive threads take consecutive butterflies of one
 // transform (global rows whose butterflies run along the contiguous
 // direction); otherwise consecutive transforms, as ct_stage.  No barrier.
+// No kernel uses it now; the host test of the stages does.
 template <typename T, int N, int ST, bool INV, int NT, int COUNT, bool JFAST, class LD, class SV>
 __device__ __forceinline__ void ct_stage_io(const LD& ld, const SV& st, const cplx<T>* __restrict__ tws) {
   constexpr int LS = ct_ls(N, ST), R = ct_radix(N, ST);

@@ -203,7 +203,7 @@ struct fg_ctx {
   double* part_ke = nullptr;
   double* part_avg = nullptr;
   double* didi = nullptr;         // Geom::didi (mixed path)
-  unsigned int* done = nullptr;   // last-block tickets: [0] kicks, [1] z k-space, [2] assemble
+  unsigned int* done = nullptr;   // last-block tickets: [0] kicks, [2] assemble ([1]: not in use)
   double* avg6 = nullptr;
   double* staging = nullptr;      // padded Fortran-layout FP64 (3 components)
   size_t staging_n = 0;
@@ -224,7 +224,7 @@ struct fg_ctx {
   bool bulk_or_film_mirror() const { return P.bulk_or_film == FG_FILM || P.bulk_or_film == FG_EPIT; }
   size_t real_bytes = 0;
   // launch plan (fg_tune, fg_wisdom_import): the z-tile width asked for
-  // (0: the widest that fits) and the resident waves of the streaming
+  // (0: plan_cw's choice) and the resident waves of the streaming
   // kernels (0: one block per 256 sites, up to grid_elem)
   int plan_zcw = 0, plan_waves = 1;
   // launch priority of the kernels this context enqueues while use_prio is
@@ -1854,6 +1854,8 @@ int np_ready_for_step(fg_ctx* ctx) {
   return FG_OK;
 }
 
+// Labels of the step's passes; "k_z_kspace" is the k-space pass, whose kernel is
+// k_z_lane at the lengths it takes.
 const char* kProfNames[FG_NPROF] = {"k_kick_drift(35a,35c)", "k_xy_fwd", "k_z_kspace", "k_xy_inv+homo_strain",
                                     "k_assemble+kick(35e,35f)+np_tail"};
 
@@ -2261,7 +2263,8 @@ int fg_set_wave(fg_ctx* ctx, int on, int i_step) {
   if ((rc = push_scalars(ctx))) return rc;
   if ((on != 0) != ctx->wave_dev) {
     ctx->wave_dev = on != 0;
-    // the step graphs gain or lose their first kernel
+    // the steps set the field or no longer do: in k_kick_drift for
+    // Nose-Poincare, in a first kernel of their own (k_wave_step) otherwise
     ++ctx->gen;
     for (cudaGraphExec_t* gx : {&ctx->g_np, &ctx->g_np_multi, &ctx->g_lf, &ctx->g_vs, &ctx->g_force})
       if (*gx) {

@@ -90,11 +90,6 @@ __device__ __forceinline__ unsigned long long l2_evict_first() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(p));
   return p;
 }
-// 16-byte cp.async with that policy
-__device__ __forceinline__ void cp_async16_first(void* smem, const void* gmem, unsigned long long pol) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "l"(pol) : "memory");
-}
 // 8- or 16-byte loads of two reals (a complex value) and 16-byte loads of
 // four floats or two doubles, with that policy
 __device__ __forceinline__ float2 ld_first(const float2* a, unsigned long long pol) {
@@ -114,16 +109,15 @@ __device__ __forceinline__ float4 ld_first(const float4* a, unsigned long long p
                : "l"(a), "l"(pol));
   return v;
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // Programmatic dependent launch.  pdl_wait(): until the previous kernel of
 // the stream has completed and its writes are visible.  pdl_launch(): the
-// next kernel may be scheduled once every block has come here; a kernel
-// calls it shortly before its end, so that only its direct successor waits
-// on the SMs (called at the start, a chain of small kernels all become
-// resident and take the running one's slots: 48^3 mixed step 52.9 us).
+// next kernel may be scheduled once every block has come here or ended; an
+// FFT kernel calls it shortly before its end, so that only its direct successor
+// waits on the SMs (called at the start, a chain of small kernels all become
+// resident and take the running one's slots: 48^3 mixed step 52.9 us).  The
+// streaming kernels call it first: their default grid is one resident wave; with
+// more waves (a plan's 0 or 2) the successor waits for the last block to start.
 // Both are no-ops for launches without the programmatic-serialization
 // attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }

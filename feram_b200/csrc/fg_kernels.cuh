@@ -39,12 +39,15 @@ struct Geom {
   long long nsite;    // Lx*Ly*Lz
   long long ncplx;    // Lz*Ly*KXP
   long long nkpos;    // Ly*Lz*KXP
-  // Mixed path: FP64 sums of u and u u, [didi_rows][9], one row per warp of a
+  // Mixed path: sums of u and u u, [didi_rows][9], one row per warp of a
   // plane's block, written by the forward x-y pass and summed by
-  // homo_strain_tail (null: FP64 path, whose spectra have them).  The homogeneous strain and the k = 0 part of the
-  // dipole energies follow these nine numbers; their FP32 rounding (4e-8 of
-  // the k = 0 spectrum) moved the energies by 1e-3 eV from step to step at 64^3,
-  // the largest part of the thermostat's error.  k0_exact: the k-space pass
+  // homo_strain_tail (null: FP64 path, whose spectra have them).  The products
+  // are FP32; the two-stage kernels add the values of one butterfly (up to 64,
+  // cv_sum) in FP32, the general kernels the two of a pair, and every sum from
+  // there on is FP64.  The homogeneous strain and the k = 0 part of the dipole
+  // energies follow these nine numbers; the rounding of the FP32 spectrum they
+  // replace (4e-8 of its k = 0 value) moved the energies by 1e-3 eV from step to
+  // step at 64^3, the largest part of the thermostat's error.  k0_exact: the k-space pass
   // leaves k = 0 out of the dipole energies and the tail adds it.
   int k0_exact, didi_rows;
   double* didi;
@@ -551,7 +554,8 @@ __device__ __forceinline__ void columns_to_class(const CV<T>* buf, CV<T>* lo, CV
   }
 }
 
-// Sum of an element's values (of FP32 lanes: the mixed path's plane sums).
+// Sum of the values of n elements, in FP32 (the mixed path's plane sums): two
+// chains of n over the pairs of lanes, then those.
 __device__ __forceinline__ float cv_sum(const CV<float>* v, int n) {
   F2 a = v[0].re, b = v[0].im;
 #pragma unroll
@@ -2679,7 +2683,7 @@ __global__ void __launch_bounds__(256, 2)
                const unsigned char* __restrict__ layer_sump, const T* __restrict__ site_minv,
                const unsigned char* __restrict__ site_sump, double* __restrict__ part_ke, T* __restrict__ Flo,
                const AsmConst k, const RepArgs* __restrict__ grp, DevScalars* host) {
-  pdl_launch();  // one resident wave: nothing of this grid is left to schedule
+  pdl_launch();  // by default one resident wave, with nothing of this grid left to schedule
   pdl_wait();
   if (grp) {
     const RepArgs& a = grp[blockIdx.y];
@@ -3128,7 +3132,7 @@ __global__ void __launch_bounds__(256) k_kick_drift(T* __restrict__ p, T* __rest
                                                     const double* __restrict__ layer_minv,
                                                     const T* __restrict__ site_minv, const Phys* __restrict__ wave,
                                                     int gap_id, const RepArgs* __restrict__ grp) {
-  pdl_launch();  // one resident wave: nothing of this grid is left to schedule
+  pdl_launch();  // by default one resident wave, with nothing of this grid left to schedule
   pdl_wait();
   if (grp) {
     const RepArgs& a = grp[blockIdx.y];
@@ -3213,7 +3217,7 @@ __global__ void __launch_bounds__(256) k_kick_close(T* __restrict__ p, const T* 
                                                     const T* __restrict__ site_minv = nullptr,
                                                     const unsigned char* __restrict__ site_sump = nullptr,
                                                     DevScalars* host = nullptr) {
-  pdl_launch();  // one resident wave: nothing of this grid is left to schedule
+  pdl_launch();  // by default one resident wave, with nothing of this grid left to schedule
   pdl_wait();
   if (!PREP && blockIdx.x == 0) force_energies_tail(ph, sc, part_r, nblk_r, true);
   const long long ns = g.nsite;
